@@ -79,7 +79,6 @@ struct srcu_ctx {
   uint32_t table_log2 = 0;
   // normals outputs
   DevBuf nout[4], ncounts;
-  DevBuf parent;  // union-find parents (Euclidean clustering)
   DevBuf cov6;    // plane-regularised covariances, 6 floats per point
   DevBuf stage_block;  // host interleaved records, copied once before deinterleaving
   // the buffers of the last destroyed streaming voxel, kept for the next one
@@ -1078,7 +1077,7 @@ void srcu_destroy(srcu_ctx *ctx) {
   DevBuf *all[] = {&ctx->in_aos, &ctx->vaos, &ctx->keys[0], &ctx->keys[1], &ctx->vals[0], &ctx->vals[1], &ctx->lb_sort,
                    &ctx->lb_seg, &ctx->lb_cells, &ctx->vkeys, &ctx->vcounts, &ctx->vkeys3,
                    &ctx->pts, &ctx->pt_cell, &ctx->cell_key, &ctx->cell_start, &ctx->table, &ctx->ranges,
-                   &ctx->ncounts, &ctx->parent, &ctx->cov6, &ctx->stage_block,
+                   &ctx->ncounts, &ctx->cov6, &ctx->stage_block,
                    &ctx->rs_hyp, &ctx->rs_planes, &ctx->rs_valid, &ctx->rs_counts,
                    &ctx->rs_partials, &ctx->rs_mask, &ctx->xyz_tmp};
   for (DevBuf *b : all) release(ctx, *b);
@@ -1280,7 +1279,6 @@ srcu_status srcu_euclidean_cluster_roots(srcu_ctx *ctx, const srcu_cloud *cloud,
   if (!roots) return fail(ctx, SRCU_ERR_MISSING_FIELD, "roots is NULL");
   ST_TRY(reserve(ctx, n, 3, needs_staging(cloud), false, true));
   ST_TRY(reserve_batch(ctx, 1));
-  ST_TRY(ensure(ctx, ctx->parent, n * 4));
   srcu_cloud xyz = *cloud;
   xyz.n_attrs = 0;
   const float *cols[MAX_COLS];
@@ -1305,13 +1303,18 @@ srcu_status srcu_euclidean_cluster_roots(srcu_ctx *ctx, const srcu_cloud *cloud,
   uint32_t *dst = cloud->on_device ? roots : ptr<uint32_t>(ctx->nout[0]);
   {
     Launch l(ctx, SRCU_K_CLUSTER);
-    k_cluster_init<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, ptr<uint32_t>(ctx->parent),
-                                                         nullptr);
-    k_cluster_union<<<grid, CL_THREADS, 0, ctx->stream>>>(
-        ctx->ctl, ptr<const float4>(ctx->pts), ptr<const uint32_t>(ctx->pt_cell),
-        ptr<const uint2>(ctx->ranges), nullptr, r2, ptr<uint32_t>(ctx->parent));
-    k_cluster_roots<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, ptr<uint32_t>(ctx->parent), dst,
-                                                          nullptr);
+    // the grid has consumed the cell sort: its key buffer holds the forest
+    uint64_t *link = ptr<uint64_t>(ctx->keys[0]);
+    const float4 *pts = ptr<const float4>(ctx->pts);
+    const uint32_t *cell = ptr<const uint32_t>(ctx->pt_cell);
+    const uint2 *ranges = ptr<const uint2>(ctx->ranges);
+    k_cluster_init<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link);
+    k_cluster_union<true><<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, cell, ranges, r2,
+                                                                link);
+    k_cluster_flatten<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, link);
+    k_cluster_union<false><<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, cell, ranges, r2,
+                                                                 link);
+    k_cluster_roots<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link, dst);
   }
   CU_TRY(cudaGetLastError());
   ST_TRY(read_control(ctx));

@@ -121,3 +121,21 @@ def test_column_hash_path_on_huge_extent(cuda_ctx):
     x, y, z = (np.ascontiguousarray(p[:, k]) for k in range(3))
     assert np.array_equal(cuda_ctx.euclidean_cluster_roots(x, y, z, 0.25),
                           oracle.euclidean_roots(x, y, z, 0.25, sparse=True))
+
+
+@pytest.mark.parametrize("order", ["ascending", "descending", "shuffled"])
+@pytest.mark.parametrize("n", [2, 31, 33, 257, 4097])
+def test_chain_roots_in_any_index_order(cuda_ctx, n, order):
+    """A chain of points one tolerance step apart, cut in the middle: two
+    components whatever order the indices run in along it, and a trailing
+    duplicate and NaN point."""
+    at = np.arange(n, dtype=F)
+    at[n // 2:] += 5
+    rank = {"ascending": np.arange(n), "descending": np.arange(n)[::-1],
+            "shuffled": np.random.default_rng(n).permutation(n)}[order]
+    x = np.concatenate([at[rank], [at[rank[0]], np.nan]]).astype(F)
+    side = np.concatenate([rank >= n // 2, [rank[0] >= n // 2]])
+    expect = np.where(side, np.argmax(side), np.argmin(side))
+    zero = np.zeros(n + 2, F)
+    got = cuda_ctx.euclidean_cluster_roots(x, zero, zero, 1.0)
+    assert np.array_equal(got, np.append(expect, n + 1))

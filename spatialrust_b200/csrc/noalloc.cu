@@ -201,8 +201,8 @@ extern "C" srcu_status srcu_voxel_centroid_noalloc(const srcu_cloud *cloud,
   // cloud's offsets and parameters on every call.
   k_begin<<<1, 256, 0, s>>>(ctl, n, bt, 0u, 1, vp0, NormalParamsDev{});
   k_bounds<<<std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4), sms * 8)),
-             BND_THREADS, 0, s>>>(in[0], in[1], in[2], ctl, nullptr, nullptr, nullptr, bt);
-  k_voxel_plans<<<1, 32, 0, s>>>(ctl, bt);
+             BND_THREADS, 0, s>>>(in[0], in[1], in[2], ctl, nullptr, nullptr, nullptr, bt,
+                              PlanTasks{1u, 0u, 0ull});
   VoxelKeySrc src;
   src.x = in[0];
   src.y = in[1];

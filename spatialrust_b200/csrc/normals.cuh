@@ -17,84 +17,6 @@
 
 namespace srcu {
 
-// Cell plan of each cloud from its bounds (any box that contains every
-// finite point works).  h >= r (1 + 1e-5): points within r (f32 predicate)
-// then differ by at most one cell per axis even after the FP64 cell
-// arithmetic.  h is also kept >= extent / 2^19 so every axis fits in 20
-// bits; larger cells only add candidates, never drop neighbours.
-__global__ void k_cell_plans(Control *ctl, Batch bt) {
-  if (ld_relaxed_u32(&ctl->status)) return;
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= bt.clouds) return;
-  const float radius = bt.nparams[b].radius;
-  if (!(radius >= 0.0f) || isinf(radius)) {
-    atomicOr(&ctl->status, ST_BAD_PARAMS);
-    return;
-  }
-  CellPlan pl{};
-  const Bounds bd = bt.bounds[b];
-  double lo[3], ext[3], max_ext = 0.0;
-  for (int a = 0; a < 3; ++a) {
-    const bool any = bd.mn[a] != 0xffffffffu;
-    lo[a] = any ? double(ord2f(bd.mn[a])) : 0.0;
-    const double hi = any ? double(ord2f(bd.mx[a])) : 0.0;
-    ext[a] = hi - lo[a];
-    max_ext = fmax(max_ext, ext[a]);
-  }
-  double h = double(radius) * (1.0 + 1e-5);
-  h = fmax(h, max_ext * (1.0 / 524288.0));
-  h = fmax(h, 1e-30);
-  uint32_t total = 0;
-  for (int a = 0; a < 3; ++a) {
-    const double d = floor(ext[a] / h) + 1.0;
-    pl.dims[a] = d > 1048576.0 ? 1048576u : uint32_t(d);
-    pl.bits[a] = bit_width_u64(pl.dims[a] - 1);
-    total += pl.bits[a];
-    pl.origin[a] = lo[a];
-  }
-  pl.h = h;
-  pl.inv_h = 1.0 / h;
-  pl.shift_y = pl.bits[2];
-  pl.shift_x = pl.bits[1] + pl.bits[2];
-  pl.total_bits = total;
-  pl.num_digits = total == 0 ? 1u : (total + RADIX_BITS - 1) / RADIX_BITS;
-  pl.r2 = __fmul_rn(radius, radius);
-  pl.shell_tol = __fmul_rn(1e-6f, pl.r2);
-  pl.valid = 1;
-  bt.cplans[b] = pl;
-  atomicMax(&ctl->ckey_bits, total);
-  if (total + ctl->cloud_bits > 64) atomicOr(&ctl->status, ST_KEY_OVERFLOW);
-}
-
-// Places every cloud's (cx, cy) columns in one dense table when all of them
-// fit its `capacity` slots: col_base per cloud by a block scan over clouds.
-// Otherwise the chain keeps the column hash.  One block.
-__global__ void k_column_base(Control *ctl, Batch bt, uint64_t capacity) {
-  if (ld_relaxed_u32(&ctl->status)) return;
-  __shared__ unsigned long long scratch[256];
-  unsigned long long running = 0;
-  for (uint32_t b0 = 0; b0 < bt.clouds; b0 += 256) {
-    const uint32_t b = b0 + threadIdx.x;
-    unsigned long long cols = 0;
-    if (b < bt.clouds) cols = (unsigned long long)bt.cplans[b].dims[0] * bt.cplans[b].dims[1];
-    scratch[threadIdx.x] = cols;
-    __syncthreads();
-    for (uint32_t off = 1; off < 256; off <<= 1) {  // inclusive Hillis-Steele scan
-      const unsigned long long v = threadIdx.x >= off ? scratch[threadIdx.x - off] : 0ull;
-      __syncthreads();
-      scratch[threadIdx.x] += v;
-      __syncthreads();
-    }
-    if (b < bt.clouds) bt.cplans[b].col_base = running + scratch[threadIdx.x] - cols;
-    running += scratch[255];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) {
-    ctl->col_total = running;
-    ctl->dense_cols = running <= capacity ? 1u : 0u;
-  }
-}
-
 __device__ __forceinline__ uint64_t dense_column(const CellPlan &pl, uint64_t cx, uint64_t cy) {
   return pl.col_base + cx * pl.dims[1] + cy;
 }

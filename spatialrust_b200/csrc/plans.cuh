@@ -25,7 +25,7 @@ constexpr int MAX_COLS = 12;   // x, y, z + up to 9 attribute columns
 
 // Bounds over finite coordinates (ordered-uint encoded), with flags for
 // NaN / infinite values per axis.
-struct Bounds {
+struct alignas(16) Bounds {
   uint32_t mn[3];
   uint32_t mx[3];
   uint32_t flags;  // bit a: NaN seen on axis a; bit 3+a: +-inf seen on axis a
@@ -174,6 +174,7 @@ constexpr int WK_CSORT = 16;  // 8 slots
 constexpr int WK_CELLS = 24;
 constexpr int WK_NORMALS = 25;
 constexpr int WK_RANGES = 26;
+constexpr int WK_BOUNDS = 27;  // blocks of k_bounds that are done
 constexpr int WK_ORDER = 32;  // 4 slots
 
 __device__ __forceinline__ int64_t rs_sat_i64(float t) {
@@ -238,6 +239,9 @@ __device__ __forceinline__ void cell_unpack(const CellPlan &pl, uint64_t key, ui
 }
 
 __host__ __device__ __forceinline__ uint32_t bit_width_u64(uint64_t v) {
+#ifdef __CUDA_ARCH__
+  return 64u - uint32_t(__clzll((long long)v));
+#endif
   uint32_t b = 0;
   while (v) {
     ++b;
@@ -245,5 +249,155 @@ __host__ __device__ __forceinline__ uint32_t bit_width_u64(uint64_t v) {
   }
   return b;
 }
+
+// Bounds of cloud b as the other blocks' atomics left them in L2.
+__device__ __forceinline__ Bounds bounds_of(const Batch &bt, uint32_t b) {
+  union {
+    uint4 w[2];
+    Bounds v;
+  } u;
+  const uint4 *src = reinterpret_cast<const uint4 *>(bt.bounds + b);
+  u.w[0] = __ldcg(src);
+  u.w[1] = __ldcg(src + 1);
+  return u.v;
+}
+
+// Voxel-key plan of cloud b from its bounds and parameters
+// (filter_internal, voxel.rs:266-275).  The per-cloud key widths are reduced
+// to their maximum (ctl->vkey_bits); a cloud whose key plus the cloud id does
+// not fit in 64 bits stops the chain with ST_KEY_OVERFLOW.
+__device__ __noinline__ void voxel_plan(Control *ctl, const Batch &bt, uint32_t b) {
+  const VoxelParamsDev prm = bt.vparams[b];
+  VoxelPlan pl{};
+  pl.inv_leaf = __fdiv_rn(1.0f, prm.leaf);  // f32 IEEE division, voxel.rs:267
+  pl.floor_mode = prm.has_origin ? 1 : 0;
+  const Bounds bd = bounds_of(bt, b);
+  float lo[3], hi[3];
+  for (int a = 0; a < 3; ++a) {
+    const bool any = bd.mn[a] != 0xffffffffu;
+    lo[a] = any ? ord2f(bd.mn[a]) : __int_as_float(0x7fc00000);  // all-NaN axis -> NaN
+    hi[a] = any ? ord2f(bd.mx[a]) : __int_as_float(0x7fc00000);
+  }
+  for (int a = 0; a < 3; ++a) pl.origin[a] = prm.has_origin ? prm.origin[a] : lo[a];
+  bool ok = (bd.flags & (7u << 3)) == 0;  // an infinite coordinate saturates the key
+  uint32_t total = 0;
+  for (int a = 0; a < 3; ++a) {
+    int64_t k0 = voxel_axis_key(lo[a], pl.origin[a], pl.inv_leaf, pl.floor_mode);
+    int64_t k1 = voxel_axis_key(hi[a], pl.origin[a], pl.inv_leaf, pl.floor_mode);
+    if (isnan(lo[a])) k0 = k1 = 0;
+    if (bd.flags & (1u << a)) {  // NaN coordinates get key 0 (saturating cast)
+      k0 = min(k0, int64_t(0));
+      k1 = max(k1, int64_t(0));
+    }
+    pl.kmin[a] = k0;
+    const uint64_t range = uint64_t(k1) - uint64_t(k0);
+    pl.bits[a] = bit_width_u64(range);
+    total += pl.bits[a];
+  }
+  pl.shift_y = pl.bits[2];
+  pl.shift_x = pl.bits[1] + pl.bits[2];
+  pl.total_bits = total;
+  pl.num_digits = total == 0 ? 1u : (total + RADIX_BITS - 1) / RADIX_BITS;
+  if (total + ctl->cloud_bits > 64) ok = false;
+  if (ctl->n_points > LB_MAX_COUNT) {
+    atomicOr(&ctl->status, ST_TOO_MANY_POINTS);
+    ok = false;
+  }
+  pl.valid = ok ? 1u : 0u;
+  bt.vplans[b] = pl;
+  atomicMax(&ctl->vkey_bits, total);
+  if (!ok) atomicOr(&ctl->status, ST_KEY_OVERFLOW);
+}
+
+// Cell plan of cloud b from its bounds (any box that contains every
+// finite point works).  h >= r (1 + 1e-5): points within r (f32 predicate)
+// then differ by at most one cell per axis even after the FP64 cell
+// arithmetic.  h is also kept >= extent / 2^19 so every axis fits in 20
+// bits; larger cells only add candidates, never drop neighbours.
+__device__ __noinline__ void cell_plan(Control *ctl, const Batch &bt, uint32_t b) {
+  const float radius = bt.nparams[b].radius;
+  if (!(radius >= 0.0f) || isinf(radius)) {
+    atomicOr(&ctl->status, ST_BAD_PARAMS);
+    return;
+  }
+  CellPlan pl{};
+  const Bounds bd = bounds_of(bt, b);
+  double lo[3], ext[3], max_ext = 0.0;
+  for (int a = 0; a < 3; ++a) {
+    const bool any = bd.mn[a] != 0xffffffffu;
+    lo[a] = any ? double(ord2f(bd.mn[a])) : 0.0;
+    const double hi = any ? double(ord2f(bd.mx[a])) : 0.0;
+    ext[a] = hi - lo[a];
+    max_ext = fmax(max_ext, ext[a]);
+  }
+  double h = double(radius) * (1.0 + 1e-5);
+  h = fmax(h, max_ext * (1.0 / 524288.0));
+  h = fmax(h, 1e-30);
+  uint32_t total = 0;
+  for (int a = 0; a < 3; ++a) {
+    const double d = floor(ext[a] / h) + 1.0;
+    pl.dims[a] = d > 1048576.0 ? 1048576u : uint32_t(d);
+    pl.bits[a] = bit_width_u64(pl.dims[a] - 1);
+    total += pl.bits[a];
+    pl.origin[a] = lo[a];
+  }
+  pl.h = h;
+  pl.inv_h = 1.0 / h;
+  pl.shift_y = pl.bits[2];
+  pl.shift_x = pl.bits[1] + pl.bits[2];
+  pl.total_bits = total;
+  pl.num_digits = total == 0 ? 1u : (total + RADIX_BITS - 1) / RADIX_BITS;
+  pl.r2 = __fmul_rn(radius, radius);
+  pl.shell_tol = __fmul_rn(1e-6f, pl.r2);
+  pl.valid = 1;
+  bt.cplans[b] = pl;
+  atomicMax(&ctl->ckey_bits, total);
+  if (total + ctl->cloud_bits > 64) atomicOr(&ctl->status, ST_KEY_OVERFLOW);
+}
+
+// Places every cloud's (cx, cy) columns in one dense table when all of them
+// fit its `capacity` slots: col_base per cloud by a block scan over clouds.
+// Otherwise the chain keeps the column hash.  One block of 256 threads, after
+// its own cell plans; scratch holds 256 words.
+__device__ __noinline__ void column_bases(Control *ctl, const Batch &bt, uint64_t capacity,
+                                          unsigned long long *scratch) {
+  unsigned long long running = 0;
+  if (bt.clouds == 1) {
+    if (threadIdx.x == 0) {
+      running = (unsigned long long)bt.cplans[0].dims[0] * bt.cplans[0].dims[1];
+      bt.cplans[0].col_base = 0;
+      ctl->col_total = running;
+      ctl->dense_cols = running <= capacity ? 1u : 0u;
+    }
+    return;
+  }
+  for (uint32_t b0 = 0; b0 < bt.clouds; b0 += 256) {
+    const uint32_t b = b0 + threadIdx.x;
+    unsigned long long cols = 0;
+    if (b < bt.clouds) cols = (unsigned long long)bt.cplans[b].dims[0] * bt.cplans[b].dims[1];
+    scratch[threadIdx.x] = cols;
+    __syncthreads();
+    for (uint32_t off = 1; off < 256; off <<= 1) {  // inclusive Hillis-Steele scan
+      const unsigned long long v = threadIdx.x >= off ? scratch[threadIdx.x - off] : 0ull;
+      __syncthreads();
+      scratch[threadIdx.x] += v;
+      __syncthreads();
+    }
+    if (b < bt.clouds) bt.cplans[b].col_base = running + scratch[threadIdx.x] - cols;
+    running += scratch[255];
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    ctl->col_total = running;
+    ctl->dense_cols = running <= capacity ? 1u : 0u;
+  }
+}
+
+// What the last block of k_bounds derives from the bounds.
+struct PlanTasks {
+  uint32_t voxel;         // the voxel-key plans
+  uint32_t cell;          // the cell plans and the column bases
+  uint64_t col_capacity;  // slots of the column table
+};
 
 }  // namespace srcu

@@ -11,6 +11,7 @@
 
 #include "../../include/srcuda.h"
 #include "cluster.cuh"
+#include "columns.cuh"
 #include "host_copy.h"
 #include "normals.cuh"
 #include "sort_tuning.h"
@@ -86,6 +87,7 @@ struct srcu_ctx {
   // RANSAC plane scoring: hypotheses, planes, validity, counts, block partials, mask
   DevBuf rs_hyp, rs_planes, rs_valid, rs_counts, rs_partials, rs_mask;
   uint32_t last_attrs = 0;  // attribute count of the last enqueued chain
+  uint64_t last_points = 0; // points of the last chain: no result has more rows
   const float *frame_attr_ptrs[MAX_COLS] = {};
   // batch arrays (clouds of the last chain) and pinned staging for their parameters
   DevBuf b_offsets, b_bounds, b_vplans, b_cplans, b_vparams, b_nparams, b_voff;
@@ -730,21 +732,29 @@ srcu_status enqueue_first_seen(srcu_ctx *ctx, const float **in, uint64_t n) {
   return SRCU_OK;
 }
 
-// Voxel stage: bounds -> plan -> sort -> fused segment/centroid reduction.
-srcu_status enqueue_voxel(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t n,
-                          const Batch &bt) {
-  const uint32_t grid_b = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4),
-                                                                    uint32_t(ctx->num_sms) * 16));
-  {
-    Launch l(ctx, SRCU_K_BOUNDS);
-    k_bounds<<<grid_b, BND_THREADS, 0, ctx->stream>>>(in[0], in[1], in[2], ctx->ctl, nullptr,
-                                                       nc > 3 ? in[3] : nullptr,
-                                                       ptr<float4>(ctx->in_aos), bt);
-  }
-  {
-    Launch l(ctx, SRCU_K_VOXEL_PLAN);
-    k_voxel_plans<<<ceil_div(bt.clouds, 128), 128, 0, ctx->stream>>>(ctx->ctl, bt);
-  }
+// Bounds of every cloud, an AoS copy of the points, and the plans of the
+// stages that follow.
+srcu_status enqueue_bounds(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t n, const Batch &bt,
+                           bool voxel, bool cell) {
+  const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4),
+                                                                  uint32_t(ctx->num_sms) * 16));
+  PlanTasks tasks;
+  tasks.voxel = voxel;
+  tasks.cell = cell;
+  tasks.col_capacity = uint64_t(1) << ctx->table_log2;
+  Launch l(ctx, SRCU_K_BOUNDS);
+  k_bounds<<<grid, BND_THREADS, 0, ctx->stream>>>(in[0], in[1], in[2], ctx->ctl, nullptr,
+                                                  nc > 3 ? in[3] : nullptr,
+                                                  ptr<float4>(ctx->in_aos), bt, tasks);
+  CU_TRY(cudaGetLastError());
+  return SRCU_OK;
+}
+
+// Voxel stage: bounds and plans -> sort -> fused segment/centroid reduction.
+// normals: the chain's cell plans are made as well.
+srcu_status enqueue_voxel(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t n, const Batch &bt,
+                          bool normals) {
+  ST_TRY(enqueue_bounds(ctx, in, nc, n, bt, true, normals));
   VoxelKeySrc src;
   src.x = in[0];
   src.y = in[1];
@@ -780,15 +790,11 @@ srcu_status enqueue_voxel(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t
 
 // Normals stage over (x, y, z) with the point count in *count_dev (device)
 // or ctl->n_points when count_dev is null; n_max bounds the grid sizes.
-// Radius grid: cell plans, cell sort, cell table, column hash, column ranges.
+// Radius grid (the cell plans are made with the bounds): cell sort, cell table,
+// column hash, column ranges.
 srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const float *z,
                          const float4 *aos, const unsigned long long *count_dev, uint64_t n_max,
                          const Batch &bt, const uint64_t *voxel_keys) {
-  {
-    Launch l(ctx, SRCU_K_CELL_PLAN);
-    k_cell_plans<<<ceil_div(bt.clouds, 128), 128, 0, ctx->stream>>>(ctx->ctl, bt);
-    k_column_base<<<1, 256, 0, ctx->stream>>>(ctx->ctl, bt, uint64_t(1) << ctx->table_log2);
-  }
   CellKeySrc src;
   src.x = x;
   src.y = y;
@@ -891,6 +897,7 @@ srcu_status begin_chain(srcu_ctx *ctx, uint64_t n, const Batch &bt, int single,
   k_begin<<<1, 256, 0, ctx->stream>>>(ctx->ctl, n, bt, cloud_bits_for(bt.clouds), single,
                                       to_dev(vp), to_dev(np));
   ctx->last_clouds = bt.clouds;
+  ctx->last_points = n;
   if (single) {
     ctx->agg_all = to_dev(vp).agg;
     ctx->count_shell = np && np->count_shell;
@@ -899,8 +906,11 @@ srcu_status begin_chain(srcu_ctx *ctx, uint64_t n, const Batch &bt, int single,
   return SRCU_OK;
 }
 
+// The control block up to its histograms, which the host has no use for.
+constexpr size_t kControlHead = offsetof(Control, hist_v);
+
 srcu_status read_control(srcu_ctx *ctx) {
-  CU_TRY(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost,
+  CU_TRY(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl, kControlHead, cudaMemcpyDeviceToHost,
                          ctx->stream));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   const uint32_t st = ctx->ctl_host->status;
@@ -961,16 +971,64 @@ srcu_status check_normal_params(srcu_ctx *ctx, const srcu_normal_params *np) {
   return SRCU_OK;
 }
 
+// Whether k_take_columns may read as many rows of a result buffer as the last
+// chain can have written: a buffer that it did not fill (normals of a chain
+// without them) can be smaller, and is left to a copy, which checks.
+bool takable(const srcu_ctx *ctx, const DevBuf &b, uint32_t words = 1) {
+  return b.p && b.bytes >= size_t(ctx->last_points) * words * 4;
+}
+
+void take_column(const srcu_ctx *ctx, TakeColumns &t, void *dst, const DevBuf &src,
+                 uint32_t words = 1) {
+  if (!dst || !takable(ctx, src, words)) return;
+  t.src[t.count] = static_cast<const uint32_t *>(src.p);
+  t.dst[t.count] = static_cast<uint32_t *>(dst);
+  t.words[t.count++] = words;
+}
+
+// Queues the copies of the chain's results that go to device memory, their
+// row count (`rows`, a device word) unread: they run before the wait for the
+// control block, and not at all when the chain failed.
+srcu_status take_results(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *vout,
+                         const srcu_normal_out *nout, const unsigned long long *rows) {
+  TakeColumns t{};
+  if (vout && vout->on_device) {
+    float *dst[MAX_COLS] = {vout->x, vout->y, vout->z};
+    for (uint32_t a = 3; a < nc; ++a) dst[a] = vout->attrs ? vout->attrs[a - 3] : nullptr;
+    for (uint32_t c = 0; c < nc; ++c) take_column(ctx, t, dst[c], ctx->vout[c]);
+    take_column(ctx, t, vout->counts, ctx->vcounts);
+    take_column(ctx, t, vout->keys, ctx->vkeys3, 6);
+  }
+  if (nout && nout->on_device) {
+    float *dst[4] = {nout->nx, nout->ny, nout->nz, nout->curvature};
+    for (int c = 0; c < 4; ++c) take_column(ctx, t, dst[c], ctx->nout[c]);
+    take_column(ctx, t, nout->neighbor_counts, ctx->ncounts);
+  }
+  if (t.count == 0) return SRCU_OK;
+  // about eight blocks per SM over all columns; rows past the count cost nothing
+  const uint32_t blocks = std::max<uint32_t>(1, uint32_t(ctx->num_sms) * 8 / t.count);
+  k_take_columns<<<dim3(blocks, t.count), TAKE_THREADS, 0, ctx->stream>>>(ctx->ctl, t, rows);
+  CU_TRY(cudaGetLastError());
+  return SRCU_OK;
+}
+
+// One result column of `rows` rows, unless take_results took it.
+srcu_status fetch_column(srcu_ctx *ctx, void *dst, const DevBuf &src, uint64_t rows, int on_device,
+                         cudaStream_t stream = nullptr, uint32_t words = 1) {
+  if (on_device && takable(ctx, src, words)) return SRCU_OK;
+  return copy_out(ctx, dst, src.p, rows * words * 4, on_device, stream);
+}
+
+// The results take_results left, once their row count is known.
 srcu_status fetch_voxels(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *out, uint64_t v,
                          cudaStream_t stream = nullptr, bool keys = true) {
   if (!out) return SRCU_OK;
   float *dst[MAX_COLS] = {out->x, out->y, out->z};
   for (uint32_t a = 3; a < nc; ++a) dst[a] = out->attrs ? out->attrs[a - 3] : nullptr;
   for (uint32_t c = 0; c < nc; ++c)
-    ST_TRY(copy_out(ctx, dst[c], ctx->vout[c].p, v * 4, out->on_device, stream));
-  ST_TRY(copy_out(ctx, out->counts, ctx->vcounts.p, v * 4, out->on_device, stream));
-  if (keys && out->keys)
-    ST_TRY(copy_out(ctx, out->keys, ctx->vkeys3.p, v * 24, out->on_device, stream));
+    ST_TRY(fetch_column(ctx, dst[c], ctx->vout[c], v, out->on_device, stream));
+  ST_TRY(fetch_column(ctx, out->counts, ctx->vcounts, v, out->on_device, stream));
+  if (keys) ST_TRY(fetch_column(ctx, out->keys, ctx->vkeys3, v, out->on_device, stream, 6));
   return SRCU_OK;
 }
 
@@ -978,8 +1036,8 @@ srcu_status fetch_normals(srcu_ctx *ctx, const srcu_normal_out *out, uint64_t m,
                           srcu_normal_stats *stats) {
   if (out) {
     float *dst[4] = {out->nx, out->ny, out->nz, out->curvature};
-    for (int c = 0; c < 4; ++c) ST_TRY(copy_out(ctx, dst[c], ctx->nout[c].p, m * 4, out->on_device));
-    ST_TRY(copy_out(ctx, out->neighbor_counts, ctx->ncounts.p, m * 4, out->on_device));
+    for (int c = 0; c < 4; ++c) ST_TRY(fetch_column(ctx, dst[c], ctx->nout[c], m, out->on_device));
+    ST_TRY(fetch_column(ctx, out->neighbor_counts, ctx->ncounts, m, out->on_device));
   }
   if (stats) {
     stats->valid_count = ctx->ctl_host->ncount.valid;
@@ -1223,8 +1281,9 @@ srcu_status srcu_voxel_centroid(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(stage_input(ctx, cloud, cols));
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, params, nullptr));
-  ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt));
+  ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, false));
   if (out && out->keys) ST_TRY(unpack_keys(ctx, n));
+  ST_TRY(take_results(ctx, nc, out, nullptr, &ctx->ctl->n_voxels));
   ST_TRY(read_control(ctx));
   const uint64_t v = ctx->ctl_host->n_voxels;
   ST_TRY(fetch_voxels(ctx, nc, out, v));
@@ -1251,15 +1310,10 @@ srcu_status srcu_radius_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(stage_input(ctx, &xyz, cols));
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, nullptr, params));
-  const uint32_t grid_b = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4),
-                                                                    uint32_t(ctx->num_sms) * 8));
-  {
-    Launch l(ctx, SRCU_K_BOUNDS);
-    k_bounds<<<grid_b, BND_THREADS, 0, ctx->stream>>>(cols[0], cols[1], cols[2], ctx->ctl, nullptr,
-                                                       nullptr, ptr<float4>(ctx->in_aos), bt);
-  }
+  ST_TRY(enqueue_bounds(ctx, cols, 3, n, bt, false, true));
   ST_TRY(enqueue_normals(ctx, cols[0], cols[1], cols[2], ptr<const float4>(ctx->in_aos), nullptr, n,
                          bt, nullptr));
+  ST_TRY(take_results(ctx, 3, nullptr, out, &ctx->ctl->n_points));
   ST_TRY(read_control(ctx));
   ST_TRY(fetch_normals(ctx, out, n, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
@@ -1288,13 +1342,7 @@ srcu_status srcu_euclidean_cluster_roots(srcu_ctx *ctx, const srcu_cloud *cloud,
   np.radius = cluster_tolerance;  // the grid of a radius search with r = tolerance
   np.min_neighbors = 1;
   ST_TRY(begin_chain(ctx, n, bt, 1, nullptr, &np));
-  const uint32_t grid_b = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4),
-                                                                    uint32_t(ctx->num_sms) * 8));
-  {
-    Launch l(ctx, SRCU_K_BOUNDS);
-    k_bounds<<<grid_b, BND_THREADS, 0, ctx->stream>>>(cols[0], cols[1], cols[2], ctx->ctl, nullptr,
-                                                       nullptr, ptr<float4>(ctx->in_aos), bt);
-  }
+  ST_TRY(enqueue_bounds(ctx, cols, 3, n, bt, false, true));
   ST_TRY(enqueue_grid(ctx, cols[0], cols[1], cols[2], ptr<const float4>(ctx->in_aos), nullptr, n,
                       bt, nullptr));
   const float r2 = cluster_tolerance * cluster_tolerance;  // radius_sq, uniform_grid.rs:109
@@ -1354,13 +1402,7 @@ srcu_status srcu_plane_covariances(srcu_ctx *ctx, const srcu_cloud *cloud, float
   np.min_neighbors = 3;
   np.include_self = 1;
   ST_TRY(begin_chain(ctx, n, bt, 1, nullptr, &np));
-  const uint32_t grid_b = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, BND_THREADS * 4),
-                                                                    uint32_t(ctx->num_sms) * 8));
-  {
-    Launch l(ctx, SRCU_K_BOUNDS);
-    k_bounds<<<grid_b, BND_THREADS, 0, ctx->stream>>>(cols[0], cols[1], cols[2], ctx->ctl, nullptr,
-                                                       nullptr, ptr<float4>(ctx->in_aos), bt);
-  }
+  ST_TRY(enqueue_bounds(ctx, cols, 3, n, bt, false, true));
   ST_TRY(enqueue_grid(ctx, cols[0], cols[1], cols[2], ptr<const float4>(ctx->in_aos), nullptr, n,
                       bt, nullptr));
   {
@@ -1402,7 +1444,7 @@ srcu_status srcu_voxel_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(stage_input(ctx, cloud, cols));
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, vparams, nparams));
-  ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt));
+  ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, true));
   // The centroids are final once the voxel stage is done: their read-back
   // runs on the side stream while the normal kernels run.  The host learns V
   // from a small copy of the control-block head taken at that point.
@@ -1414,8 +1456,9 @@ srcu_status srcu_voxel_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
                          ptr<float>(ctx->vout[2]), ptr<const float4>(ctx->vaos),
                          &ctx->ctl->n_voxels, n, bt, ptr<uint64_t>(ctx->vkeys)));
   if (vout && vout->keys) ST_TRY(unpack_keys(ctx, n));
+  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels));
   bool early = false;
-  if (vout) {
+  if (vout && !vout->on_device) {
     CU_TRY(cudaEventSynchronize(ctx->ev_voxel));
     const Control *head = reinterpret_cast<const Control *>(ctx->head_host);
     if (head->status == 0) {  // otherwise read_control below reports the failure
@@ -1429,10 +1472,10 @@ srcu_status srcu_voxel_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
   if (st != SRCU_OK) return st;
   const uint64_t v = ctx->ctl_host->n_voxels;
   if (!early) ST_TRY(fetch_voxels(ctx, nc, vout, v));
-  else if (vout->keys) ST_TRY(copy_out(ctx, vout->keys, ctx->vkeys3.p, v * 24, vout->on_device));
+  else if (vout->keys) ST_TRY(copy_out(ctx, vout->keys, ctx->vkeys3.p, v * 24, 0));
   ST_TRY(fetch_normals(ctx, nout, v, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
-  CU_TRY(cudaStreamSynchronize(ctx->side_stream));
+  if (early) CU_TRY(cudaStreamSynchronize(ctx->side_stream));
   if (out_voxels) *out_voxels = v;
   return SRCU_OK;
 }
@@ -1455,7 +1498,7 @@ srcu_status srcu_voxel_normals_enqueue(srcu_ctx *ctx, const srcu_cloud *cloud,
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, vparams, nparams));
   if (n > 0) {
-    ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt));
+    ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, true));
     ST_TRY(enqueue_normals(ctx, ptr<float>(ctx->vout[0]), ptr<float>(ctx->vout[1]),
                            ptr<float>(ctx->vout[2]), ptr<const float4>(ctx->vaos),
                            &ctx->ctl->n_voxels, n, bt, ptr<uint64_t>(ctx->vkeys)));
@@ -1480,7 +1523,7 @@ srcu_status srcu_voxel_centroid_enqueue(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(stage_input(ctx, cloud, cols));
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, vparams, nullptr));
-  if (n > 0) ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt));
+  if (n > 0) ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, false));
   ctx->last_attrs = cloud->n_attrs;
   CU_TRY(cudaGetLastError());
   return SRCU_OK;
@@ -1523,7 +1566,7 @@ static srcu_status batch_enqueue(srcu_ctx *ctx, const srcu_cloud *points, const 
   ctx->count_shell = false;
   for (uint32_t b = 0; b < count; ++b) ctx->count_shell |= nparams[b].count_shell != 0;
   if (n > 0) {
-    ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt));
+    ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, true));
     ST_TRY(enqueue_normals(ctx, ptr<float>(ctx->vout[0]), ptr<float>(ctx->vout[1]),
                            ptr<float>(ctx->vout[2]), ptr<const float4>(ctx->vaos),
                            &ctx->ctl->n_voxels, n, bt, ptr<uint64_t>(ctx->vkeys)));
@@ -1545,6 +1588,7 @@ struct srcu_graph {
   cudaGraphExec_t exec = nullptr;
   uint32_t clouds = 1;
   uint32_t attrs = 0;
+  uint64_t points = 0;
 };
 
 srcu_status srcu_chain_graph_create(srcu_ctx *ctx, const srcu_cloud *points,
@@ -1567,6 +1611,7 @@ srcu_status srcu_chain_graph_create(srcu_ctx *ctx, const srcu_cloud *points,
   srcu_graph *g = new srcu_graph();
   g->clouds = cnt;
   g->attrs = points->n_attrs;
+  g->points = points->n;
   const uint64_t mask = ctx->prof_mask;
   ctx->prof_mask = 0;  // no timing events inside a graph
   cudaError_t e = cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal);
@@ -1597,6 +1642,7 @@ srcu_status srcu_graph_launch(srcu_ctx *ctx, srcu_graph *g) {
   CU_TRY(cudaGraphLaunch(g->exec, ctx->stream));
   ctx->last_clouds = g->clouds;
   ctx->last_attrs = g->attrs;
+  ctx->last_points = g->points;
   return SRCU_OK;
 }
 
@@ -1650,11 +1696,15 @@ srcu_status srcu_frame_check(srcu_ctx *ctx, uint64_t *out_voxels, srcu_normal_st
 srcu_status srcu_frame_fetch(srcu_ctx *ctx, const srcu_voxel_out *vout, const srcu_normal_out *nout,
                              uint64_t *out_voxels, srcu_normal_stats *stats) {
   if (!ctx) return SRCU_ERR_INVALID_ARGUMENT;
+  if (vout && vout->keys) {
+    ST_TRY(read_control(ctx));  // a failed chain is reported before the argument
+    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "frame read-back does not unpack voxel keys");
+  }
+  const uint32_t nc = 3 + ctx->last_attrs;
+  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels));
   ST_TRY(read_control(ctx));
   const uint64_t v = ctx->ctl_host->n_voxels;
-  if (vout && vout->keys)
-    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "frame read-back does not unpack voxel keys");
-  ST_TRY(fetch_voxels(ctx, 3 + ctx->last_attrs, vout, v));
+  ST_TRY(fetch_voxels(ctx, nc, vout, v));
   ST_TRY(fetch_normals(ctx, nout, v, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   if (out_voxels) *out_voxels = v;
@@ -1663,7 +1713,7 @@ srcu_status srcu_frame_fetch(srcu_ctx *ctx, const srcu_voxel_out *vout, const sr
 
 srcu_status srcu_chain_info_get(srcu_ctx *ctx, srcu_chain_info *info) {
   if (!ctx || !info) return SRCU_ERR_INVALID_ARGUMENT;
-  CU_TRY(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl, sizeof(Control), cudaMemcpyDeviceToHost,
+  CU_TRY(cudaMemcpyAsync(ctx->ctl_host, ctx->ctl, kControlHead, cudaMemcpyDeviceToHost,
                          ctx->stream));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   const Control &c = *ctx->ctl_host;

@@ -94,77 +94,73 @@ __global__ void k_deinterleave(Interleaved iv, uint64_t n) {
     for (uint32_t c = 0; c < iv.nc; ++c) iv.dst[c][i] = iv.src[c][i * iv.stride];
 }
 
-// Per-cloud min/max over finite coordinates plus NaN / inf flags
-// (compute_bounds, voxel.rs:1067-1079, ignores NaN through f32::min/max).
-// The point count comes from *count_dev when non-null, else ctl->n_points.
-// Optionally writes an AoS copy (x, y, z, first attribute) so that later
-// gathers by point index touch one 32-byte sector per point.
-__global__ void __launch_bounds__(BND_THREADS) k_bounds(const float *x, const float *y,
-                                                        const float *z, Control *ctl,
-                                                        const unsigned long long *count_dev,
-                                                        const float *a0, float4 *aos, Batch bt) {
-  if (ld_relaxed_u32(&ctl->status)) return;
-  const uint64_t n = count_dev ? *count_dev : ctl->n_points;
-  if (bt.clouds == 1) {
-    BoundsAcc acc;
-    acc.reset();
-    const uint64_t stride = uint64_t(gridDim.x) * BND_THREADS;
-    uint64_t i = blockIdx.x * uint64_t(BND_THREADS) + threadIdx.x;
-    // four points per thread in flight: all loads first, then the stores
-    for (; i + 3 * stride < n; i += 4 * stride) {
-      float px[4], py[4], pz[4], pa[4];
+// k_bounds over one cloud of n points.
+__device__ __forceinline__ void bounds_one_cloud(const float *x, const float *y, const float *z,
+                                                 uint64_t n, const float *a0, float4 *aos,
+                                                 Bounds *bounds) {
+  BoundsAcc acc;
+  acc.reset();
+  const uint64_t stride = uint64_t(gridDim.x) * BND_THREADS;
+  uint64_t i = blockIdx.x * uint64_t(BND_THREADS) + threadIdx.x;
+  // four points per thread in flight: all loads first, then the stores
+  for (; i + 3 * stride < n; i += 4 * stride) {
+    float px[4], py[4], pz[4], pa[4];
 #pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint64_t k = i + uint64_t(q) * stride;
-        px[q] = x[k];
-        py[q] = y[k];
-        pz[q] = z[k];
-        pa[q] = a0 ? a0[k] : 0.0f;
-      }
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        if (aos) aos[i + uint64_t(q) * stride] = make_float4(px[q], py[q], pz[q], pa[q]);
-        acc.add(px[q], py[q], pz[q]);
-      }
-    }
-    for (; i < n; i += stride) {
-      const float xi = x[i], yi = y[i], zi = z[i];
-      if (aos) aos[i] = make_float4(xi, yi, zi, a0 ? a0[i] : 0.0f);
-      acc.add(xi, yi, zi);
+    for (int q = 0; q < 4; ++q) {
+      const uint64_t k = i + uint64_t(q) * stride;
+      px[q] = x[k];
+      py[q] = y[k];
+      pz[q] = z[k];
+      pa[q] = a0 ? a0[k] : 0.0f;
     }
 #pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        acc.mn[a] = min(acc.mn[a], __shfl_xor_sync(FULL_MASK, acc.mn[a], o));
-        acc.mx[a] = max(acc.mx[a], __shfl_xor_sync(FULL_MASK, acc.mx[a], o));
-      }
+    for (int q = 0; q < 4; ++q) {
+      if (aos) aos[i + uint64_t(q) * stride] = make_float4(px[q], py[q], pz[q], pa[q]);
+      acc.add(px[q], py[q], pz[q]);
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) acc.flags |= __shfl_xor_sync(FULL_MASK, acc.flags, o);
-    // one flush per block: warp results meet in shared memory first
-    __shared__ uint32_t sred[BND_THREADS / 32][7];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    if (lane == 0) {
-      for (int a = 0; a < 3; ++a) {
-        sred[warp][a] = acc.mn[a];
-        sred[warp][3 + a] = acc.mx[a];
-      }
-      sred[warp][6] = acc.flags;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      for (uint32_t w = 1; w < BND_THREADS / 32; ++w) {
-        for (int a = 0; a < 3; ++a) {
-          acc.mn[a] = min(acc.mn[a], sred[w][a]);
-          acc.mx[a] = max(acc.mx[a], sred[w][3 + a]);
-        }
-        acc.flags |= sred[w][6];
-      }
-      acc.flush(bt.bounds[0]);
-    }
-    return;
   }
+  for (; i < n; i += stride) {
+    const float xi = x[i], yi = y[i], zi = z[i];
+    if (aos) aos[i] = make_float4(xi, yi, zi, a0 ? a0[i] : 0.0f);
+    acc.add(xi, yi, zi);
+  }
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      acc.mn[a] = min(acc.mn[a], __shfl_xor_sync(FULL_MASK, acc.mn[a], o));
+      acc.mx[a] = max(acc.mx[a], __shfl_xor_sync(FULL_MASK, acc.mx[a], o));
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) acc.flags |= __shfl_xor_sync(FULL_MASK, acc.flags, o);
+  // one flush per block: warp results meet in shared memory first
+  __shared__ uint32_t sred[BND_THREADS / 32][7];
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  if (lane == 0) {
+    for (int a = 0; a < 3; ++a) {
+      sred[warp][a] = acc.mn[a];
+      sred[warp][3 + a] = acc.mx[a];
+    }
+    sred[warp][6] = acc.flags;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (uint32_t w = 1; w < BND_THREADS / 32; ++w) {
+      for (int a = 0; a < 3; ++a) {
+        acc.mn[a] = min(acc.mn[a], sred[w][a]);
+        acc.mx[a] = max(acc.mx[a], sred[w][3 + a]);
+      }
+      acc.flags |= sred[w][6];
+    }
+    acc.flush(bounds[0]);
+  }
+}
+
+// k_bounds over the concatenated clouds of a batch.
+__device__ __forceinline__ void bounds_many_clouds(const float *x, const float *y, const float *z,
+                                                   uint64_t n, const float *a0, float4 *aos,
+                                                   const Batch &bt) {
   // Many clouds: each warp owns a span of 32 * BND_CHUNK consecutive points,
   // read coalesced.  A span inside one cloud (all but at most one span per
   // cloud boundary) reduces across the warp and flushes once; a span that
@@ -235,54 +231,44 @@ __global__ void __launch_bounds__(BND_THREADS) k_bounds(const float *x, const fl
   }
 }
 
-// One voxel-key plan per cloud from its bounds and parameters
-// (filter_internal, voxel.rs:266-275).  The per-cloud key widths are reduced
-// to their maximum (ctl->vkey_bits); a cloud whose key plus the cloud id does
-// not fit in 64 bits stops the chain with ST_KEY_OVERFLOW.
-__global__ void k_voxel_plans(Control *ctl, Batch bt) {
+// Per-cloud min/max over finite coordinates plus NaN / inf flags
+// (compute_bounds, voxel.rs:1067-1079, ignores NaN through f32::min/max).
+// The point count comes from *count_dev when non-null, else ctl->n_points.
+// Optionally writes an AoS copy (x, y, z, first attribute) so that later
+// gathers by point index touch one 32-byte sector per point.
+//
+// The block that finishes last derives the chain's plans from the bounds: they
+// move no data, so as launches of their own (voxel plans, cell plans, column
+// bases) they cost a launch latency each, 10 us of a chain, against 4 us in this
+// kernel's tail.  Six blocks per SM: the plans' registers would leave five, which
+// cost the loop 8 us at 2M points.
+__global__ void __launch_bounds__(BND_THREADS, 6) k_bounds(const float *x, const float *y,
+                                                        const float *z, Control *ctl,
+                                                        const unsigned long long *count_dev,
+                                                        const float *a0, float4 *aos, Batch bt,
+                                                        PlanTasks tasks) {
   if (ld_relaxed_u32(&ctl->status)) return;
-  const uint32_t b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= bt.clouds) return;
-  const VoxelParamsDev prm = bt.vparams[b];
-  VoxelPlan pl{};
-  pl.inv_leaf = __fdiv_rn(1.0f, prm.leaf);  // f32 IEEE division, voxel.rs:267
-  pl.floor_mode = prm.has_origin ? 1 : 0;
-  const Bounds bd = bt.bounds[b];
-  float lo[3], hi[3];
-  for (int a = 0; a < 3; ++a) {
-    const bool any = bd.mn[a] != 0xffffffffu;
-    lo[a] = any ? ord2f(bd.mn[a]) : __int_as_float(0x7fc00000);  // all-NaN axis -> NaN
-    hi[a] = any ? ord2f(bd.mx[a]) : __int_as_float(0x7fc00000);
-  }
-  for (int a = 0; a < 3; ++a) pl.origin[a] = prm.has_origin ? prm.origin[a] : lo[a];
-  bool ok = (bd.flags & (7u << 3)) == 0;  // an infinite coordinate saturates the key
-  uint32_t total = 0;
-  for (int a = 0; a < 3; ++a) {
-    int64_t k0 = voxel_axis_key(lo[a], pl.origin[a], pl.inv_leaf, pl.floor_mode);
-    int64_t k1 = voxel_axis_key(hi[a], pl.origin[a], pl.inv_leaf, pl.floor_mode);
-    if (isnan(lo[a])) k0 = k1 = 0;
-    if (bd.flags & (1u << a)) {  // NaN coordinates get key 0 (saturating cast)
-      k0 = min(k0, int64_t(0));
-      k1 = max(k1, int64_t(0));
-    }
-    pl.kmin[a] = k0;
-    const uint64_t range = uint64_t(k1) - uint64_t(k0);
-    pl.bits[a] = bit_width_u64(range);
-    total += pl.bits[a];
-  }
-  pl.shift_y = pl.bits[2];
-  pl.shift_x = pl.bits[1] + pl.bits[2];
-  pl.total_bits = total;
-  pl.num_digits = total == 0 ? 1u : (total + RADIX_BITS - 1) / RADIX_BITS;
-  if (total + ctl->cloud_bits > 64) ok = false;
-  if (ctl->n_points > LB_MAX_COUNT) {
-    atomicOr(&ctl->status, ST_TOO_MANY_POINTS);
-    ok = false;
-  }
-  pl.valid = ok ? 1u : 0u;
-  bt.vplans[b] = pl;
-  atomicMax(&ctl->vkey_bits, total);
-  if (!ok) atomicOr(&ctl->status, ST_KEY_OVERFLOW);
+  const uint64_t n = count_dev ? *count_dev : ctl->n_points;
+  if (bt.clouds == 1) bounds_one_cloud(x, y, z, n, a0, aos, bt.bounds);
+  else bounds_many_clouds(x, y, z, n, a0, aos, bt);
+
+  __shared__ uint32_t last;
+  __shared__ unsigned long long scratch[256];
+  __threadfence();  // this thread's bounds, before the block counts as done
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(&ctl->work[WK_BOUNDS], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // the two kinds of plan do not depend on each other: half a block each
+  constexpr uint32_t HALF = BND_THREADS / 2;
+  const uint32_t t = threadIdx.x;
+  if (tasks.voxel && t < HALF)
+    for (uint32_t b = t; b < bt.clouds; b += HALF) voxel_plan(ctl, bt, b);
+  if (tasks.cell && t >= HALF)
+    for (uint32_t b = t - HALF; b < bt.clouds; b += HALF) cell_plan(ctl, bt, b);
+  __syncthreads();
+  if (tasks.cell) column_bases(ctl, bt, tasks.col_capacity, scratch);
 }
 
 // Key source for the voxel sort: the reference's voxel key of point i,

@@ -442,6 +442,7 @@ constexpr int NM_THREADS = 256;
 constexpr int NM_FLUSH = 32;  // f32 partial moments are folded into FP64 every NM_FLUSH candidates
 constexpr double NM_REFINE_GAP = 0.05;  // (l1 - l0) / trace below this -> FP64 moments
 constexpr double NM_REFINE_MEAN = 0.875;  // |E[d]|^2 / E|d|^2 above this -> FP64 moments
+constexpr uint32_t NM_OVERREAD = 8;  // records the packed walk may read past a range's end
 constexpr uint32_t NM_STAGE = 256;  // candidate records staged per warp (4 KB), staged gather
 
 // Staged gather: one mbarrier per warp, completed by the bulk copies' bytes.
@@ -473,6 +474,17 @@ __device__ const uint2 nm_no_ranges[9] = {};  // the walk of a lane whose cell i
 constexpr int WALK_L1 = 0;      // range by range through L1, two candidates per step
 constexpr int WALK_STAGED = 1;  // range by range from shared memory filled by bulk copies
 constexpr int WALK_PACKED = 2;  // range by range through L1, packed f32x2 arithmetic
+constexpr int WALK_DEEP = 3;    // the packed walk with more loads in flight, for dense cells
+
+// Which of the packed walks a launch is for: a launch that is not for the grid
+// at hand returns at once.
+constexpr int GRID_ANY = 0, GRID_SPARSE = 1, GRID_DENSE = 2;
+
+// Cells of eight points and more on average take the deep walk: its first loads
+// of a range run four records ahead, which short ranges waste.  Normals of 5M
+// points at 32 per cell: 4590 us deep, 5230 us not; of 1.8M voxels at 4.4 per
+// cell: 327 us deep, 291 us not.
+__device__ __forceinline__ bool dense_cells(uint32_t n, uint64_t cells) { return n >= 8 * cells; }
 
 // Packed f32x2 arithmetic (sm_100): two IEEE round-to-nearest f32 operations
 // per instruction, component by component -- the same results as
@@ -506,6 +518,52 @@ __device__ __forceinline__ uint64_t f2_fma(uint64_t a, uint64_t b, uint64_t c) {
   return r;
 }
 
+// The packed walk's accumulators of one query: f32 partial moments and hits.
+struct PackedAcc {
+  uint64_t a01 = 0, a34 = 0, a78 = 0;  // (sx, sy), (sxx, syy), (sxz, syz)
+  float a2 = 0.f, a5 = 0.f, a6 = 0.f;  // sz, szz, sxy
+  uint32_t hits = 0;
+};
+
+// One candidate: the reference predicate ((dx^2 + dy^2) + dz^2 <= r^2,
+// kdtree.rs:544-549), whose d2 it returns, and the moments of a hit.
+__device__ __forceinline__ float packed_visit(PackedAcc &q, uint64_t cxy, float cz, uint64_t qxy,
+                                              float qz, float r2) {
+  const uint64_t dxy = f2_sub(cxy, qxy);
+  const uint64_t pxy = f2_mul(dxy, dxy);
+  float dx, dy, xx, yy;
+  f2_unpack(dxy, dx, dy);
+  f2_unpack(pxy, xx, yy);
+  const float dz = __fsub_rn(cz, qz);
+  const float zz = __fmul_rn(dz, dz);
+  const float d2 = __fadd_rn(__fadd_rn(xx, yy), zz);
+  if (d2 <= r2) {
+    ++q.hits;
+    q.a01 = f2_add(q.a01, dxy);
+    q.a34 = f2_add(q.a34, pxy);
+    q.a78 = f2_fma(dxy, f2_pack(dz, dz), q.a78);
+    q.a2 += dz;
+    q.a5 += zz;
+    q.a6 = fmaf(dx, dy, q.a6);
+  }
+  return d2;
+}
+
+// Folds the partial moments into the lane's FP64 sums (stride NM_THREADS).
+__device__ __forceinline__ void packed_flush(PackedAcc &q, double *sums) {
+  float v[9];
+  f2_unpack(q.a01, v[0], v[1]);
+  f2_unpack(q.a34, v[3], v[4]);
+  f2_unpack(q.a78, v[7], v[8]);
+  v[2] = q.a2;
+  v[5] = q.a5;
+  v[6] = q.a6;
+#pragma unroll
+  for (int k = 0; k < 9; ++k) sums[k * NM_THREADS] += double(v[k]);
+  q.a01 = q.a34 = q.a78 = 0;
+  q.a2 = q.a5 = q.a6 = 0.f;
+}
+
 // Covariance from moments about the query (S: sx sy sz sxx syy szz sxy sxz syz
 // over n points) and its smallest eigenpair, FP64.
 __device__ __forceinline__ Eig3 eig_from_moments(const double (&S)[9], uint32_t n) {
@@ -532,33 +590,165 @@ __device__ __forceinline__ Eig3 eig_from_moments_f32(const double (&S)[9], uint3
 }
 
 // The same neighbour set (the f32 predicate), with every moment term formed
-// and summed in FP64 -- used for near-degenerate covariances only.
-__device__ __noinline__ void moments_fp64(const float4 *pts, const uint2 *rg, float4 qp, float r2,
-                                          double (&S)[9]) {
+// and summed in FP64, in the walk's order; returns the hits.  Four candidate
+// loads are in flight: a lone lane's walk is a chain of their latencies.
+__device__ __forceinline__ uint32_t moments_fp64(const float4 *pts, const uint2 *rg, float4 qp,
+                                                 float r2, double (&S)[9]) {
 #pragma unroll
   for (int k = 0; k < 9; ++k) S[k] = 0.0;
+  uint32_t hits = 0;
+  auto visit = [&](const float4 c) {
+    const float fx = __fsub_rn(c.x, qp.x), fy = __fsub_rn(c.y, qp.y), fz = __fsub_rn(c.z, qp.z);
+    const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)), __fmul_rn(fz, fz));
+    if (!(d2 <= r2)) return;
+    ++hits;
+    const double dx = double(c.x) - double(qp.x);
+    const double dy = double(c.y) - double(qp.y);
+    const double dz = double(c.z) - double(qp.z);
+    S[0] += dx;
+    S[1] += dy;
+    S[2] += dz;
+    S[3] = __fma_rn(dx, dx, S[3]);
+    S[4] = __fma_rn(dy, dy, S[4]);
+    S[5] = __fma_rn(dz, dz, S[5]);
+    S[6] = __fma_rn(dx, dy, S[6]);
+    S[7] = __fma_rn(dx, dz, S[7]);
+    S[8] = __fma_rn(dy, dz, S[8]);
+  };
+#pragma unroll 1
   for (int r = 0; r < 9; ++r) {
     const uint2 range = rg[r];
-    for (uint32_t j = range.x; j < range.y; ++j) {
-      const float4 c = __ldg(pts + j);
-      const float fx = __fsub_rn(c.x, qp.x), fy = __fsub_rn(c.y, qp.y), fz = __fsub_rn(c.z, qp.z);
-      const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)), __fmul_rn(fz, fz));
-      if (!(d2 <= r2)) continue;
-      const double dx = double(c.x) - double(qp.x);
-      const double dy = double(c.y) - double(qp.y);
-      const double dz = double(c.z) - double(qp.z);
-      S[0] += dx;
-      S[1] += dy;
-      S[2] += dz;
-      S[3] += dx * dx;
-      S[4] += dy * dy;
-      S[5] += dz * dz;
-      S[6] += dx * dy;
-      S[7] += dx * dz;
-      S[8] += dy * dz;
+    uint32_t j = range.x;
+    for (; j + 4 <= range.y; j += 4) {
+      const float4 c0 = __ldg(pts + j), c1 = __ldg(pts + j + 1);
+      const float4 c2 = __ldg(pts + j + 2), c3 = __ldg(pts + j + 3);
+      visit(c0);
+      visit(c1);
+      visit(c2);
+      visit(c3);
+    }
+    for (; j < range.y; ++j) visit(__ldg(pts + j));
+  }
+  return hits;
+}
+
+// Where the normals kernels write, by original point index.
+struct NormalDst {
+  float *nx, *ny, *nz, *curv;
+  uint32_t *counts;  // may be null
+  float *cov;        // PlaneCov: six floats per point
+  float cov_eps;
+  uint32_t *refine;  // the list for k_normals_refine, up to one word per point
+};
+
+// One lane's share of the chain's counters, and their sum over the warp.
+struct NormalTally {
+  uint32_t valid = 0, invalid = 0, shell = 0, fp64 = 0;
+  __device__ __forceinline__ void flush(Control *ctl, uint32_t lane) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      valid += __shfl_xor_sync(FULL_MASK, valid, o);
+      invalid += __shfl_xor_sync(FULL_MASK, invalid, o);
+      shell += __shfl_xor_sync(FULL_MASK, shell, o);
+      fp64 += __shfl_xor_sync(FULL_MASK, fp64, o);
+    }
+    if (lane == 0) {  // one atomic per warp
+      if (valid) atomicAdd(&ctl->ncount.valid, (unsigned long long)valid);
+      if (invalid) atomicAdd(&ctl->ncount.invalid, (unsigned long long)invalid);
+      if (shell) atomicAdd(&ctl->ncount.shell, (unsigned long long)shell);
+      if (fp64) atomicAdd(&ctl->ncount.fp64, (unsigned long long)fp64);
     }
   }
+};
+
+// Neighbours a query counts (`hits` points by the predicate, itself among them
+// when it is finite) and whether it gets a normal.
+struct QueryCount {
+  uint32_t cnt, n_eff;
+  bool valid;
+};
+__device__ __forceinline__ QueryCount query_count(uint32_t hits, float4 qp,
+                                                  const NormalParamsDev &prm) {
+  QueryCount c;
+  const bool finite = isfinite(qp.x) && isfinite(qp.y) && isfinite(qp.z);
+  c.cnt = (finite && hits > 0) ? hits - 1 : 0;
+  c.n_eff = prm.include_self ? c.cnt + (finite ? 1 : 0) : c.cnt;
+  c.valid = prm.include_self ? (c.n_eff >= 3) : (c.cnt >= prm.min_neighbors && c.cnt > 0);
+  return c;
 }
+
+// Writes one query's outputs: e is its smallest eigenpair when it is valid.
+template <bool PlaneCov>
+__device__ __forceinline__ void write_query(const Eig3 &e, bool valid, float4 qp,
+                                            const NormalParamsDev &prm, uint32_t qidx,
+                                            const NormalDst &o) {
+  float ox, oy, oz, oc;
+  if (valid) {
+    // Orientation and normalisation in f32, as the reference computes them
+    // (orient_normal_towards_viewpoint, normal.rs:408-421, with Vec3::dot
+    // and Vec3::normalize, vec.rs:66-100): the unit eigenvector rounded to
+    // f32 moves by ~1e-7 rad at most, and the sign test matches the
+    // reference's own f32 test.
+    float v0 = float(e.v[0]), v1 = float(e.v[1]), v2 = float(e.v[2]);
+    if (!PlaneCov && prm.has_viewpoint) {
+      const float wx = __fsub_rn(prm.vp[0], qp.x);
+      const float wy = __fsub_rn(prm.vp[1], qp.y);
+      const float wz = __fsub_rn(prm.vp[2], qp.z);
+      const float dot = __fadd_rn(__fadd_rn(__fmul_rn(v0, wx), __fmul_rn(v1, wy)), __fmul_rn(v2, wz));
+      if (dot < 0.0f) {
+        v0 = -v0;
+        v1 = -v1;
+        v2 = -v2;
+      }
+    }
+    const float len =
+        sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(v0, v0), __fmul_rn(v1, v1)), __fmul_rn(v2, v2)));
+    ox = len != 0.0f ? v0 / len : v0;
+    oy = len != 0.0f ? v1 / len : v1;
+    oz = len != 0.0f ? v2 / len : v2;
+    const float sum = float(e.l0 + e.l1 + e.l2);
+    oc = sum > 0.0f ? float(e.l0) / sum : 0.0f;
+  } else {
+    // include_self: (0, 0, 1) (normals_grid.rs:129-132), turned toward the
+    // viewpoint as GpuNormalEstimator turns every normal (normal_gpu.rs:
+    // 63-70): the f32 dot with vp - q is fl(vp.z - q.z), negative exactly
+    // when vp.z < q.z.
+    const float nanv = __int_as_float(0x7fc00000);
+    ox = prm.include_self ? 0.0f : nanv;
+    oy = prm.include_self ? 0.0f : nanv;
+    oz = prm.include_self ? ((prm.has_viewpoint && prm.vp[2] < qp.z) ? -1.0f : 1.0f) : nanv;
+    oc = 0.0f;
+  }
+  if constexpr (PlaneCov) {
+    float *c6 = o.cov + size_t(qidx) * 6;
+    if (valid) {
+      // (ox, oy, oz) is the unit normal; I + (eps - 1) n n^T
+      const float s = o.cov_eps - 1.0f;
+      c6[0] = fmaf(s * ox, ox, 1.0f);
+      c6[1] = fmaf(s * oy, oy, 1.0f);
+      c6[2] = fmaf(s * oz, oz, 1.0f);
+      c6[3] = s * ox * oy;
+      c6[4] = s * ox * oz;
+      c6[5] = s * oy * oz;
+    } else {
+      c6[0] = o.cov_eps;
+      c6[1] = o.cov_eps;
+      c6[2] = o.cov_eps;
+      c6[3] = 0.0f;
+      c6[4] = 0.0f;
+      c6[5] = 0.0f;
+    }
+  } else {
+    o.nx[qidx] = ox;
+    o.ny[qidx] = oy;
+    o.nz[qidx] = oz;
+    o.curv[qidx] = oc;
+  }
+}
+
+// The list of queries k_normals leaves to k_normals_refine: the cell-sorted
+// position, with REFINE_SOLVE where the eigensolve is in FP64 as well.
+constexpr uint32_t REFINE_SOLVE = 1u << 31;
 
 // Radius normals.  One warp per 32 consecutive cell-sorted points, one query
 // per lane; the persistent warps claim these batches from a counter.  Each lane walks the 9 column ranges of its own cell (the 27-cell
@@ -598,26 +788,26 @@ __device__ __noinline__ void moments_fp64(const float4 *pts, const uint2 *rg, fl
 // walk reads through L1 instead; which one a context runs is a tuning choice
 // (srcu_set_neighbor_staging).
 template <bool CountShell, bool PlaneCov = false, int Walk = WALK_L1>
-__global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const float4 *pts,
+__global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_normals(Control *ctl, const float4 *pts,
                                                            const uint32_t *pt_cell,
                                                            const uint2 *ranges,
                                                            const uint64_t *cell_key, Batch bt,
                                                            const unsigned long long *count_dev,
-                                                           float *nx, float *ny, float *nz,
-                                                           float *curv, uint32_t *counts,
-                                                           float *cov, float cov_eps) {
+                                                           NormalDst o, int grid) {
   if (ld_relaxed_u32(&ctl->status)) return;
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t n = uint32_t(count_dev ? *count_dev : ctl->n_points);
   const uint64_t u_count = ctl->n_cells;
+  if (grid != GRID_ANY && dense_cells(n, u_count) != (grid == GRID_DENSE)) return;
   const uint32_t lb = ctl->ckey_bits;
   const uint32_t batches = (n + 31) / 32;
-  unsigned long long n_valid = 0, n_invalid = 0, n_shell = 0, n_fp64 = 0;
+  NormalTally tally;
   float4 *sbuf = nullptr;  // this warp's staging buffer (Staged)
   uint64_t *sbar = nullptr;
   uint32_t phase = 0;
   bool timed_out = false;
   constexpr bool Staged = Walk == WALK_STAGED;
+  constexpr bool Packed = Walk == WALK_PACKED || Walk == WALK_DEEP;
   if constexpr (Staged) {
     __shared__ float4 nm_stage[(NM_THREADS / 32) * NM_STAGE];
     __shared__ __align__(8) uint64_t nm_bar[NM_THREADS / 32];
@@ -626,6 +816,8 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
     if (lane == 0) nm_bar_init(sbar);
     __syncwarp();
   }
+
+  __shared__ double nm_sums[Packed ? 9 * NM_THREADS : 1];  // FP64 sums, one column a lane
 
   // Each warp claims its next batch of 32 queries from the chain's counter:
   // batches differ in cost (dense and sparse parts of a cloud), so claiming
@@ -644,11 +836,7 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
     bool bad = false;
     if (u >= u_count) {  // cannot happen for a consistent cell table
       atomicOr(&ctl->status, ST_INTERNAL);
-      if constexpr (Staged) {
-        bad = true;  // the lane stays for the warp's collectives and walks nothing
-      } else {
-        continue;
-      }
+      bad = true;  // the lane stays for the warp's collectives and walks nothing
     }
     uint32_t cb = 0;  // the query's cloud
     if (!bad && bt.clouds > 1 && lb < 64) cb = uint32_t(cell_key[u] >> lb);
@@ -780,51 +968,35 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
           walk([&](uint32_t j) { return __ldg(pts + j); }, range.x, range.y);
         }
       }
-    } else if constexpr (Walk == WALK_PACKED) {
+    } else if constexpr (Packed) {
       // The L1 walk's candidate order and flush points, with the predicate and
       // the moments in packed f32x2 arithmetic: the same IEEE operation on each
-      // half, so every result is bit-identical to WALK_L1's.
+      // half, so every result is bit-identical to WALK_L1's.  The walk waits on
+      // L2: a record's sector is shared by one other record only, so every two
+      // candidates miss L1.  So candidates are loaded a group ahead of the one
+      // being visited (the FP64 sums live in shared memory to make room), up to
+      // NM_OVERREAD records past a range's end.
       const uint64_t qxy = f2_pack(qp.x, qp.y);
-      uint64_t a01 = 0, a34 = 0, a78 = 0;  // (sx, sy), (sxx, syy), (sxz, syz)
-      float a2 = 0.f, a5 = 0.f, a6 = 0.f;  // sz, szz, sxy
-      auto pvisit = [&](const float4 c) {
-        // the reference predicate ((dx^2 + dy^2) + dz^2 <= r^2, kdtree.rs:544-549)
-        const uint64_t dxy = f2_sub(f2_pack(c.x, c.y), qxy);
-        const uint64_t pxy = f2_mul(dxy, dxy);
-        float dx, dy, xx, yy;
-        f2_unpack(dxy, dx, dy);
-        f2_unpack(pxy, xx, yy);
-        const float dz = __fsub_rn(c.z, qp.z);
-        const float zz = __fmul_rn(dz, dz);
-        const float d2 = __fadd_rn(__fadd_rn(xx, yy), zz);
-        if (d2 <= r2) {
-          hits += 1.f;
-          a01 = f2_add(a01, dxy);
-          a34 = f2_add(a34, pxy);
-          a78 = f2_fma(dxy, f2_pack(dz, dz), a78);
-          a2 += dz;
-          a5 += zz;
-          a6 = fmaf(dx, dy, a6);
-        }
-        if (CountShell && prm.count_shell && d2 != 0.f && fabsf(__fsub_rn(d2, r2)) <= shell_tol)
-          shell = 1;
+      PackedAcc acc;
+      double *sums = nm_sums + threadIdx.x;
+#pragma unroll
+      for (int k = 0; k < 9; ++k) sums[k * NM_THREADS] = 0.0;
+      float shell_min = 3.4e38f;  // least |d2 - r2|
+      auto visit1 = [&](const float4 &c) {
+        const float d2 = packed_visit(acc, f2_pack(c.x, c.y), c.z, qxy, qp.z, r2);
+        if (CountShell) shell_min = fminf(shell_min, fabsf(__fsub_rn(d2, r2)));
       };
-      auto pflush = [&]() {
-        float v0, v1, v3, v4, v7, v8;
-        f2_unpack(a01, v0, v1);
-        f2_unpack(a34, v3, v4);
-        f2_unpack(a78, v7, v8);
-        S[0] += double(v0);
-        S[1] += double(v1);
-        S[2] += double(a2);
-        S[3] += double(v3);
-        S[4] += double(v4);
-        S[5] += double(a5);
-        S[6] += double(a6);
-        S[7] += double(v7);
-        S[8] += double(v8);
-        a01 = a34 = a78 = 0;
-        a2 = a5 = a6 = 0.f;
+      auto taken = [&](uint32_t count) {  // after every two candidates and a last single one
+        since += count;
+        if (since >= NM_FLUSH) {
+          since = 0;
+          packed_flush(acc, sums);
+        }
+      };
+      auto visit2 = [&](const float4 &c0, const float4 &c1) {
+        visit1(c0);
+        visit1(c1);
+        taken(2);
       };
       uint2 next = rg[0];
 #pragma unroll 1
@@ -832,26 +1004,66 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
         const uint2 range = next;
         if (r < 8) next = rg[r + 1];  // the next column's range loads under this one
         uint32_t j = range.x;
-        for (; j + 2 <= range.y; j += 2) {  // two independent candidate loads per step
-          const float4 c0 = __ldg(pts + j);
-          const float4 c1 = __ldg(pts + j + 1);
-          pvisit(c0);
-          pvisit(c1);
-          since += 2;
-          if (since >= NM_FLUSH) {
-            since = 0;
-            pflush();
+        if (j >= range.y) continue;
+        if constexpr (Walk == WALK_DEEP) {  // two groups of four in turn
+          auto tail = [&](const float4 &c0, const float4 &c1, const float4 &c2) {
+            const uint32_t left = range.y - j;  // 0 to 3
+            if (left >= 2) visit2(c0, c1);
+            if (left & 1u) {
+              visit1(left == 1 ? c0 : c2);
+              taken(1);
+            }
+          };
+          float4 a0 = __ldg(pts + j), a1 = __ldg(pts + j + 1);
+          float4 a2 = __ldg(pts + j + 2), a3 = __ldg(pts + j + 3);
+          for (;;) {
+            if (j + 4 > range.y) {
+              tail(a0, a1, a2);
+              break;
+            }
+            const float4 b0 = __ldg(pts + j + 4), b1 = __ldg(pts + j + 5);
+            const float4 b2 = __ldg(pts + j + 6), b3 = __ldg(pts + j + 7);
+            visit2(a0, a1);
+            visit2(a2, a3);
+            j += 4;
+            if (j + 4 > range.y) {
+              tail(b0, b1, b2);
+              break;
+            }
+            a0 = __ldg(pts + j + 4), a1 = __ldg(pts + j + 5);
+            a2 = __ldg(pts + j + 6), a3 = __ldg(pts + j + 7);
+            visit2(b0, b1);
+            visit2(b2, b3);
+            j += 4;
           }
-        }
-        if (j < range.y) {
-          pvisit(__ldg(pts + j));
-          if (++since >= NM_FLUSH) {
-            since = 0;
-            pflush();
+        } else {  // two pairs in turn
+          float4 c0 = __ldg(pts + j), c1 = __ldg(pts + j + 1);
+          for (; j + 4 <= range.y; j += 4) {
+            const float4 d0 = __ldg(pts + j + 2), d1 = __ldg(pts + j + 3);
+            visit2(c0, c1);
+            c0 = __ldg(pts + j + 4);
+            c1 = __ldg(pts + j + 5);
+            visit2(d0, d1);
+          }
+          if (j + 2 <= range.y) {
+            const float4 d0 = __ldg(pts + j + 2);
+            visit2(c0, c1);
+            c0 = d0;
+            j += 2;
+          }
+          if (j < range.y) {
+            visit1(c0);
+            taken(1);
           }
         }
       }
-      pflush();
+      packed_flush(acc, sums);
+      hits = float(acc.hits);
+#pragma unroll
+      for (int k = 0; k < 9; ++k) S[k] = sums[k * NM_THREADS];
+      // on the shell: d2 != 0 and |d2 - r2| <= tol; d2 = 0 is within tol of r2 only
+      // at r2 = 0, where no other d2 is
+      if (CountShell && prm.count_shell && r2 > 0.f && shell_min <= shell_tol) shell = 1;
     } else {
       uint2 next = rg[0];
 #pragma unroll 1
@@ -880,113 +1092,58 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
         }
       }
     }
-#pragma unroll
-    for (int k = 0; k < 9; ++k) S[k] += double(F[k]);
-    if (!active || bad) continue;
-    // hits includes the query itself exactly once when it is finite.
-    const bool finite = isfinite(qp.x) && isfinite(qp.y) && isfinite(qp.z);
-    const uint32_t h = uint32_t(hits);
-    const uint32_t cnt = (finite && h > 0) ? h - 1 : 0;
-    const uint32_t n_eff = prm.include_self ? cnt + (finite ? 1 : 0) : cnt;
-    const bool valid = prm.include_self ? (n_eff >= 3) : (cnt >= prm.min_neighbors && cnt > 0);
-    float ox, oy, oz, oc;
-    if (valid) {
-      // The f32 moments carry ~1e-7 of E|d|^2 in rounding (d = p - q, about
-      // the query), and the covariance E[d d^T] - E[d] E[d]^T inherits it
-      // whole: where the neighbours' mean lies far from the query against
-      // their spread (|E[d]|^2 > NM_REFINE_MEAN E|d|^2, so the trace is under
-      // an eighth of E|d|^2) that is too much of the trace for the curvature
-      // and, over a small gap, for the normal, so the moments are recomputed
-      // with FP64 products (same neighbour set) and solved again in FP32.
-      // The FP32 solve carries ~6e-8 of the trace; where the gap to the
-      // second eigenvalue is under NM_REFINE_GAP of the trace the normal can
-      // tilt by more than 1e-5 rad, and the point is solved in FP64 from FP64
-      // moments.  One call site for the FP64 walk keeps the common path lean.
-      const double inv_n = __drcp_rn(double(n_eff));
-      const double e2 = (S[3] + S[4] + S[5]) * inv_n;
-      const double m2 = (S[0] * S[0] + S[1] * S[1] + S[2] * S[2]) * (inv_n * inv_n);
-      const bool exact_moments = !(m2 <= NM_REFINE_MEAN * e2);
-      Eig3 e = eig_from_moments_f32(S, n_eff);
-      const bool small_gap = !(e.l1 - e.l0 >= NM_REFINE_GAP * (e.l0 + e.l1 + e.l2));
-      if (exact_moments || small_gap) {
-        moments_fp64(pts, rg, qp, r2, S);
-        if (small_gap) {
-          e = eig_from_moments(S, n_eff);
-          ++n_fp64;
-        } else {
-          e = eig_from_moments_f32(S, n_eff);
-        }
-      }
-      // Orientation and normalisation in f32, as the reference computes them
-      // (orient_normal_towards_viewpoint, normal.rs:408-421, with Vec3::dot
-      // and Vec3::normalize, vec.rs:66-100): the unit eigenvector rounded to
-      // f32 moves by ~1e-7 rad at most, and the sign test matches the
-      // reference's own f32 test.
-      float v0 = float(e.v[0]), v1 = float(e.v[1]), v2 = float(e.v[2]);
-      if (!PlaneCov && prm.has_viewpoint) {
-        const float wx = __fsub_rn(prm.vp[0], qp.x);
-        const float wy = __fsub_rn(prm.vp[1], qp.y);
-        const float wz = __fsub_rn(prm.vp[2], qp.z);
-        const float dot = __fadd_rn(__fadd_rn(__fmul_rn(v0, wx), __fmul_rn(v1, wy)), __fmul_rn(v2, wz));
-        if (dot < 0.0f) {
-          v0 = -v0;
-          v1 = -v1;
-          v2 = -v2;
-        }
-      }
-      const float len =
-          sqrtf(__fadd_rn(__fadd_rn(__fmul_rn(v0, v0), __fmul_rn(v1, v1)), __fmul_rn(v2, v2)));
-      ox = len != 0.0f ? v0 / len : v0;
-      oy = len != 0.0f ? v1 / len : v1;
-      oz = len != 0.0f ? v2 / len : v2;
-      const float sum = float(e.l0 + e.l1 + e.l2);
-      oc = sum > 0.0f ? float(e.l0) / sum : 0.0f;
-      ++n_valid;
-    } else {
-      // include_self: (0, 0, 1) (normals_grid.rs:129-132), turned toward the
-      // viewpoint as GpuNormalEstimator turns every normal (normal_gpu.rs:
-      // 63-70): the f32 dot with vp - q is fl(vp.z - q.z), negative exactly
-      // when vp.z < q.z.
-      const float nanv = __int_as_float(0x7fc00000);
-      ox = prm.include_self ? 0.0f : nanv;
-      oy = prm.include_self ? 0.0f : nanv;
-      oz = prm.include_self ? ((prm.has_viewpoint && prm.vp[2] < qp.z) ? -1.0f : 1.0f) : nanv;
-      oc = 0.0f;
-      ++n_invalid;
-    }
-    n_shell += shell;
+    if constexpr (!Packed) flush();
+    bool run = active && !bad;
     const uint32_t qidx = __float_as_uint(qp.w);
-    if (qidx >= n) {  // cannot happen: records carry indices < n
+    if (run && qidx >= n) {  // cannot happen: records carry indices < n
       atomicOr(&ctl->status, ST_INTERNAL);
-      continue;
+      run = false;
     }
-    if constexpr (PlaneCov) {
-      float *o = cov + size_t(qidx) * 6;
-      if (valid) {
-        // (ox, oy, oz) is the unit normal; I + (eps - 1) n n^T
-        const float s = cov_eps - 1.0f;
-        o[0] = fmaf(s * ox, ox, 1.0f);
-        o[1] = fmaf(s * oy, oy, 1.0f);
-        o[2] = fmaf(s * oz, oz, 1.0f);
-        o[3] = s * ox * oy;
-        o[4] = s * ox * oz;
-        o[5] = s * oy * oz;
+    uint32_t refine = 0;
+    if (run) {
+      const QueryCount c = query_count(uint32_t(hits), qp, prm);
+      Eig3 e;
+      bool exact_moments = false, small_gap = false;
+      if (c.valid) {
+        // The f32 moments carry ~1e-7 of E|d|^2 in rounding (d = p - q, about
+        // the query), and the covariance E[d d^T] - E[d] E[d]^T inherits it
+        // whole: where the neighbours' mean lies far from the query against
+        // their spread (|E[d]|^2 > NM_REFINE_MEAN E|d|^2, so the trace is under
+        // an eighth of E|d|^2) that is too much of the trace for the curvature
+        // and, over a small gap, for the normal, so the moments are recomputed
+        // with FP64 products (same neighbour set) and solved again in FP32.
+        // The FP32 solve carries ~6e-8 of the trace; where the gap to the
+        // second eigenvalue is under NM_REFINE_GAP of the trace the normal can
+        // tilt by more than 1e-5 rad, and the point is solved in FP64 from FP64
+        // moments.  Both are left to k_normals_refine.
+        const double inv_n = __drcp_rn(double(c.n_eff));
+        const double e2 = (S[3] + S[4] + S[5]) * inv_n;
+        const double m2 = (S[0] * S[0] + S[1] * S[1] + S[2] * S[2]) * (inv_n * inv_n);
+        exact_moments = !(m2 <= NM_REFINE_MEAN * e2);
+        e = eig_from_moments_f32(S, c.n_eff);
+        small_gap = !(e.l1 - e.l0 >= NM_REFINE_GAP * (e.l0 + e.l1 + e.l2));
+        ++tally.valid;
       } else {
-        o[0] = cov_eps;
-        o[1] = cov_eps;
-        o[2] = cov_eps;
-        o[3] = 0.0f;
-        o[4] = 0.0f;
-        o[5] = 0.0f;
+        ++tally.invalid;
       }
-      if (counts) counts[qidx] = n_eff;
-      continue;
+      tally.shell += shell;
+      if (o.counts) o.counts[qidx] = PlaneCov ? c.n_eff : (prm.include_self ? c.n_eff : c.cnt);
+      if (exact_moments || small_gap) {
+        refine = i | (small_gap ? REFINE_SOLVE : 0u);
+        if (small_gap) ++tally.fp64;
+      } else {
+        write_query<PlaneCov>(e, c.valid, qp, prm, qidx, o);
+      }
+      exact_moments |= small_gap;
+      run = exact_moments;  // deferred
     }
-    nx[qidx] = ox;
-    ny[qidx] = oy;
-    nz[qidx] = oz;
-    curv[qidx] = oc;
-    if (counts) counts[qidx] = prm.include_self ? n_eff : cnt;
+    const uint32_t deferred = __ballot_sync(FULL_MASK, run);
+    if (deferred) {  // one atomic per warp
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&ctl->work[WK_REFINE], uint32_t(__popc(deferred)));
+      at = __shfl_sync(FULL_MASK, at, 0) + __popc(deferred & lanemask_lt());
+      if (run && at < n) o.refine[at] = refine;  // at < n: a query defers once
+    }
   }
   if constexpr (Staged) {
     if (timed_out) {  // a copy that was given up on may still land: wait for it, bounded
@@ -995,19 +1152,134 @@ __global__ void __launch_bounds__(NM_THREADS, 4) k_normals(Control *ctl, const f
       }
     }
   }
-  // one atomic per warp for the counters
+  tally.flush(ctl, lane);
+}
+
+// The queries k_normals left: FP64 moments over the same neighbour set, solved in
+// FP64 where the gap is small and in FP32 otherwise.  In k_normals, where they
+// are a few percent of the lanes but at least one in many warps, each of them
+// held its whole warp for the FP64 walk and solve, and their code cost the whole
+// kernel registers (batch of 14M points: 1990 us in one kernel; 1280 us and 230 us
+// here for the 628k points of this list).
+//
+// Long lists go one lane per query.  Short ones would leave most of the chip
+// idle behind a few lanes' chains of candidate loads, so there a warp takes its
+// few queries one after the other: the lanes test 32 candidates at a time and
+// nine of them add the hits' terms in the walk's order, the same operations in
+// the same order as one lane's.
+constexpr int RF_BLOCKS = 4;  // resident blocks per SM: 231 us of the batch's list, 296 at 2
+struct RefineWarp {
+  double hit[32][4];  // dx, dy, dz, 1 of a hit
+  double sums[32][9];
+  uint2 ranges[32][9];
+};
+
+template <bool PlaneCov>
+__global__ void __launch_bounds__(NM_THREADS, RF_BLOCKS) k_normals_refine(
+    Control *ctl, const float4 *pts, const uint32_t *pt_cell, const uint2 *ranges,
+    const uint64_t *cell_key, Batch bt, const unsigned long long *count_dev, NormalDst o) {
+  __shared__ RefineWarp rw[NM_THREADS / 32];
+  if (ld_relaxed_u32(&ctl->status)) return;
+  const uint32_t n = uint32_t(count_dev ? *count_dev : ctl->n_points);
+  const uint32_t count = min(ctl->work[WK_REFINE], n);
+  const uint64_t u_count = ctl->n_cells;
+  const uint32_t lb = ctl->ckey_bits;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t warps = gridDim.x * (NM_THREADS / 32);
+  const uint32_t warp = blockIdx.x * (NM_THREADS / 32) + (threadIdx.x >> 5);
+  const bool alone = count >= warps * 16;  // one lane per query
+  const uint32_t per = alone ? 32 : max(1u, min(32u, (count + warps - 1) / warps));
+  RefineWarp &sh = rw[threadIdx.x >> 5];
+  for (uint64_t first = uint64_t(warp) * per; first < count; first += uint64_t(warps) * per) {
+    const uint32_t mine = min(per, uint32_t(count - first));
+    const uint32_t w = lane < mine ? o.refine[first + lane] : 0u;
+    const uint32_t i = w & ~REFINE_SOLVE;
+    bool run = lane < mine;
+    const uint32_t u = run && i < n ? pt_cell[i] : 0xffffffffu;
+    const float4 qp = run && i < n ? pts[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t qidx = __float_as_uint(qp.w);
+    if (run && (u >= u_count || qidx >= n)) {  // cannot happen: k_normals checked both
+      atomicOr(&ctl->status, ST_INTERNAL);
+      run = false;
+    }
+    uint32_t cb = 0;  // the query's cloud
+    if (run && bt.clouds > 1 && lb < 64) cb = uint32_t(cell_key[u] >> lb);
+    if (cb >= bt.clouds) cb = 0;
+    const float r2 = bt.cplans[cb].r2;
+    double S[9];
+    uint32_t hits = 0;
+    if (alone) {
+      if (run) hits = moments_fp64(pts, ranges + size_t(u) * 9, qp, r2, S);
+    } else {
+      if (run) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    n_valid += __shfl_xor_sync(FULL_MASK, n_valid, o);
-    n_invalid += __shfl_xor_sync(FULL_MASK, n_invalid, o);
-    n_shell += __shfl_xor_sync(FULL_MASK, n_shell, o);
-    n_fp64 += __shfl_xor_sync(FULL_MASK, n_fp64, o);
-  }
-  if (lane == 0) {
-    if (n_valid) atomicAdd(&ctl->ncount.valid, n_valid);
-    if (n_invalid) atomicAdd(&ctl->ncount.invalid, n_invalid);
-    if (n_shell) atomicAdd(&ctl->ncount.shell, n_shell);
-    if (n_fp64) atomicAdd(&ctl->ncount.fp64, n_fp64);
+        for (int r = 0; r < 9; ++r) sh.ranges[lane][r] = ranges[size_t(u) * 9 + r];
+      }
+      __syncwarp();
+      // term k of lane k < 9: hit[ka] * hit[kb]
+      const uint32_t ka = lane < 3 ? lane : lane < 6 ? lane - 3 : lane == 8 ? 1 : 0;
+      const uint32_t kb = lane < 3 ? 3 : lane < 6 ? lane - 3 : lane == 6 ? 1 : 2;
+      for (uint32_t e = 0; e < mine; ++e) {
+        if (!__shfl_sync(FULL_MASK, run, e)) continue;
+        const float qx = __shfl_sync(FULL_MASK, qp.x, e), qy = __shfl_sync(FULL_MASK, qp.y, e);
+        const float qz = __shfl_sync(FULL_MASK, qp.z, e), rr = __shfl_sync(FULL_MASK, r2, e);
+        const uint2 range = lane < 9 ? sh.ranges[e][lane] : make_uint2(0, 0);
+        uint32_t total;
+        const uint32_t before = warp_exclusive_sum(range.y - range.x, &total);
+        double sum = 0.0;
+        uint32_t found = 0;
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+          // candidate t of the nine ranges laid end to end
+          const uint32_t t = t0 + lane;
+          uint32_t j = 0;
+#pragma unroll
+          for (int r = 0; r < 9; ++r) {
+            const uint32_t at = __shfl_sync(FULL_MASK, before, r);
+            const uint32_t start = __shfl_sync(FULL_MASK, range.x, r);
+            if (t >= at) j = start + (t - at);
+          }
+          bool hit = t < total;
+          float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (hit) {
+            c = __ldg(pts + j);
+            const float fx = __fsub_rn(c.x, qx), fy = __fsub_rn(c.y, qy), fz = __fsub_rn(c.z, qz);
+            hit = __fadd_rn(__fadd_rn(__fmul_rn(fx, fx), __fmul_rn(fy, fy)), __fmul_rn(fz, fz)) <= rr;
+          }
+          const uint32_t mask = __ballot_sync(FULL_MASK, hit);
+          if (hit) {
+            double *h = sh.hit[__popc(mask & lanemask_lt())];
+            h[0] = double(c.x) - double(qx);
+            h[1] = double(c.y) - double(qy);
+            h[2] = double(c.z) - double(qz);
+            h[3] = 1.0;
+          }
+          __syncwarp();
+          const uint32_t nh = __popc(mask);
+#pragma unroll 4
+          for (uint32_t m = 0; m < nh; ++m) sum = __fma_rn(sh.hit[m][ka], sh.hit[m][kb], sum);
+          found += nh;
+          __syncwarp();
+        }
+        if (lane < 9) sh.sums[e][lane] = sum;
+        if (lane == e) hits = found;
+      }
+      __syncwarp();
+      if (run) {
+#pragma unroll
+        for (int k = 0; k < 9; ++k) S[k] = sh.sums[lane][k];
+      }
+      __syncwarp();
+    }
+    if (!run) continue;
+    const NormalParamsDev prm = bt.nparams[cb];
+    const QueryCount c = query_count(hits, qp, prm);
+    Eig3 e;
+    if (w & REFINE_SOLVE) {
+      e = eig_from_moments(S, c.n_eff);
+    } else {
+      e = eig_from_moments_f32(S, c.n_eff);
+    }
+    write_query<PlaneCov>(e, c.valid, qp, prm, qidx, o);
   }
 }
 

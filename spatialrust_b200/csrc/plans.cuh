@@ -175,6 +175,7 @@ constexpr int WK_CELLS = 24;
 constexpr int WK_NORMALS = 25;
 constexpr int WK_RANGES = 26;
 constexpr int WK_BOUNDS = 27;  // blocks of k_bounds that are done
+constexpr int WK_REFINE = 28;  // queries listed for k_normals_refine
 constexpr int WK_ORDER = 32;  // 4 slots
 
 __device__ __forceinline__ int64_t rs_sat_i64(float t) {

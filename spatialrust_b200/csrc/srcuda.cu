@@ -55,7 +55,8 @@ struct srcu_ctx {
   cudaStream_t side_stream = nullptr;
   cudaEvent_t ev_voxel = nullptr;
   unsigned char *head_host = nullptr;
-  int occ_normals = 1, occ_normals_staged = 1, occ_normals_packed = 1, occ_seg = 1, occ_cells = 1;
+  int occ_normals = 1, occ_normals_staged = 1, occ_normals_packed = 1, occ_normals_deep = 1;
+  int occ_seg = 1, occ_cells = 1;
   int neighbor_staging = 0;  // k_normals' neighbour walk: WALK_L1, WALK_STAGED or WALK_PACKED
   // co-resident blocks per SM of each sort launch shape, voxel-key and cell-key sorts
   int occ_sort_v[SORT_CONFIGS] = {}, occ_sort_c[SORT_CONFIGS] = {};
@@ -352,7 +353,7 @@ srcu_status reserve(srcu_ctx *ctx, uint64_t n, uint32_t cols, bool host_input, b
   }
   if (normals) {
     ST_TRY(ensure(ctx, ctx->lb_cells, size_t(ceil_div(m, CELL_TILE)) * 8, true));
-    ST_TRY(ensure(ctx, ctx->pts, m * 16));
+    ST_TRY(ensure(ctx, ctx->pts, (m + NM_OVERREAD) * 16));
     ST_TRY(ensure(ctx, ctx->pt_cell, m * 4));
     ST_TRY(ensure(ctx, ctx->cell_key, m * 8));
     ST_TRY(ensure(ctx, ctx->cell_start, (m + 1) * 4));
@@ -834,30 +835,54 @@ srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const fl
   return SRCU_OK;
 }
 
+// The normals kernels over the grid, in the context's neighbour walk.  raw: the
+// points are a caller's cloud, whose cells may be dense or not; voxel centroids
+// never fill a cell as the deep walk wants, so their chains do without it.
+template <bool Shell, bool PlaneCov>
+srcu_status launch_normals(srcu_ctx *ctx, const unsigned long long *count_dev, const Batch &bt,
+                           NormalDst dst, bool raw) {
+  Launch l(ctx, SRCU_K_NORMALS, 2);
+  const uint32_t sms = uint32_t(ctx->num_sms);
+  const float4 *pts = ptr<float4>(ctx->pts);
+  const uint32_t *pt_cell = ptr<uint32_t>(ctx->pt_cell);
+  const uint2 *ranges = ptr<uint2>(ctx->ranges);
+  const uint64_t *cell_key = ptr<uint64_t>(ctx->cell_key);
+  dst.refine = ptr<uint32_t>(ctx->vals[0]);  // the cell sort is consumed
+  auto kernel = k_normals<Shell, PlaneCov, WALK_L1>;
+  int occ = ctx->occ_normals, grid = GRID_ANY;
+  if (ctx->neighbor_staging == WALK_PACKED) {
+    kernel = k_normals<Shell, PlaneCov, WALK_PACKED>;
+    occ = ctx->occ_normals_packed;
+    if (raw) {
+      grid = GRID_SPARSE;
+      k_normals<Shell, PlaneCov, WALK_DEEP><<<sms * uint32_t(ctx->occ_normals_deep), NM_THREADS, 0,
+                                              ctx->stream>>>(ctx->ctl, pts, pt_cell, ranges,
+                                                             cell_key, bt, count_dev, dst,
+                                                             GRID_DENSE);
+    }
+  } else if (ctx->neighbor_staging == WALK_STAGED) {
+    if constexpr (!PlaneCov) {  // the covariances have no staged walk
+      kernel = k_normals<Shell, PlaneCov, WALK_STAGED>;
+      occ = ctx->occ_normals_staged;
+    }
+  }
+  kernel<<<sms * uint32_t(occ), NM_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, pt_cell, ranges,
+                                                              cell_key, bt, count_dev, dst, grid);
+  k_normals_refine<PlaneCov><<<sms * RF_BLOCKS, NM_THREADS, 0, ctx->stream>>>(
+      ctx->ctl, pts, pt_cell, ranges, cell_key, bt, count_dev, dst);
+  CU_TRY(cudaGetLastError());
+  return SRCU_OK;
+}
+
 srcu_status enqueue_normals(srcu_ctx *ctx, const float *x, const float *y, const float *z,
                             const float4 *aos, const unsigned long long *count_dev, uint64_t n_max,
                             const Batch &bt, const uint64_t *voxel_keys) {
   ST_TRY(enqueue_grid(ctx, x, y, z, aos, count_dev, n_max, bt, voxel_keys));
-  const uint32_t grid_n = uint32_t(ctx->num_sms) * uint32_t(ctx->occ_normals);
-  Launch l(ctx, SRCU_K_NORMALS);
-  const int walk = ctx->neighbor_staging;
-  auto kernel = walk == WALK_STAGED
-                    ? (ctx->count_shell ? k_normals<true, false, WALK_STAGED>
-                                        : k_normals<false, false, WALK_STAGED>)
-                : walk == WALK_PACKED
-                    ? (ctx->count_shell ? k_normals<true, false, WALK_PACKED>
-                                        : k_normals<false, false, WALK_PACKED>)
-                    : (ctx->count_shell ? k_normals<true> : k_normals<false>);
-  const uint32_t grid = walk == WALK_STAGED ? uint32_t(ctx->num_sms) * uint32_t(ctx->occ_normals_staged)
-                        : walk == WALK_PACKED ? uint32_t(ctx->num_sms) * uint32_t(ctx->occ_normals_packed)
-                                            : grid_n;
-  kernel<<<grid, NM_THREADS, 0, ctx->stream>>>(
-      ctx->ctl, ptr<float4>(ctx->pts), ptr<uint32_t>(ctx->pt_cell), ptr<uint2>(ctx->ranges),
-      ptr<uint64_t>(ctx->cell_key), bt, count_dev, ptr<float>(ctx->nout[0]),
-      ptr<float>(ctx->nout[1]), ptr<float>(ctx->nout[2]), ptr<float>(ctx->nout[3]),
-      ptr<uint32_t>(ctx->ncounts), nullptr, 0.0f);
-  CU_TRY(cudaGetLastError());
-  return SRCU_OK;
+  const NormalDst dst{ptr<float>(ctx->nout[0]), ptr<float>(ctx->nout[1]), ptr<float>(ctx->nout[2]),
+                      ptr<float>(ctx->nout[3]), ptr<uint32_t>(ctx->ncounts), nullptr, 0.0f,
+                      nullptr};
+  return ctx->count_shell ? launch_normals<true, false>(ctx, count_dev, bt, dst, !voxel_keys)
+                          : launch_normals<false, false>(ctx, count_dev, bt, dst, !voxel_keys);
 }
 
 // Keeps look-back and hash tags unique.  Every chain's k_begin advances the
@@ -1111,6 +1136,8 @@ srcu_status srcu_create(int device, uint64_t hbm_budget_bytes, srcu_ctx **out) {
                                                 k_normals<true, false, WALK_STAGED>, NM_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->occ_normals_packed,
                                                 k_normals<true, false, WALK_PACKED>, NM_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->occ_normals_deep,
+                                                k_normals<true, false, WALK_DEEP>, NM_THREADS, 0);
   ctx->neighbor_staging = kNeighborStaging;
   if (configure_segment_kernels() != cudaSuccess) return bail(SRCU_ERR_CUDA);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->occ_seg, k_voxel_segments<4>, SEG_THREADS,
@@ -1119,6 +1146,7 @@ srcu_status srcu_create(int device, uint64_t hbm_budget_bytes, srcu_ctx **out) {
   ctx->occ_normals = std::max(1, ctx->occ_normals);
   ctx->occ_normals_staged = std::max(1, ctx->occ_normals_staged);
   ctx->occ_normals_packed = std::max(1, ctx->occ_normals_packed);
+  ctx->occ_normals_deep = std::max(1, ctx->occ_normals_deep);
   ctx->occ_seg = std::max(1, ctx->occ_seg);
   ctx->occ_cells = std::max(1, ctx->occ_cells);
   if (cudaGetLastError() != cudaSuccess) return bail(SRCU_ERR_CUDA);
@@ -1405,16 +1433,9 @@ srcu_status srcu_plane_covariances(srcu_ctx *ctx, const srcu_cloud *cloud, float
   ST_TRY(enqueue_bounds(ctx, cols, 3, n, bt, false, true));
   ST_TRY(enqueue_grid(ctx, cols[0], cols[1], cols[2], ptr<const float4>(ctx->in_aos), nullptr, n,
                       bt, nullptr));
-  {
-    const bool flat = ctx->neighbor_staging == WALK_PACKED;
-    const uint32_t grid_n =
-        uint32_t(ctx->num_sms) * uint32_t(flat ? ctx->occ_normals_packed : ctx->occ_normals);
-    Launch l(ctx, SRCU_K_NORMALS);
-    (flat ? k_normals<false, true, WALK_PACKED> : k_normals<false, true>)<<<grid_n, NM_THREADS, 0, ctx->stream>>>(
-        ctx->ctl, ptr<float4>(ctx->pts), ptr<uint32_t>(ctx->pt_cell), ptr<uint2>(ctx->ranges),
-        ptr<uint64_t>(ctx->cell_key), bt, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr,
-        dst, epsilon);
-  }
+  ST_TRY((launch_normals<false, true>(
+      ctx, nullptr, bt,
+      NormalDst{nullptr, nullptr, nullptr, nullptr, nullptr, dst, epsilon, nullptr}, true)));
   CU_TRY(cudaGetLastError());
   ST_TRY(read_control(ctx));
   if (!cloud->on_device) ST_TRY(copy_out(ctx, cov, dst, n * 24, 0));

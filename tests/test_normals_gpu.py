@@ -259,3 +259,68 @@ def test_column_hash_path_on_huge_extent(cuda_ctx):
     ref = oracle.brute_radius_counts(x, y, z, 0.5)
     assert np.array_equal(counts, ref)
     assert stats["valid_count"] + stats["invalid_count"] == len(x)
+
+
+@pytest.mark.parametrize("per_cell", [1, 2, 3, 7, 8, 40])
+@pytest.mark.parametrize("n", [1, 5, 33, 6000])
+def test_packed_walks_equal_the_plain_walk(cuda_ctx, n, per_cell):
+    """The packed walks (dense grids take the deep one) load candidates ahead
+    over every remainder of a range; neighbours, moments and so the normals are
+    bit-identical to the plain walk's, non-finite points included.  Covariances
+    come from separately compiled solves of the same moments: each eigenvector is
+    within 1e-6 rad, so the elements I + (eps - 1) n n^T agree within 2 * 2e-6 and
+    their own rounding."""
+    rng = np.random.default_rng(n * 64 + per_cell)
+    side = (n / per_cell) ** (1 / 2)
+    p = np.stack([rng.random(n) * side, rng.random(n) * side, rng.random(n) * 0.3], 1).astype(np.float32)
+    if n > 5:
+        p[3], p[4] = p[2], [np.nan, 0, 0]
+        p[5] = [np.inf, 0, 0]
+    x, y, z = np.ascontiguousarray(p.T)
+    got = {}
+    for walk in (2, 0):
+        cuda_ctx.set_neighbor_staging(walk)
+        *cols, stats = cuda_ctx.radius_normals(x, y, z, 1.0, 3, (0.0, 0.0, 9.0))
+        got[walk] = cols, stats, cuda_ctx.plane_covariances(x, y, z, 1.0, 1e-3)
+    cuda_ctx.set_neighbor_staging(-1)
+    assert got[2][1] == got[0][1]
+    for a, b in zip(got[2][0], got[0][0]):
+        assert np.array_equal(a, b, equal_nan=True)
+    assert np.abs(got[2][2] - got[0][2]).max() <= 5e-6
+
+
+@pytest.mark.parametrize("copies", [1, 60])
+def test_refined_queries_alone_and_in_long_lists(cuda_ctx, copies):
+    """Nearly collinear neighbourhoods are all solved from FP64 moments: a short
+    list of them by whole warps, a long one (60 clouds' worth) by single lanes,
+    with equal results; the FP64 oracle bounds both."""
+    import torch
+    from spatialrust_b200 import _native
+    rng = np.random.default_rng(8)
+    n = 2500
+    p = np.stack([np.arange(n) * 0.21, rng.normal(0, 0.01, n), rng.normal(0, 0.01, n)], 1)
+    x, y, z = np.ascontiguousarray(p.T.astype(np.float32))
+    ref = oracle.radius_normals_fp64(x, y, z, 1.0, 3, (0.0, 50.0, 100.0))
+    cols = [torch.from_numpy(np.tile(a, copies)).cuda() for a in (x, y, z)]
+    keep = _native._Keep()
+    cloud = _native.make_cloud(*cols, [], keep)
+    cuda_ctx.batch_voxel_normals_enqueue(cloud, [n * k for k in range(copies + 1)], [1e-4] * copies,
+                                         [1.0] * copies, 3, [(0.0, 50.0, 100.0)] * copies)
+    voff = cuda_ctx.batch_voxel_offsets()
+    assert np.array_equal(voff, n * np.arange(copies + 1))  # a voxel per point, in x order
+    out = cuda_ctx.frame_fetch(n * copies)
+    assert out["stats"]["fp64_eigensolves"] > 0.9 * n * copies
+    first = {k: out[k][:n] for k in ("nx", "ny", "nz", "curvature", "neighbor_counts")}
+    for k, v in first.items():
+        for c in range(1, copies):
+            assert np.array_equal(out[k][c * n:(c + 1) * n], v, equal_nan=True), (k, c)
+    assert np.array_equal(first["neighbor_counts"], ref.counts)
+    g = np.stack([first[k] for k in ("nx", "ny", "nz")], 1).astype(np.float64)
+    well = ref.gap >= 1e-3
+    err = np.linalg.norm(np.cross(g, ref.normals), axis=1)[well]
+    assert err.max() <= 1e-4
+    if copies > 1:  # and equal to the one cloud on its own
+        alone = cuda_ctx.voxel_normals(x, y, z, [], leaf=1e-4, radius=1.0,
+                                       viewpoint=(0.0, 50.0, 100.0))
+        for k, v in first.items():
+            assert np.array_equal(alone[k], v, equal_nan=True), k

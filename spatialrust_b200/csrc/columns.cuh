@@ -17,20 +17,21 @@ struct TakeColumns {
   uint32_t count;
 };
 
-// Copies the first *rows rows of every column; blockIdx.y names the column.
-// The row count is read on the device, so the copies follow the chain without
+// Copies the first rows of every column, *rows of them or, with rows null, count;
+// blockIdx.y names the column.  A chain's row count is read on the device, so the copies follow the chain without
 // waiting for the host to learn it, and one launch takes them all, where a copy
 // per column after the wait left the GPU idle for its launch latency ten times
 // (call and fetch of a 131k-point frame 250 -> 212 us; of a 2M-point scan with
 // seven columns 578 -> 478 us).  Memory-bound at large sizes, hence the 16-byte
 // accesses where both ends are aligned.
 __global__ void __launch_bounds__(TAKE_THREADS) k_take_columns(const Control *ctl, TakeColumns t,
-                                                               const unsigned long long *rows) {
-  if (ctl->status) return;
+                                                               const unsigned long long *rows,
+                                                               unsigned long long count) {
+  if (rows && ctl->status) return;
   const uint32_t c = blockIdx.y;
   const uint32_t *src = t.src[c];
   uint32_t *dst = t.dst[c];
-  const uint64_t n = *rows * t.words[c];
+  const uint64_t n = (rows ? *rows : count) * t.words[c];
   const uint64_t stride = uint64_t(gridDim.x) * TAKE_THREADS;
   uint64_t i = blockIdx.x * uint64_t(TAKE_THREADS) + threadIdx.x;
   uint64_t done = 0;

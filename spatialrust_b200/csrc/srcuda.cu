@@ -343,7 +343,7 @@ srcu_status reserve(srcu_ctx *ctx, uint64_t n, uint32_t cols, bool host_input, b
   // (lookback_fits), so this covers every shape up to one tile's rounding.
   ST_TRY(ensure(ctx, ctx->lb_sort,
                 (size_t(ceil_div(m, SORT_MIN_TILE)) * RADIX_BINS + MAX_RADIX_BINS) * 8, true));
-  ST_TRY(ensure(ctx, ctx->in_aos, m * 16));
+  if (voxel || normals) ST_TRY(ensure(ctx, ctx->in_aos, m * 16));
   if (voxel) {
     ST_TRY(ensure(ctx, ctx->vaos, m * 16));
     ST_TRY(ensure(ctx, ctx->lb_seg, size_t(ceil_div(m, SEG_TILE)) * 8, true));
@@ -1003,12 +1003,26 @@ bool takable(const srcu_ctx *ctx, const DevBuf &b, uint32_t words = 1) {
   return b.p && b.bytes >= size_t(ctx->last_points) * words * 4;
 }
 
-void take_column(const srcu_ctx *ctx, TakeColumns &t, void *dst, const DevBuf &src,
-                 uint32_t words = 1) {
-  if (!dst || !takable(ctx, src, words)) return;
-  t.src[t.count] = static_cast<const uint32_t *>(src.p);
+void take_column(TakeColumns &t, void *dst, const void *src, uint32_t words) {
+  if (!dst) return;
+  t.src[t.count] = static_cast<const uint32_t *>(src);
   t.dst[t.count] = static_cast<uint32_t *>(dst);
   t.words[t.count++] = words;
+}
+
+void take_result(const srcu_ctx *ctx, TakeColumns &t, void *dst, const DevBuf &src,
+                 uint32_t words = 1) {
+  if (takable(ctx, src, words)) take_column(t, dst, src.p, words);
+}
+
+srcu_status take_columns(srcu_ctx *ctx, const TakeColumns &t, const unsigned long long *rows,
+                         uint64_t count) {
+  if (t.count == 0) return SRCU_OK;
+  // about eight blocks per SM over all columns; rows past the count cost nothing
+  const uint32_t blocks = std::max<uint32_t>(1, uint32_t(ctx->num_sms) * 8 / t.count);
+  k_take_columns<<<dim3(blocks, t.count), TAKE_THREADS, 0, ctx->stream>>>(ctx->ctl, t, rows, count);
+  CU_TRY(cudaGetLastError());
+  return SRCU_OK;
 }
 
 // Queues the copies of the chain's results that go to device memory, their
@@ -1020,21 +1034,16 @@ srcu_status take_results(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *vout,
   if (vout && vout->on_device) {
     float *dst[MAX_COLS] = {vout->x, vout->y, vout->z};
     for (uint32_t a = 3; a < nc; ++a) dst[a] = vout->attrs ? vout->attrs[a - 3] : nullptr;
-    for (uint32_t c = 0; c < nc; ++c) take_column(ctx, t, dst[c], ctx->vout[c]);
-    take_column(ctx, t, vout->counts, ctx->vcounts);
-    take_column(ctx, t, vout->keys, ctx->vkeys3, 6);
+    for (uint32_t c = 0; c < nc; ++c) take_result(ctx, t, dst[c], ctx->vout[c]);
+    take_result(ctx, t, vout->counts, ctx->vcounts);
+    take_result(ctx, t, vout->keys, ctx->vkeys3, 6);
   }
   if (nout && nout->on_device) {
     float *dst[4] = {nout->nx, nout->ny, nout->nz, nout->curvature};
-    for (int c = 0; c < 4; ++c) take_column(ctx, t, dst[c], ctx->nout[c]);
-    take_column(ctx, t, nout->neighbor_counts, ctx->ncounts);
+    for (int c = 0; c < 4; ++c) take_result(ctx, t, dst[c], ctx->nout[c]);
+    take_result(ctx, t, nout->neighbor_counts, ctx->ncounts);
   }
-  if (t.count == 0) return SRCU_OK;
-  // about eight blocks per SM over all columns; rows past the count cost nothing
-  const uint32_t blocks = std::max<uint32_t>(1, uint32_t(ctx->num_sms) * 8 / t.count);
-  k_take_columns<<<dim3(blocks, t.count), TAKE_THREADS, 0, ctx->stream>>>(ctx->ctl, t, rows);
-  CU_TRY(cudaGetLastError());
-  return SRCU_OK;
+  return take_columns(ctx, t, rows, 0);
 }
 
 // One result column of `rows` rows, unless take_results took it.

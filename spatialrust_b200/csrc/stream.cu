@@ -4,11 +4,12 @@
 //
 // Mirrors StreamingVoxelSource::try_build / next_chunk
 // (crates/spatialrust-pipeline/src/streaming.rs:414-535, 594-676):
-//   push()    appends a chunk to the device run buffer; a full buffer is a run:
+//   push()    packs a chunk into the device run buffer; a full buffer is a run:
 //             bounds -> plan -> onesweep sort -> segment reduction into partial
 //             records (key, count, compensated FP64 column sums);
 //   finish()  reduces the last run, checks the reference's run and spool
-//             limits, sorts every partial record by key and reduces again;
+//             limits, sorts every partial record by key and reduces again; the
+//             only run of a short stream is reduced into the outputs directly;
 //   fetch()   copies a window of the final voxels (next_chunk's chunks).
 #include "stream.cuh"
 
@@ -25,16 +26,19 @@ struct srcu_stream_voxel {
   uint64_t rec_cap = 0;
   uint64_t voxels = 0;
   bool finished = false;
-  int occ_point = 1, occ_record = 1;
-  DevBuf run[MAX_COLS];                       // run buffer, 4 or 8 bytes per element
+  StreamLayout lay{};
+  int occ_point[2] = {1, 1}, occ_record[2] = {1, 1};  // by kStreamSort shape
+  DevBuf run;                                  // run buffer: packed points
+  DevBuf stage[MAX_COLS];                      // columns of a host (or misaligned) chunk
   DevBuf rk[3], rcnt, rsum[MAX_COLS];          // partial records
-  DevBuf fk[3], fcnt, fsum[MAX_COLS];          // final records
-  DevBuf opos[3], oattr[MAX_COLS], okeys;      // finished outputs
+  DevBuf opos[3], oattr[MAX_COLS], okeys, ocnt; // finished outputs
   DevBuf tile_heads, tile_off, long_list, plan, state;
   StreamState *state_host = nullptr;           // pinned
 };
 
 namespace {
+
+constexpr uint64_t kStreamStage = uint64_t(1) << 20;  // points of a chunk staged at a time
 
 uint32_t sv_elem(const srcu_stream_voxel *sv, uint32_t c) {
   return (c >= 3 && ((sv->prm.attr_f64_mask >> (c - 3)) & 1u)) ? 8u : 4u;
@@ -66,20 +70,68 @@ srcu_status sv_reserve_records(srcu_stream_voxel *sv, uint64_t need) {
   return SRCU_OK;
 }
 
-StreamOut sv_out(DevBuf (&k)[3], DevBuf &cnt, DevBuf *sum, uint32_t nc, uint64_t base, uint64_t cap) {
+// The f64 columns first, then the f32 ones in pairs, in 16-byte units.
+void sv_layout(srcu_stream_voxel *sv) {
+  StreamLayout &l = sv->lay;
+  l = StreamLayout{};
+  l.nc = sv->nc;
+  for (uint32_t c = 0; c < sv->nc; ++c)
+    if (sv_elem(sv, c) == 8) l.col_d[l.nd++] = c;
+    else l.col_f[l.nf++] = c;
+  l.units = (l.nd + (l.nf + 1) / 2 + 1) / 2;
+}
+
+StreamOut sv_partial_out(srcu_stream_voxel *sv) {
   StreamOut o{};
-  o.kx = ptr<long long>(k[0]);
-  o.ky = ptr<long long>(k[1]);
-  o.kz = ptr<long long>(k[2]);
-  o.cnt = ptr<unsigned long long>(cnt);
-  for (uint32_t c = 0; c < nc; ++c) o.sum[c] = ptr<double>(sum[c]);
-  o.base = base;
-  o.cap = cap;
+  o.kx = ptr<long long>(sv->rk[0]);
+  o.ky = ptr<long long>(sv->rk[1]);
+  o.kz = ptr<long long>(sv->rk[2]);
+  o.cnt = ptr<unsigned long long>(sv->rcnt);
+  for (uint32_t c = 0; c < sv->nc; ++c) o.sum[c] = ptr<double>(sv->rsum[c]);
+  o.base = sv->records;
+  o.cap = sv->rec_cap;
   return o;
 }
 
+// The outputs, for up to r voxels.
+srcu_status sv_final_out(srcu_stream_voxel *sv, uint64_t r, StreamOut &o) {
+  srcu_ctx *ctx = sv->ctx;
+  for (int a = 0; a < 3; ++a) ST_TRY(ensure(ctx, sv->opos[a], r * 4));
+  for (uint32_t c = 3; c < sv->nc; ++c) ST_TRY(ensure(ctx, sv->oattr[c], r * 8));
+  ST_TRY(ensure(ctx, sv->okeys, r * 24));
+  ST_TRY(ensure(ctx, sv->ocnt, r * 8));
+  o = StreamOut{};
+  for (int a = 0; a < 3; ++a) o.pos[a] = ptr<float>(sv->opos[a]);
+  for (uint32_t c = 3; c < sv->nc; ++c) o.attr[c - 3] = ptr<double>(sv->oattr[c]);
+  o.keys3 = ptr<long long>(sv->okeys);
+  o.cnt = ptr<unsigned long long>(sv->ocnt);
+  o.cap = r;
+  return SRCU_OK;
+}
+
+// The streams' sorts run in two of the sort's launch shapes, as the voxel sort's
+// table has them: 8 keys per thread x 3 blocks of 256 threads up to 441k keys, 8 x 2
+// x 512 with 9-bit digits above (16 x 2 x 256, used for all before: 4.2M points
+// 238 us, 205 us here).
+constexpr int kStreamSort[2] = {1, 6};
+constexpr uint64_t kStreamSortSmall = 441000;
+
+template <class Src>
+srcu_status sv_sort(srcu_stream_voxel *sv, const Src &src, uint64_t n, const int (&occ)[2]) {
+  srcu_ctx *ctx = sv->ctx;
+  Launch l(ctx, SRCU_K_VOXEL_SORT);
+  const SortBuffers sb = sort_buffers(ctx);
+  const bool large = n > kStreamSortSmall;
+  const uint32_t cap = uint32_t(ctx->num_sms) * uint32_t(occ[large]);
+  CU_TRY((large ? launch_sort_config<Src, kStreamSort[1]>
+                : launch_sort_config<Src, kStreamSort[0]>)(ctx->stream, cap, src, ctx->ctl,
+                                                           ctx->ctl->hist_v, sb, EP_VSORT, WK_VSORT,
+                                                           &ctx->ctl->vsort, n));
+  return SRCU_OK;
+}
+
 // Segment reduction of the current sort (ctl->n_points = n sorted items).
-template <bool Records>
+template <bool Records, bool Final>
 srcu_status sv_reduce(srcu_stream_voxel *sv, uint64_t n, const StreamIn &in, const StreamOut &out,
                       int count_finite) {
   srcu_ctx *ctx = sv->ctx;
@@ -98,10 +150,10 @@ srcu_status sv_reduce(srcu_stream_voxel *sv, uint64_t n, const StreamIn &in, con
                                                        count_finite);
   k_stream_scan<<<1, 1024, 0, ctx->stream>>>(ctx->ctl, ptr<const uint32_t>(sv->tile_heads),
                                              ptr<uint32_t>(sv->tile_off), st);
-  k_stream_emit<Records><<<grid, SV_THREADS, 0, ctx->stream>>>(
+  k_stream_emit<Records, Final><<<grid, SV_THREADS, 0, ctx->stream>>>(
       ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, pl, ptr<const uint32_t>(sv->tile_off), in, out,
       st, ptr<ulonglong2>(sv->long_list), uint32_t(std::min<uint64_t>(long_cap, 0xffffffffu)));
-  k_stream_long<Records><<<uint32_t(ctx->num_sms) * 2, SV_THREADS, 0, ctx->stream>>>(
+  k_stream_long<Records, Final><<<uint32_t(ctx->num_sms) * 2, SV_THREADS, 0, ctx->stream>>>(
       ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, pl, in, out, st,
       ptr<const ulonglong2>(sv->long_list));
   CU_TRY(cudaGetLastError());
@@ -124,24 +176,30 @@ srcu_status sv_sync(srcu_stream_voxel *sv) {
   return s;
 }
 
-// Sorts and reduces the run buffer into partial records.
+// Sorts and reduces the run buffer into partial records, or, as the stream's only
+// run, into the outputs.
+template <bool Final>
 srcu_status sv_flush(srcu_stream_voxel *sv) {
   const uint64_t n = sv->fill;
   if (n == 0) return SRCU_OK;
   srcu_ctx *ctx = sv->ctx;
-  ST_TRY(sv_reserve_records(sv, sv->records + n));
+  StreamOut out{};
+  if (Final) {
+    ST_TRY(sv_final_out(sv, n, out));
+  } else {
+    ST_TRY(sv_reserve_records(sv, sv->records + n));
+    out = sv_partial_out(sv);
+  }
   ST_TRY(reserve(ctx, n, 0, false, false, false));
   ST_TRY(reserve_batch(ctx, 1));
   const Batch bt = make_batch(ctx, 1);
   ST_TRY(begin_chain(ctx, n, bt, 1, nullptr, nullptr));
-  const float *x = ptr<const float>(sv->run[0]);
-  const float *y = ptr<const float>(sv->run[1]);
-  const float *z = ptr<const float>(sv->run[2]);
+  const uint4 *points = ptr<const uint4>(sv->run);
   {
     Launch l(ctx, SRCU_K_BOUNDS);
     const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256),
-                                                                    uint32_t(ctx->num_sms) * 2));
-    k_stream_bounds<<<grid, 256, 0, ctx->stream>>>(ctx->ctl, x, y, z, bt.bounds);
+                                                                    uint32_t(ctx->num_sms) * 8));
+    k_stream_bounds<<<grid, 256, 0, ctx->stream>>>(ctx->ctl, points, sv->lay, bt.bounds);
   }
   {
     Launch l(ctx, SRCU_K_VOXEL_PLAN);
@@ -149,19 +207,15 @@ srcu_status sv_flush(srcu_stream_voxel *sv) {
                                              ptr<StreamPlan>(sv->plan), ptr<StreamState>(sv->state));
   }
   StreamPointSrc src{};
-  src.x = x;
-  src.y = y;
-  src.z = z;
+  src.points = points;
+  src.lay = sv->lay;
   src.plan_ptr = ptr<const StreamPlan>(sv->plan);
   src.leaf = sv->leaf;
-  ST_TRY(launch_sort(ctx, src, n, ctx->ctl->hist_v, EP_VSORT, WK_VSORT, &ctx->ctl->vsort,
-                     sv->occ_point, SRCU_K_VOXEL_SORT));
+  ST_TRY(sv_sort(sv, src, n, sv->occ_point));
   StreamIn in{};
-  in.nc = sv->nc;
-  in.f64_mask = sv->prm.attr_f64_mask << 3;
-  for (uint32_t c = 0; c < sv->nc; ++c) in.col[c] = sv->run[c].p;
-  ST_TRY(sv_reduce<false>(sv, n, in,
-                          sv_out(sv->rk, sv->rcnt, sv->rsum, sv->nc, sv->records, sv->rec_cap), 1));
+  in.points = points;
+  in.lay = sv->lay;
+  ST_TRY((sv_reduce<false, Final>(sv, n, in, out, 1)));
   ST_TRY(sv_sync(sv));
   sv->records += sv->state_host->segments;
   sv->device_runs += 1;
@@ -171,13 +225,12 @@ srcu_status sv_flush(srcu_stream_voxel *sv) {
 
 srcu_status sv_finish(srcu_stream_voxel *sv) {
   srcu_ctx *ctx = sv->ctx;
-  ST_TRY(sv_flush(sv));
+  const bool one_run = sv->device_runs == 0;
+  ST_TRY(one_run ? sv_flush<true>(sv) : sv_flush<false>(sv));
   // The reference spills every finite point into runs of run_points
   // (streaming.rs:458-485): its run count and spool extent follow from the
-  // finite-point count alone, and so do its two fail-closed limits.
-  CU_TRY(cudaMemcpyAsync(sv->state_host, sv->state.p, sizeof(StreamState), cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  CU_TRY(cudaStreamSynchronize(ctx->stream));
+  // finite-point count alone, and so do its two fail-closed limits.  (The
+  // last run's flush read the state back.)
   const uint64_t finite = sv->state_host->finite;
   const uint64_t runs = (finite + sv->prm.run_points - 1) / sv->prm.run_points;
   if (runs > sv->prm.max_runs)
@@ -193,13 +246,12 @@ srcu_status sv_finish(srcu_stream_voxel *sv) {
   if (r > LB_MAX_COUNT)
     return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "%llu partial voxel records exceed the merge limit %llu",
                 (unsigned long long)r, (unsigned long long)LB_MAX_COUNT);
-  // final records and outputs, r at most
-  for (int a = 0; a < 3; ++a) ST_TRY(ensure(ctx, sv->fk[a], r * 8));
-  ST_TRY(ensure(ctx, sv->fcnt, r * 8));
-  for (uint32_t c = 0; c < sv->nc; ++c) ST_TRY(ensure(ctx, sv->fsum[c], r * 8));
-  for (int a = 0; a < 3; ++a) ST_TRY(ensure(ctx, sv->opos[a], r * 4));
-  for (uint32_t c = 3; c < sv->nc; ++c) ST_TRY(ensure(ctx, sv->oattr[c], r * 8));
-  ST_TRY(ensure(ctx, sv->okeys, r * 24));
+  if (one_run) {
+    sv->voxels = r;
+    return SRCU_OK;
+  }
+  StreamOut out{};
+  ST_TRY(sv_final_out(sv, r, out));
   ST_TRY(reserve(ctx, r, 0, false, false, false));
   ST_TRY(reserve_batch(ctx, 1));
   ST_TRY(begin_chain(ctx, r, make_batch(ctx, 1), 1, nullptr, nullptr));
@@ -213,25 +265,12 @@ srcu_status sv_finish(srcu_stream_voxel *sv) {
   src.ky = ptr<const long long>(sv->rk[1]);
   src.kz = ptr<const long long>(sv->rk[2]);
   src.plan_ptr = ptr<const StreamPlan>(sv->plan);
-  ST_TRY(launch_sort(ctx, src, r, ctx->ctl->hist_v, EP_VSORT, WK_VSORT, &ctx->ctl->vsort,
-                     sv->occ_record, SRCU_K_VOXEL_SORT));
+  ST_TRY(sv_sort(sv, src, r, sv->occ_record));
   StreamIn in{};
-  in.nc = sv->nc;
-  in.f64_mask = ~0u;
+  in.lay = sv->lay;
   in.cnt = ptr<const unsigned long long>(sv->rcnt);
-  for (uint32_t c = 0; c < sv->nc; ++c) in.col[c] = sv->rsum[c].p;
-  const StreamOut fin = sv_out(sv->fk, sv->fcnt, sv->fsum, sv->nc, 0, r);
-  ST_TRY(sv_reduce<true>(sv, r, in, fin, 0));
-  StreamFinal o{};
-  for (int a = 0; a < 3; ++a) o.pos[a] = ptr<float>(sv->opos[a]);
-  for (uint32_t c = 3; c < sv->nc; ++c) o.attr[c - 3] = ptr<double>(sv->oattr[c]);
-  o.keys3 = ptr<long long>(sv->okeys);
-  {
-    Launch l(ctx, SRCU_K_UNPACK_KEYS);
-    const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(r, 256),
-                                                                    uint32_t(ctx->num_sms) * 8));
-    k_stream_finalize<<<grid, 256, 0, ctx->stream>>>(ctx->ctl, fin, sv->nc, o);
-  }
+  for (uint32_t c = 0; c < sv->nc; ++c) in.sum[c] = ptr<const double>(sv->rsum[c]);
+  ST_TRY((sv_reduce<true, true>(sv, r, in, out, 0)));
   CU_TRY(cudaGetLastError());
   ST_TRY(sv_sync(sv));
   sv->voxels = sv->state_host->segments;
@@ -240,14 +279,12 @@ srcu_status sv_finish(srcu_stream_voxel *sv) {
 
 void sv_release(srcu_stream_voxel *sv) {
   srcu_ctx *ctx = sv->ctx;
-  for (auto &b : sv->run) release(ctx, b);
+  for (auto &b : sv->stage) release(ctx, b);
   for (auto &b : sv->rk) release(ctx, b);
   for (auto &b : sv->rsum) release(ctx, b);
-  for (auto &b : sv->fk) release(ctx, b);
-  for (auto &b : sv->fsum) release(ctx, b);
   for (auto &b : sv->opos) release(ctx, b);
   for (auto &b : sv->oattr) release(ctx, b);
-  DevBuf *rest[] = {&sv->rcnt, &sv->fcnt, &sv->okeys, &sv->tile_heads, &sv->tile_off,
+  DevBuf *rest[] = {&sv->run, &sv->rcnt, &sv->ocnt, &sv->okeys, &sv->tile_heads, &sv->tile_off,
                     &sv->long_list, &sv->plan, &sv->state};
   for (DevBuf *b : rest) release(ctx, *b);
 }
@@ -294,20 +331,13 @@ srcu_status srcu_stream_voxel_create(srcu_ctx *ctx, const srcu_stream_voxel_para
     stream_voxel_free(sv);
     return st;
   };
-  if (cudaFuncSetAttribute(k_sort<StreamPointSrc>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           sizeof(OnesweepSmem)) != cudaSuccess ||
-      cudaFuncSetAttribute(k_sort<StreamRecordSrc>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           sizeof(OnesweepSmem)) != cudaSuccess)
+  sv_layout(sv);
+  if (sort_config_setup<StreamPointSrc, kStreamSort[0]>(&sv->occ_point[0]) != cudaSuccess ||
+      sort_config_setup<StreamPointSrc, kStreamSort[1]>(&sv->occ_point[1]) != cudaSuccess ||
+      sort_config_setup<StreamRecordSrc, kStreamSort[0]>(&sv->occ_record[0]) != cudaSuccess ||
+      sort_config_setup<StreamRecordSrc, kStreamSort[1]>(&sv->occ_record[1]) != cudaSuccess)
     return bail(fail(ctx, SRCU_ERR_CUDA, "cannot configure the streaming sort kernels"));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sv->occ_point, k_sort<StreamPointSrc>, OS_THREADS,
-                                                sizeof(OnesweepSmem));
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sv->occ_record, k_sort<StreamRecordSrc>,
-                                                OS_THREADS, sizeof(OnesweepSmem));
-  sv->occ_point = std::max(1, sv->occ_point);
-  sv->occ_record = std::max(1, sv->occ_record);
-  srcu_status s = SRCU_OK;
-  for (uint32_t c = 0; c < sv->nc && s == SRCU_OK; ++c)
-    s = ensure(ctx, sv->run[c], sv->dev_run * sv_elem(sv, c));
+  srcu_status s = ensure(ctx, sv->run, sv->dev_run * sv->lay.units * 16);
   if (s == SRCU_OK) s = ensure(ctx, sv->plan, sizeof(StreamPlan));
   if (s == SRCU_OK) s = ensure(ctx, sv->state, sizeof(StreamState));
   if (s != SRCU_OK) return bail(s);
@@ -341,19 +371,34 @@ srcu_status srcu_stream_voxel_push(srcu_stream_voxel *sv, const srcu_cloud *chun
   CU_TRY(cudaSetDevice(ctx->device));
   const void *src[MAX_COLS] = {chunk->x, chunk->y, chunk->z};
   for (uint32_t a = 0; a < chunk->n_attrs; ++a) src[3 + a] = chunk->attrs[a];
+  // device columns are read where they are, unless one is not aligned to its elements
   const cudaMemcpyKind kind = chunk->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
+  bool in_place = chunk->on_device != 0;
+  for (uint32_t c = 0; c < sv->nc; ++c)
+    in_place = in_place && reinterpret_cast<uintptr_t>(src[c]) % sv_elem(sv, c) == 0;
   uint64_t done = 0;
   while (done < chunk->n) {
-    const uint64_t take = std::min<uint64_t>(chunk->n - done, sv->dev_run - sv->fill);
+    uint64_t take = std::min<uint64_t>(chunk->n - done, sv->dev_run - sv->fill);
+    if (!in_place) take = std::min(take, kStreamStage);
+    StreamChunk ch{};
     for (uint32_t c = 0; c < sv->nc; ++c) {
       const uint32_t e = sv_elem(sv, c);
-      CU_TRY(cudaMemcpyAsync(static_cast<char *>(sv->run[c].p) + sv->fill * e,
-                             static_cast<const char *>(src[c]) + done * e, take * e, kind,
-                             ctx->stream));
+      const char *from = static_cast<const char *>(src[c]) + done * e;
+      ch.col[c] = from;
+      if (in_place) continue;
+      ST_TRY(ensure(ctx, sv->stage[c], take * e));
+      if (take) CU_TRY(cudaMemcpyAsync(sv->stage[c].p, from, take * e, kind, ctx->stream));
+      ch.col[c] = sv->stage[c].p;
+    }
+    if (take) {
+      const uint32_t grid = std::min<uint32_t>(ceil_div(take, 256), uint32_t(ctx->num_sms) * 8);
+      k_stream_pack<<<grid, 256, 0, ctx->stream>>>(ch, sv->lay, take,
+                                                   ptr<uint4>(sv->run) + sv->fill * sv->lay.units);
+      CU_TRY(cudaGetLastError());
     }
     sv->fill += take;
     done += take;
-    if (sv->fill == sv->dev_run) ST_TRY(sv_flush(sv));
+    if (sv->fill == sv->dev_run) ST_TRY(sv_flush<false>(sv));
   }
   sv->points += chunk->n;
   CU_TRY(cudaStreamSynchronize(ctx->stream));  // the chunk's memory may be reused on return
@@ -394,15 +439,19 @@ srcu_status srcu_stream_voxel_fetch(srcu_stream_voxel *sv, uint64_t first, uint6
   if (count == 0) return SRCU_OK;
   CU_TRY(cudaSetDevice(ctx->device));
   float *pos[3] = {out->x, out->y, out->z};
-  for (int a = 0; a < 3; ++a)
-    ST_TRY(copy_out(ctx, pos[a], ptr<float>(sv->opos[a]) + first, count * 4, out->on_device));
+  TakeColumns t{};
+  auto column = [&](void *dst, const DevBuf &src, uint32_t words) -> srcu_status {
+    const uint32_t *from = static_cast<const uint32_t *>(src.p) + first * words;
+    if (!out->on_device) return copy_out(ctx, dst, from, count * words * 4, 0);
+    take_column(t, dst, from, words);
+    return SRCU_OK;
+  };
+  for (int a = 0; a < 3; ++a) ST_TRY(column(pos[a], sv->opos[a], 1));
   for (uint32_t c = 3; c < sv->nc; ++c)
-    if (out->attrs && out->attrs[c - 3])
-      ST_TRY(copy_out(ctx, out->attrs[c - 3], ptr<double>(sv->oattr[c]) + first, count * 8,
-                      out->on_device));
-  ST_TRY(copy_out(ctx, out->keys, ptr<long long>(sv->okeys) + 3 * first, count * 24, out->on_device));
-  ST_TRY(copy_out(ctx, out->counts, ptr<unsigned long long>(sv->fcnt) + first, count * 8,
-                  out->on_device));
+    if (out->attrs) ST_TRY(column(out->attrs[c - 3], sv->oattr[c], 2));
+  ST_TRY(column(out->keys, sv->okeys, 6));
+  ST_TRY(column(out->counts, sv->ocnt, 2));
+  ST_TRY(take_columns(ctx, t, nullptr, count));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   return SRCU_OK;
 }

@@ -11,14 +11,20 @@
 //     whole stream, sum / count (:852-858, :631-633);
 //   - voxels come out in ascending (ix, iy, iz) order (:805-838).
 //
-// Device design.  Chunks fill a device run buffer.  A full run is sorted by
-// packed key with the onesweep sort (stable, so a voxel's points stay in
-// stream order) and reduced to partial records -- key, count and a
-// compensated FP64 sum of every column -- appended to a device record store.
-// finish() sorts all partial records by key (stable, so runs stay in stream
-// order) and reduces them again into the final records.  Only reduced runs
-// stay resident: device memory grows with the distinct voxels of each run,
-// not with the length of the stream.
+// Device design.  Chunks are packed into a device run buffer, one record per
+// point.  A full run is sorted by packed key with the onesweep sort (stable, so
+// a voxel's points stay in stream order) and reduced to partial records -- key,
+// count and a compensated FP64 sum of every column -- appended to a device
+// record store.  finish() sorts all partial records by key (stable, so runs stay
+// in stream order) and reduces them again, straight into the outputs; a stream
+// that fits one run is reduced into the outputs at once.  Only reduced runs stay
+// resident: device memory grows with the distinct voxels of each run, not with
+// the length of the stream.
+//
+// The reductions gather points in key order, which is random in the run buffer.
+// A packed record is one 32-byte sector for up to four f32 and two f64 columns,
+// where the columns apart cost a sector each (run reduction of 4.2M points of
+// three positions and two attributes: 580 us and 1.6 GB read; 193 us here).
 //
 // A voxel's sum is compensated (Kahan) within each run and across runs, as
 // the reference's CompensatedSum is over the whole stream (:240-262); the
@@ -58,20 +64,34 @@ struct StreamState {
   uint32_t pad;
 };
 
-// One reduction's inputs: f32 or f64 point columns (bit c of f64_mask), or
-// the partial records' FP64 sums and counts.
+// Packed point records: the f64 columns, then the f32 columns in pairs, padded
+// to 16-byte units.  The positions are the first three f32 columns.
+struct StreamLayout {
+  uint32_t nc, nd, nf;  // columns: all, f64, f32
+  uint32_t units;       // 16-byte units per record
+  uint32_t col_d[MAX_COLS], col_f[MAX_COLS];  // the column behind each f64 / f32 field
+};
+
+// One reduction's inputs: packed points, or the partial records' FP64 sums and
+// counts.
 struct StreamIn {
-  const void *col[MAX_COLS];
-  uint32_t nc;
-  uint32_t f64_mask;
+  const uint4 *points;
+  StreamLayout lay;
+  const double *sum[MAX_COLS];    // records only
   const unsigned long long *cnt;  // records only
 };
 
-// Record store (partial or final): SoA, written at base + slot < cap.
+// One reduction's outputs, written at base + slot < cap: the partial record
+// store (SoA), or with Final the stream's own -- positions as f32, the other
+// columns' means in FP64 (narrowed by the caller per field type, as push_scalar
+// does, streaming.rs:922-938), (ix, iy, iz) triples.
 struct StreamOut {
   long long *kx, *ky, *kz;
   unsigned long long *cnt;
   double *sum[MAX_COLS];
+  float *pos[3];
+  double *attr[MAX_COLS];
+  long long *keys3;
   unsigned long long base, cap;
 };
 
@@ -105,18 +125,49 @@ __device__ __forceinline__ bool finite3(float x, float y, float z) {
   return isfinite(x) && isfinite(y) && isfinite(z);
 }
 
+__device__ __forceinline__ float3 stream_pos(const uint4 *points, const StreamLayout &lay,
+                                             uint64_t i) {
+  const float *f = reinterpret_cast<const float *>(points + i * lay.units) + 2 * lay.nd;
+  return make_float3(f[0], f[1], f[2]);
+}
+
+// A chunk's columns -> packed records.
+struct StreamChunk {
+  const void *col[MAX_COLS];
+};
+__global__ void __launch_bounds__(256) k_stream_pack(const __grid_constant__ StreamChunk ch,
+                                                     const __grid_constant__ StreamLayout lay,
+                                                     uint64_t n, uint4 *points) {
+  for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
+       i += uint64_t(gridDim.x) * blockDim.x) {
+    auto pair = [&](uint32_t p) -> uint2 {  // 8 bytes: one f64 field or two f32 fields
+      uint2 w = make_uint2(0, 0);
+      if (p < lay.nd) return static_cast<const uint2 *>(ch.col[lay.col_d[p]])[i];
+      const uint32_t f = 2 * (p - lay.nd);
+      if (f < lay.nf) w.x = static_cast<const uint32_t *>(ch.col[lay.col_f[f]])[i];
+      if (f + 1 < lay.nf) w.y = static_cast<const uint32_t *>(ch.col[lay.col_f[f + 1]])[i];
+      return w;
+    };
+    for (uint32_t u = 0; u < lay.units; ++u) {
+      const uint2 a = pair(2 * u), b = pair(2 * u + 1);
+      points[i * lay.units + u] = make_uint4(a.x, a.y, b.x, b.y);
+    }
+  }
+}
+
 // Per-axis min/max over the points whose three coordinates are finite (the
 // points the stream keeps) of the current run (ctl->n_points of them):
 // warp then block reductions, six atomics per block.
-__global__ void __launch_bounds__(256) k_stream_bounds(Control *ctl, const float *x, const float *y,
-                                                       const float *z, Bounds *out) {
+__global__ void __launch_bounds__(256) k_stream_bounds(Control *ctl, const uint4 *points,
+                                                       StreamLayout lay, Bounds *out) {
   __shared__ uint32_t red[6][8];
   if (ld_relaxed_u32(&ctl->status)) return;
   const uint64_t n = ctl->n_points;
   uint32_t v6[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};  // mn xyz, mx xyz
   for (uint64_t i = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; i < n;
        i += uint64_t(gridDim.x) * blockDim.x) {
-    const float v[3] = {x[i], y[i], z[i]};
+    const float3 p = stream_pos(points, lay, i);
+    const float v[3] = {p.x, p.y, p.z};
     if (!finite3(v[0], v[1], v[2])) continue;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
@@ -209,7 +260,8 @@ __global__ void k_stream_merge_plan(Control *ctl, StreamPlan *plan, StreamState 
 
 // Sort key of a run's points (ctl->n_points of them).
 struct StreamPointSrc {
-  const float *x, *y, *z;
+  const uint4 *points;
+  StreamLayout lay;
   const StreamPlan *plan_ptr;
   double leaf;
   StreamPlan pl;
@@ -217,11 +269,11 @@ struct StreamPointSrc {
   __device__ __forceinline__ uint32_t count(const Control *ctl) const { return uint32_t(ctl->n_points); }
   __device__ __forceinline__ uint32_t key_bits() const { return pl.total_bits + 1; }
   __device__ __forceinline__ uint64_t key(uint32_t i) const {
-    const float px = x[i], py = y[i], pz = z[i];
+    const float3 p = stream_pos(points, lay, i);
     long long kx, ky, kz;
     // a finite point lies inside the run's bounds, so its keys are in range
-    if (!finite3(px, py, pz) || !stream_axis_key(px, leaf, kx) || !stream_axis_key(py, leaf, ky) ||
-        !stream_axis_key(pz, leaf, kz))
+    if (!finite3(p.x, p.y, p.z) || !stream_axis_key(p.x, leaf, kx) ||
+        !stream_axis_key(p.y, leaf, ky) || !stream_axis_key(p.z, leaf, kz))
       return 1ull << pl.total_bits;
     return stream_pack(pl, kx, ky, kz);
   }
@@ -306,12 +358,6 @@ __global__ void __launch_bounds__(1024) k_stream_scan(Control *ctl, const uint32
   }
 }
 
-template <bool Records>
-__device__ __forceinline__ double stream_value(const StreamIn &in, uint32_t c, uint32_t v) {
-  if (Records || ((in.f64_mask >> c) & 1u)) return static_cast<const double *>(in.col[c])[v];
-  return double(static_cast<const float *>(in.col[c])[v]);
-}
-
 // Compensated sum (Kahan): the running correction is subtracted from each
 // addend, as CompensatedSum::add does (streaming.rs:246-257).
 struct Kahan {
@@ -324,86 +370,164 @@ struct Kahan {
   }
 };
 
-// Writes the record of the voxel at sorted positions [i, j), reduced by one
-// thread in sorted order.
-template <bool Records>
-__device__ void stream_reduce_short(Control *ctl, const SortedView &sv, const StreamPlan &pl,
-                                    const StreamIn &in, const StreamOut &out, uint64_t key,
-                                    uint32_t i, uint32_t j, uint64_t slot) {
-  const uint64_t r = out.base + slot;
-  if (r >= out.cap) {
-    atomicOr(&ctl->status, ST_INTERNAL);
-    return;
-  }
+// Key and count of output record r; one column's sum, or its mean with Final.
+template <bool Final>
+__device__ __forceinline__ void stream_put_key(const StreamOut &out, const StreamPlan &pl,
+                                               uint64_t key, uint64_t r, unsigned long long cnt) {
   long long kx, ky, kz;
   stream_unpack(pl, key, kx, ky, kz);
-  out.kx[r] = kx;
-  out.ky[r] = ky;
-  out.kz[r] = kz;
-  if (j == i + 1) {
-    // one item (the common case): every column's value is its sum, and the
-    // column loads are independent, so they are all issued before any is used
-    const uint32_t v = sv.val(i);
-    out.cnt[r] = Records ? in.cnt[v] : 1ull;
-    for (uint32_t c0 = 0; c0 < in.nc; c0 += 4) {
-      double val[4];
+  if (Final) {
+    out.keys3[3 * r] = kx;
+    out.keys3[3 * r + 1] = ky;
+    out.keys3[3 * r + 2] = kz;
+  } else {
+    out.kx[r] = kx;
+    out.ky[r] = ky;
+    out.kz[r] = kz;
+  }
+  out.cnt[r] = cnt;
+}
+template <bool Final>
+__device__ __forceinline__ void stream_put(const StreamOut &out, uint32_t c, uint64_t r, double sum,
+                                           unsigned long long cnt) {
+  if (!Final) out.sum[c][r] = sum;
+  else if (c < 3) out.pos[c][r] = __double2float_rn(__ddiv_rn(sum, __ull2double_rn(cnt)));
+  else out.attr[c - 3][r] = __ddiv_rn(sum, __ull2double_rn(cnt));
+}
+
+// The fields of unit u of a packed point, in order: at most four, of which slot
+// 0 and 2 may be f64 (then slot 1 or 3 is empty).  visit(slot, column, value).
+template <class Visit>
+__device__ __forceinline__ void stream_fields(const StreamLayout &lay, uint32_t u, uint4 q,
+                                              Visit visit) {
 #pragma unroll
-      for (uint32_t k = 0; k < 4; ++k)
-        if (c0 + k < in.nc) val[k] = stream_value<Records>(in, c0 + k, v);
+  for (uint32_t h = 0; h < 2; ++h) {
+    const uint32_t p = 2 * u + h;
+    const uint32_t lo = h ? q.z : q.x, hi = h ? q.w : q.y;
+    if (p < lay.nd) {
+      visit(2 * h, lay.col_d[p], __hiloint2double(int(hi), int(lo)));
+    } else {
+      const uint32_t f = 2 * (p - lay.nd);
+      if (f < lay.nf) visit(2 * h, lay.col_f[f], double(__uint_as_float(lo)));
+      if (f + 1 < lay.nf) visit(2 * h + 1, lay.col_f[f + 1], double(__uint_as_float(hi)));
+    }
+  }
+}
+
+// A compensated sum that starts from its first value as it is; `more` when others
+// follow (they start from 0.0 + v, which differs for v = -0).
+__device__ __forceinline__ void stream_first(Kahan &k, double v, bool more) {
+  k.s = more ? __dadd_rn(0.0, v) : v;
+  k.c = 0.0;
+}
+
+// Reduces the voxel at sorted positions [i, j), one thread in sorted order, into
+// output record r; v is the item at i.  A warp's voxels hold one item or a few:
+// all lanes take their first item together, then loop over the rest, a group of
+// columns at a time.
+template <bool Records, bool Final>
+__device__ __forceinline__ void stream_reduce(const SortedView &sv, const StreamPlan &pl,
+                                              const StreamIn &in, const StreamOut &out,
+                                              uint64_t key, uint32_t i, uint32_t j, uint32_t v,
+                                              uint64_t r) {
+  const bool more = j > i + 1;
+  unsigned long long cnt = j - i;
+  if (Records) {
+    cnt = in.cnt[v];
+    for (uint32_t p = i + 1; p < j; ++p) cnt += in.cnt[sv.val(p)];
+  }
+  stream_put_key<Final>(out, pl, key, r, cnt);
+  if (Records) {
+    for (uint32_t c0 = 0; c0 < in.lay.nc; c0 += 4) {
+      double x[4];
+      Kahan k[4];
 #pragma unroll
-      for (uint32_t k = 0; k < 4; ++k)
-        if (c0 + k < in.nc) out.sum[c0 + k][r] = val[k];
+      for (uint32_t m = 0; m < 4; ++m)
+        if (c0 + m < in.lay.nc) x[m] = in.sum[c0 + m][v];
+#pragma unroll
+      for (uint32_t m = 0; m < 4; ++m)
+        if (c0 + m < in.lay.nc) stream_first(k[m], x[m], more);
+      for (uint32_t p = i + 1; p < j; ++p) {
+        const uint32_t w = sv.val(p);
+#pragma unroll
+        for (uint32_t m = 0; m < 4; ++m)
+          if (c0 + m < in.lay.nc) k[m].add(in.sum[c0 + m][w]);
+      }
+#pragma unroll
+      for (uint32_t m = 0; m < 4; ++m)
+        if (c0 + m < in.lay.nc) stream_put<Final>(out, c0 + m, r, k[m].s, cnt);
     }
     return;
   }
-  unsigned long long cnt = j - i;
-  if (Records) {
-    cnt = 0;
-    for (uint32_t p = i; p < j; ++p) cnt += in.cnt[sv.val(p)];
-  }
-  out.cnt[r] = cnt;
-  for (uint32_t c = 0; c < in.nc; ++c) {
-    Kahan k;
-    for (uint32_t p = i; p < j; ++p) k.add(stream_value<Records>(in, c, sv.val(p)));
-    out.sum[c][r] = k.s;
+  const uint32_t units = in.lay.units;
+  for (uint32_t u = 0; u < units; ++u) {
+    Kahan k[4];
+    stream_fields(in.lay, u, in.points[uint64_t(v) * units + u],
+                  [&](uint32_t s, uint32_t, double x) { stream_first(k[s], x, more); });
+    for (uint32_t p = i + 1; p < j; ++p)
+      stream_fields(in.lay, u, in.points[uint64_t(sv.val(p)) * units + u],
+                    [&](uint32_t s, uint32_t, double x) { k[s].add(x); });
+    stream_fields(in.lay, u, make_uint4(0, 0, 0, 0), [&](uint32_t s, uint32_t c, double) {
+      stream_put<Final>(out, c, r, k[s].s, cnt);
+    });
   }
 }
 
 // Records of the voxels that start in each tile: a voxel of at most SV_SHORT
 // positions is reduced by the thread holding its start; a longer one is
-// queued for k_stream_long.
-template <bool Records>
-__global__ void __launch_bounds__(SV_THREADS) k_stream_emit(Control *ctl, SortBuffers sort,
+// queued for k_stream_long.  Thread t owns positions t, t + 256, ... of the
+// tile, so that a warp's voxels, and what it writes, are consecutive.
+template <bool Records, bool Final>
+__global__ void __launch_bounds__(SV_THREADS, 4) k_stream_emit(Control *ctl,
+                                                            SortBuffers sort,
                                                             const SortState *ss,
                                                             const StreamPlan *plan,
-                                                            const uint32_t *tile_off, StreamIn in,
-                                                            StreamOut out, StreamState *st,
+                                                            const uint32_t *tile_off,
+                                                            const __grid_constant__ StreamIn in,
+                                                            const __grid_constant__ StreamOut out,
+                                                            StreamState *st,
                                                             ulonglong2 *long_list,
                                                             uint32_t long_cap) {
-  __shared__ uint32_t scratch[SV_THREADS / 32];
+  constexpr int WARPS = SV_THREADS / 32;
+  static_assert(SV_ITEMS * WARPS == 32, "one lane per warp row of the tile");
+  __shared__ uint32_t row[SV_ITEMS * WARPS];  // voxel starts, then their prefix
   if (ld_relaxed_u32(&ctl->status)) return;
   const uint32_t n = uint32_t(ctl->n_points);
   const uint32_t tiles = (n + SV_TILE - 1) / SV_TILE;
   const SortedView sv = sorted_view(sort, *ss);
   const StreamPlan pl = *plan;
   const uint64_t flag = 1ull << pl.total_bits;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
   for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
-    uint32_t heads = 0;
     uint64_t keys[SV_ITEMS];
-    bool is_head[SV_ITEMS];
+    uint32_t vals[SV_ITEMS], starts[SV_ITEMS];
 #pragma unroll
     for (int k = 0; k < SV_ITEMS; ++k) {
-      const uint32_t i = tile * SV_TILE + threadIdx.x * SV_ITEMS + k;
-      is_head[k] = i < n && stream_head(sv, flag, i, keys[k]);
-      heads += is_head[k] ? 1u : 0u;
+      const uint32_t i = tile * SV_TILE + k * SV_THREADS + threadIdx.x;
+      bool head = false;
+      keys[k] = 0;
+      vals[k] = 0;
+      if (i < n) {
+        sv.get(i, keys[k], vals[k]);
+        head = !(keys[k] & flag) && (i == 0 || sv.key(i - 1) != keys[k]);
+      }
+      starts[k] = __ballot_sync(FULL_MASK, head);
+      if (lane == 0) row[k * WARPS + warp] = __popc(starts[k]);
     }
-    uint32_t total;
-    uint32_t rank = block_exclusive_sum<SV_THREADS>(heads, scratch, &total);
+    __syncthreads();
+    if (warp == 0) {
+      uint32_t total;
+      const uint32_t ex = warp_exclusive_sum(row[lane], &total);
+      __syncwarp();
+      row[lane] = ex;
+    }
+    __syncthreads();
 #pragma unroll
     for (int k = 0; k < SV_ITEMS; ++k) {
-      if (!is_head[k]) continue;
-      const uint32_t i = tile * SV_TILE + threadIdx.x * SV_ITEMS + k;
-      const uint64_t slot = uint64_t(tile_off[tile]) + rank++;
+      if (!((starts[k] >> lane) & 1u)) continue;
+      const uint32_t i = tile * SV_TILE + k * SV_THREADS + threadIdx.x;
+      const uint64_t slot = uint64_t(tile_off[tile]) + row[k * WARPS + warp] +
+                            __popc(starts[k] & lanemask_lt());
       uint32_t j = i + 1;
       while (j < n && j - i < SV_SHORT && sv.key(j) == keys[k]) ++j;
       if (j < n && j - i == SV_SHORT && sv.key(j) == keys[k]) {
@@ -412,18 +536,23 @@ __global__ void __launch_bounds__(SV_THREADS) k_stream_emit(Control *ctl, SortBu
         else atomicOr(&ctl->status, ST_INTERNAL);
         continue;
       }
-      stream_reduce_short<Records>(ctl, sv, pl, in, out, keys[k], i, j, slot);
+      const uint64_t r = out.base + slot;
+      if (r < out.cap) stream_reduce<Records, Final>(sv, pl, in, out, keys[k], i, j, vals[k], r);
+      else atomicOr(&ctl->status, ST_INTERNAL);
     }
+    __syncthreads();
   }
 }
 
 // One block per queued long voxel: finds its end, then reduces every column
 // with per-thread compensated sums combined in thread order.
-template <bool Records>
+template <bool Records, bool Final>
 __global__ void __launch_bounds__(SV_THREADS) k_stream_long(Control *ctl, SortBuffers sort,
                                                             const SortState *ss,
-                                                            const StreamPlan *plan, StreamIn in,
-                                                            StreamOut out, const StreamState *st,
+                                                            const StreamPlan *plan,
+                                                            const __grid_constant__ StreamIn in,
+                                                            const __grid_constant__ StreamOut out,
+                                                            const StreamState *st,
                                                             const ulonglong2 *long_list) {
   __shared__ unsigned long long end_s;
   __shared__ double red[SV_THREADS];
@@ -459,57 +588,38 @@ __global__ void __launch_bounds__(SV_THREADS) k_stream_long(Control *ctl, SortBu
       if (t < w) redc[t] += redc[t + w];
       __syncthreads();
     }
+    cnt = redc[0];
     if (t == 0) {
-      if (ok) {
-        long long kx, ky, kz;
-        stream_unpack(pl, key, kx, ky, kz);
-        out.kx[r] = kx;
-        out.ky[r] = ky;
-        out.kz[r] = kz;
-        out.cnt[r] = redc[0];
-      } else {
-        atomicOr(&ctl->status, ST_INTERNAL);
-      }
+      if (ok) stream_put_key<Final>(out, pl, key, r, cnt);
+      else atomicOr(&ctl->status, ST_INTERNAL);
     }
-    for (uint32_t c = 0; c < in.nc; ++c) {
-      Kahan k;
-      for (uint32_t p = start + t; p < end; p += SV_THREADS)
-        k.add(stream_value<Records>(in, c, sv.val(p)));
-      red[t] = k.s;
+    // column c's compensated sum over the block: `mine` per thread, then in thread order
+    auto column = [&](uint32_t c, const Kahan &mine) {
+      red[t] = mine.s;
       __syncthreads();
       if (t == 0) {
         Kahan tot;
         for (uint32_t w = 0; w < SV_THREADS; ++w) tot.add(red[w]);
-        if (ok) out.sum[c][r] = tot.s;
+        if (ok) stream_put<Final>(out, c, r, tot.s, cnt);
       }
       __syncthreads();
+    };
+    if (Records) {
+      for (uint32_t c = 0; c < in.lay.nc; ++c) {
+        Kahan k;
+        for (uint32_t p = start + t; p < end; p += SV_THREADS) k.add(in.sum[c][sv.val(p)]);
+        column(c, k);
+      }
+    } else {
+      for (uint32_t u = 0; u < in.lay.units; ++u) {
+        Kahan k[4];
+        for (uint32_t p = start + t; p < end; p += SV_THREADS)
+          stream_fields(in.lay, u, in.points[uint64_t(sv.val(p)) * in.lay.units + u],
+                        [&](uint32_t s, uint32_t, double x) { k[s].add(x); });
+        stream_fields(in.lay, u, make_uint4(0, 0, 0, 0),
+                      [&](uint32_t s, uint32_t c, double) { column(c, k[s]); });
+      }
     }
-  }
-}
-
-// Outputs of finish(): positions as f32, the other columns' means in FP64,
-// (ix, iy, iz) triples.
-struct StreamFinal {
-  float *pos[3];
-  double *attr[MAX_COLS];
-  long long *keys3;
-};
-
-// Final records -> outputs: positions (sum / count) as f32, the other
-// columns' means in FP64 (narrowed by the caller per field type, as
-// push_scalar does, streaming.rs:922-938).
-__global__ void __launch_bounds__(256) k_stream_finalize(Control *ctl, StreamOut fin, uint32_t nc,
-                                                         StreamFinal o) {
-  if (ld_relaxed_u32(&ctl->status)) return;
-  const unsigned long long v = ctl->n_voxels;
-  for (unsigned long long r = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; r < v;
-       r += uint64_t(gridDim.x) * blockDim.x) {
-    const double cnt = __ull2double_rn(fin.cnt[r]);
-    for (uint32_t c = 0; c < 3; ++c) o.pos[c][r] = __double2float_rn(__ddiv_rn(fin.sum[c][r], cnt));
-    for (uint32_t c = 3; c < nc; ++c) o.attr[c - 3][r] = __ddiv_rn(fin.sum[c][r], cnt);
-    o.keys3[3 * r] = fin.kx[r];
-    o.keys3[3 * r + 1] = fin.ky[r];
-    o.keys3[3 * r + 2] = fin.kz[r];
   }
 }
 

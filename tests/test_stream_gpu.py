@@ -167,3 +167,41 @@ def test_key_range_error_and_bad_arguments(cuda_ctx):
     with pytest.raises(sr.BufferLengthMismatch):
         sv.push(np.zeros(3, F), np.zeros(2, F), np.zeros(3, F), [np.zeros(3, F)])
     sv.close()
+
+
+@pytest.mark.parametrize("f64", ["", "d", "f", "dfd", "ddff", "fdfdfdfdf", "ddddddddd"])
+@pytest.mark.parametrize("n,device_run", [(1, 0), (1023, 0), (1025, 1025), (5000, 700)])
+def test_record_layouts(cuda_ctx, f64, n, device_run):
+    """Every mix of attribute types is packed into point records and back: one
+    run straight into the outputs, exactly one full run, and merged runs."""
+    rng = np.random.default_rng(n + len(f64))
+    p = rng.uniform(-2, 2, (3, n)).astype(F)
+    attrs = [rng.normal(0, 3, n).astype(np.float64 if t == "d" else F) for t in f64]
+    info = check_stream(cuda_ctx, *p, attrs, leaf=0.4, chunk=333, device_run=device_run)
+    assert info["device_runs"] == (1 if device_run == 0 else -(-n // device_run))
+
+
+def test_device_columns_off_their_alignment(cuda_ctx):
+    """FP64 device columns that start off an 8-byte boundary are staged."""
+    import ctypes
+    import torch
+    n = 4000
+    rng = np.random.default_rng(3)
+    p = rng.uniform(0, 5, (3, n)).astype(F)
+    g = rng.normal(0, 1, n)
+    raw = torch.zeros(8 * n + 4, dtype=torch.uint8, device="cuda")
+    raw[4:] = torch.from_numpy(g.view(np.uint8)).cuda()
+    cols = [torch.from_numpy(a).cuda() for a in p]
+    out = []
+    aligned = torch.from_numpy(g).cuda()
+    for address in (raw.data_ptr() + 4, aligned.data_ptr()):
+        sv = _native.StreamVoxel(cuda_ctx, 0.5, [True])
+        attrs = (ctypes.c_void_p * 1)(address)
+        cloud = _native.SrcuCloud(*[c.data_ptr() for c in cols],
+                                  ctypes.cast(attrs, ctypes.c_void_p), 1, 1, n)
+        cuda_ctx._check(cuda_ctx._lib.srcu_stream_voxel_push(sv._h, ctypes.byref(cloud)))
+        sv.finish()
+        out.append(sv.fetch())
+        sv.close()
+    for a, b in zip(*out):
+        assert np.array_equal(a, b)

@@ -101,49 +101,43 @@ srcu_status ransac_reserve(srcu_ctx *ctx, uint32_t count, uint32_t grid_m) {
   ST_TRY(ensure(ctx, ctx->rs_planes, size_t(std::max<uint32_t>(count, 1)) * 16));
   ST_TRY(ensure(ctx, ctx->rs_valid, size_t(std::max<uint32_t>(count, 1)) * 4));
   ST_TRY(ensure(ctx, ctx->rs_counts, size_t(std::max<uint32_t>(count, 1)) * 4));
-  ST_TRY(ensure(ctx, ctx->rs_partials, size_t(grid_m) * 6 * 8));
+  ST_TRY(ensure(ctx, ctx->rs_partials, sizeof(RansacBest) + size_t(grid_m) * 6 * 8));
   return SRCU_OK;
 }
 
-// Stages the positions and scores `count` hypotheses (host triples); leaves
-// planes, validity and counts on the device and copies them to the host.
-srcu_status ransac_score(srcu_ctx *ctx, const srcu_cloud *cloud, const float **cols,
-                         const uint32_t *hyp_host, uint32_t count, float thr,
-                         std::vector<float4> &planes, std::vector<uint32_t> &valid,
-                         std::vector<uint32_t> &counts) {
-  const uint64_t n = cloud->n;
+// Queues the planes and inlier counts of `count` > 0 hypotheses (host triples).
+srcu_status ransac_score(srcu_ctx *ctx, uint64_t n, const float **cols, const uint32_t *hyp_host,
+                         uint32_t count, float thr) {
   CU_TRY(cudaMemcpyAsync(ctx->rs_hyp.p, hyp_host, size_t(count) * 12, cudaMemcpyHostToDevice,
                          ctx->stream));
-  CU_TRY(cudaMemsetAsync(ctx->rs_counts.p, 0, size_t(count) * 4, ctx->stream));
   uint32_t *status = &ctx->ctl->status;
   CU_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t), ctx->stream));
-  {
-    Launch l(ctx, SRCU_K_RANSAC);
-    k_ransac_planes<<<ceil_div(count, 256), 256, 0, ctx->stream>>>(
-        cols[0], cols[1], cols[2], n, ptr<const uint32_t>(ctx->rs_hyp), count,
-        ptr<float4>(ctx->rs_planes), ptr<uint32_t>(ctx->rs_valid), status);
-    // enough blocks for every SM: point tiles x hypothesis chunks (>= 32 planes each)
-    const uint32_t tiles = std::max<uint32_t>(1, ceil_div(n, RS_TILE));
-    const uint32_t want = uint32_t(ctx->num_sms) * 8;
-    const uint32_t chunks = std::max<uint32_t>(
-        1, std::min<uint32_t>(ceil_div(count, 32), ceil_div(want, tiles)));
-    const uint32_t per_chunk = ceil_div(count, chunks);
-    k_ransac_score<<<dim3(tiles, ceil_div(count, per_chunk)), RS_THREADS, 0, ctx->stream>>>(
-        cols[0], cols[1], cols[2], n, ptr<const float4>(ctx->rs_planes), count, per_chunk, thr,
-        ptr<uint32_t>(ctx->rs_counts));
-  }
+  Launch l(ctx, SRCU_K_RANSAC);
+  k_ransac_planes<<<ceil_div(count, 256), 256, 0, ctx->stream>>>(
+      cols[0], cols[1], cols[2], n, ptr<const uint32_t>(ctx->rs_hyp), count,
+      ptr<float4>(ctx->rs_planes), ptr<uint32_t>(ctx->rs_valid), ptr<uint32_t>(ctx->rs_counts),
+      status);
+  // Point tiles x hypothesis chunks (32 planes at least).  Sixteen points per
+  // thread where the tiles alone come near a block per SM, four below, where the
+  // chunks have to fill the GPU.
+  const bool wide = n >= uint64_t(ctx->num_sms) * (RS_THREADS * 16) / 2;
+  const uint32_t tiles = std::max<uint32_t>(1, ceil_div(n, RS_THREADS * (wide ? 16 : 4)));
+  const uint32_t want = uint32_t(ctx->num_sms) * 16;
+  const uint32_t chunks = std::max<uint32_t>(
+      1, std::min<uint32_t>(ceil_div(count, 32), ceil_div(want, tiles)));
+  const uint32_t per_chunk = ceil_div(count, chunks);
+  (wide ? k_ransac_score<8> : k_ransac_score<2>)<<<dim3(tiles, ceil_div(count, per_chunk)),
+                                                   RS_THREADS, 0, ctx->stream>>>(
+      cols[0], cols[1], cols[2], n, ptr<const float4>(ctx->rs_planes), count, per_chunk, thr,
+      ptr<uint32_t>(ctx->rs_counts));
   CU_TRY(cudaGetLastError());
-  planes.resize(count);
-  valid.resize(count);
-  counts.resize(count);
-  CU_TRY(cudaMemcpyAsync(planes.data(), ctx->rs_planes.p, size_t(count) * 16, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  CU_TRY(cudaMemcpyAsync(valid.data(), ctx->rs_valid.p, size_t(count) * 4, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  CU_TRY(cudaMemcpyAsync(counts.data(), ctx->rs_counts.p, size_t(count) * 4, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  CU_TRY(cudaMemcpyAsync(&ctx->ctl_host->status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                         ctx->stream));
+  return SRCU_OK;
+}
+
+// Waits for what was queued; the status word says whether an index was out of range.
+srcu_status ransac_sync(srcu_ctx *ctx) {
+  CU_TRY(cudaMemcpyAsync(&ctx->ctl_host->status, &ctx->ctl->status, sizeof(uint32_t),
+                         cudaMemcpyDeviceToHost, ctx->stream));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   if (ctx->ctl_host->status)
     return fail(ctx, SRCU_ERR_CUDA, "internal consistency check failed on the device (status 0x%x)",
@@ -177,10 +171,16 @@ srcu_status srcu_ransac_plane_scores(srcu_ctx *ctx, const srcu_cloud *cloud,
   const float *cols[MAX_COLS];
   ST_TRY(ransac_stage(ctx, cloud, cols));
   ST_TRY(ransac_reserve(ctx, count, 1));
-  std::vector<float4> planes;
-  std::vector<uint32_t> valid, counts;
-  ST_TRY(ransac_score(ctx, cloud, cols, hypotheses, count, distance_threshold, planes, valid,
-                      counts));
+  ST_TRY(ransac_score(ctx, cloud->n, cols, hypotheses, count, distance_threshold));
+  std::vector<float4> planes(count);
+  std::vector<uint32_t> valid(count), counts(count);
+  CU_TRY(cudaMemcpyAsync(planes.data(), ctx->rs_planes.p, size_t(count) * 16, cudaMemcpyDeviceToHost,
+                         ctx->stream));
+  CU_TRY(cudaMemcpyAsync(valid.data(), ctx->rs_valid.p, size_t(count) * 4, cudaMemcpyDeviceToHost,
+                         ctx->stream));
+  CU_TRY(cudaMemcpyAsync(counts.data(), ctx->rs_counts.p, size_t(count) * 4, cudaMemcpyDeviceToHost,
+                         ctx->stream));
+  ST_TRY(ransac_sync(ctx));
   for (uint32_t h = 0; h < count; ++h) {
     scores[h].inlier_count = valid[h] ? counts[h] : 0;
     scores[h].normal[0] = planes[h].x;
@@ -213,35 +213,9 @@ srcu_status srcu_ransac_plane_segment(srcu_ctx *ctx, const srcu_cloud *cloud,
   for (uint32_t h = 0; h < count; ++h) sample_indices(rng, n, &hyp[3 * size_t(h)]);
   const float *cols[MAX_COLS];
   ST_TRY(ransac_stage(ctx, cloud, cols));
-  const uint32_t grid_m = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, RM_THREADS),
-                                                                    uint32_t(ctx->num_sms) * 2));
+  const uint32_t grid_m = std::max<uint32_t>(
+      1, std::min<uint32_t>({ceil_div(n, RM_THREADS), uint32_t(ctx->num_sms) * 2, RM_MAX_BLOCKS}));
   ST_TRY(ransac_reserve(ctx, count, grid_m));
-  std::vector<float4> planes;
-  std::vector<uint32_t> valid, counts;
-  if (count) ST_TRY(ransac_score(ctx, cloud, cols, hyp.data(), count, params->distance_threshold,
-                                 planes, valid, counts));
-  // the CPU loop: a candidate replaces the best only with strictly more inliers
-  int64_t best = -1;
-  uint32_t best_count = 0;
-  for (uint32_t h = 0; h < count; ++h)
-    if (valid[h] && counts[h] > best_count) {
-      best = h;
-      best_count = counts[h];
-    }
-  result->hypotheses = count;
-  result->best_hypothesis = best < 0 ? UINT32_MAX : uint32_t(best);
-  result->inlier_count = best_count;
-  if (best_count < params->min_inliers)  // plane.rs:318-324
-    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "RANSAC found only %u inliers, minimum is %llu",
-                best_count, (unsigned long long)params->min_inliers);
-  if (best < 0)  // min_inliers == 0 and no plane with an inlier: no model to refine (:326-328)
-    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "failed to refine plane model");
-  const float4 bp = planes[size_t(best)];
-  result->hypothesis_normal[0] = bp.x;
-  result->hypothesis_normal[1] = bp.y;
-  result->hypothesis_normal[2] = bp.z;
-  result->hypothesis_d = bp.w;
-  // inlier mask + FP64 sums (pass 0), centred moments (pass 1)
   uint8_t *mask_dev = nullptr;
   if (inlier_mask && cloud->on_device) {
     mask_dev = inlier_mask;
@@ -249,44 +223,64 @@ srcu_status srcu_ransac_plane_segment(srcu_ctx *ctx, const srcu_cloud *cloud,
     ST_TRY(ensure(ctx, ctx->rs_mask, n));
     mask_dev = ptr<uint8_t>(ctx->rs_mask);
   }
-  const float4 *plane_dev = ptr<const float4>(ctx->rs_planes) + best;
-  std::vector<double> part(size_t(grid_m) * 6);
-  {
-    Launch l(ctx, SRCU_K_RANSAC);
-    k_ransac_moments<<<grid_m, RM_THREADS, 0, ctx->stream>>>(
-        cols[0], cols[1], cols[2], n, plane_dev, params->distance_threshold, mask_dev, 0,
-        make_double3(0, 0, 0), ptr<double>(ctx->rs_partials));
+  // Scores, the choice, the inlier mask with FP64 sums and the centred moments are
+  // queued as one chain; the host reads the choice and the moments at its end.  (A
+  // wait after the scores and one after the sums took 110 us of a 320 us call.)
+  RansacBest best{};
+  best.index = -1;
+  RansacBest *best_dev = ptr<RansacBest>(ctx->rs_partials);
+  double *partials = reinterpret_cast<double *>(best_dev + 1);
+  std::vector<unsigned char> back(sizeof(RansacBest) + size_t(grid_m) * 6 * 8);
+  if (count) {
+    ST_TRY(ransac_score(ctx, n, cols, hyp.data(), count, params->distance_threshold));
+    {
+      Launch l(ctx, SRCU_K_RANSAC);
+      k_ransac_best<<<1, 1024, 0, ctx->stream>>>(ptr<const float4>(ctx->rs_planes),
+                                                 ptr<const uint32_t>(ctx->rs_valid),
+                                                 ptr<const uint32_t>(ctx->rs_counts), count,
+                                                 best_dev);
+      k_ransac_moments<<<grid_m, RM_THREADS, 0, ctx->stream>>>(
+          cols[0], cols[1], cols[2], n, best_dev, params->min_inliers, params->distance_threshold,
+          mask_dev, 0, partials);
+      k_ransac_mean<<<1, 256, 0, ctx->stream>>>(partials, grid_m, params->min_inliers, best_dev);
+      k_ransac_moments<<<grid_m, RM_THREADS, 0, ctx->stream>>>(
+          cols[0], cols[1], cols[2], n, best_dev, params->min_inliers, params->distance_threshold,
+          nullptr, 1, partials);
+    }
+    CU_TRY(cudaGetLastError());
+    CU_TRY(cudaMemcpyAsync(back.data(), ctx->rs_partials.p, back.size(), cudaMemcpyDeviceToHost,
+                           ctx->stream));
+    ST_TRY(ransac_sync(ctx));
+    memcpy(&best, back.data(), sizeof(best));
   }
-  CU_TRY(cudaGetLastError());
-  CU_TRY(cudaMemcpyAsync(part.data(), ctx->rs_partials.p, part.size() * 8, cudaMemcpyDeviceToHost,
-                         ctx->stream));
-  CU_TRY(cudaStreamSynchronize(ctx->stream));
-  double cnt = 0, sx = 0, sy = 0, sz = 0;
-  for (uint32_t b = 0; b < grid_m; ++b) {
-    cnt += part[6 * b];
-    sx += part[6 * b + 1];
-    sy += part[6 * b + 2];
-    sz += part[6 * b + 3];
-  }
+  const uint32_t best_count = best.count;
+  result->hypotheses = count;
+  result->best_hypothesis = best.index < 0 ? UINT32_MAX : uint32_t(best.index);
+  result->inlier_count = best_count;
+  if (best_count < params->min_inliers)  // plane.rs:318-324
+    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "RANSAC found only %u inliers, minimum is %llu",
+                best_count, (unsigned long long)params->min_inliers);
+  if (best.index < 0)  // min_inliers == 0 and no plane with an inlier: no model to refine (:326-328)
+    return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "failed to refine plane model");
+  const float4 bp = best.plane;
+  result->hypothesis_normal[0] = bp.x;
+  result->hypothesis_normal[1] = bp.y;
+  result->hypothesis_normal[2] = bp.z;
+  result->hypothesis_d = bp.w;
+  const double cnt = best.cnt;
   if (uint64_t(cnt) != best_count)
     return fail(ctx, SRCU_ERR_CUDA, "inlier recount %llu differs from the score %u",
                 (unsigned long long)cnt, best_count);
   float model[4] = {bp.x, bp.y, bp.z, bp.w};
   if (best_count >= 3) {  // refine_plane_from_inliers (plane_ransac.rs:96-150)
-    const double mean[3] = {sx / cnt, sy / cnt, sz / cnt};
-    {
-      Launch l(ctx, SRCU_K_RANSAC);
-      k_ransac_moments<<<grid_m, RM_THREADS, 0, ctx->stream>>>(
-          cols[0], cols[1], cols[2], n, plane_dev, params->distance_threshold, nullptr, 1,
-          make_double3(mean[0], mean[1], mean[2]), ptr<double>(ctx->rs_partials));
-    }
-    CU_TRY(cudaGetLastError());
-    CU_TRY(cudaMemcpyAsync(part.data(), ctx->rs_partials.p, part.size() * 8,
-                           cudaMemcpyDeviceToHost, ctx->stream));
-    CU_TRY(cudaStreamSynchronize(ctx->stream));
+    const double *mean = best.mean;
     double c6[6] = {0, 0, 0, 0, 0, 0};  // c00 c11 c22 c01 c02 c12
     for (uint32_t b = 0; b < grid_m; ++b)
-      for (int k = 0; k < 6; ++k) c6[k] += part[6 * b + k];
+      for (int k = 0; k < 6; ++k) {
+        double part;
+        memcpy(&part, back.data() + sizeof(RansacBest) + (size_t(b) * 6 + k) * 8, 8);
+        c6[k] += part;
+      }
     const double inv = 1.0 / cnt;
     const double cov[3][3] = {{c6[0] * inv, c6[3] * inv, c6[4] * inv},
                               {c6[3] * inv, c6[1] * inv, c6[5] * inv},

@@ -97,3 +97,43 @@ def test_errors(cuda_ctx):
         cuda_ctx.ransac_plane_segment(line, line, line, 0.05, 20, 1, 3)
     with pytest.raises(sr.InvalidArgument):
         cuda_ctx.ransac_plane_scores(p[:, 0], p[:, 1], p[:, 2], [[0, 1, 500]], 0.05)
+
+
+@pytest.mark.parametrize("n", [3, 1023, 1025, 4097, 303_103, 303_104, 310_000])
+def test_scores_at_tile_edges(cuda_ctx, n):
+    """Inlier counts at the edges of the scoring kernels' point tiles (four and
+    sixteen points per thread) and plane chunks, against the CPU segmenter's
+    f32 expression; and the whole answer against the oracle."""
+    rng = np.random.default_rng(n)
+    p = rng.normal(0, 1, (3, n)).astype(np.float32)
+    p[2, : n // 2] *= np.float32(0.01)
+    if n > 3:
+        p[0, n - 1] = np.nan
+    hyp = rng.integers(0, n, (67, 3)).astype(np.uint32)
+    got = cuda_ctx.ransac_plane_scores(*p, hyp, 0.02)
+    for count, normal, d in got[:: 11]:
+        a, b, c = (np.float32(v) for v in normal)
+        s = ((a * p[0] + b * p[1]) + c * p[2]) + np.float32(d)
+        expect = int((np.abs(s) <= np.float32(0.02)).sum()) if any(normal) or d else count
+        assert count == expect
+    ref = oracle.ransac_plane(*p, 0.02, 67, 1, 9)
+    info, mask = cuda_ctx.ransac_plane_segment(*p, 0.02, 67, 1, 9)
+    assert info["inlier_count"] == ref["inlier_count"] == mask.sum()
+    assert info["best_hypothesis"] == ref["best_index"]
+
+
+def test_too_few_inliers_leave_a_device_mask_alone(cuda_ctx):
+    import ctypes
+    import torch
+    from spatialrust_b200 import _native
+    x, y, z = (torch.rand(5000, device="cuda") for _ in range(3))
+    mask = torch.full((5000,), 7, dtype=torch.uint8, device="cuda")
+    keep = _native._Keep()
+    cloud = _native.make_cloud(x, y, z, [], keep)
+    prm = _native.SrcuRansacParams(0.01, 50, 5001, 1)
+    st = cuda_ctx._lib.srcu_ransac_plane_segment(cuda_ctx.handle, ctypes.byref(cloud),
+                                                 ctypes.byref(prm),
+                                                 ctypes.byref(_native.SrcuRansacResult()),
+                                                 mask.data_ptr())
+    assert st == _native.SRCU_ERR_INVALID_ARGUMENT
+    assert bool((mask == 7).all())

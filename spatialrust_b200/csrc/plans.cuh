@@ -125,9 +125,8 @@ struct SortState {
   uint32_t packed;     // 1: items are (key << idx_bits) | index; 0: keys[] + vals[]
   uint32_t idx_bits;
   uint32_t key_bits;
-  uint32_t bar_count;
-  uint32_t bar_gen;
-  uint32_t pad;
+  uint32_t arrived;    // grid barrier: blocks that have arrived, over all its rounds
+  uint32_t pad[2];
 };
 
 struct NormalCounters {

@@ -119,7 +119,8 @@ __global__ void __launch_bounds__(CELL_THREADS) k_cells(Control *ctl, SortBuffer
     uint32_t tile_count;
     const uint32_t local = block_exclusive_sum<CELL_THREADS>(__popc(flags), sm.scratch, &tile_count);
     if (t < 32) {
-      const uint32_t cb = lookback_exclusive_warp(lookback, tile, tile_count, epoch, &ctl->status);
+      const uint32_t cb = lookback_exclusive_warp(lookback, tile, tile_count, epoch, &ctl->status,
+                                                  num_tiles <= gridDim.x);
       if (t == 0) sm.scratch[0] = cb;
     }
     __syncthreads();

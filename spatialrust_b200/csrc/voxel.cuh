@@ -305,13 +305,19 @@ constexpr int SEG_THREADS = 256;
 constexpr int SEG_ITEMS = 4;
 constexpr int SEG_TILE = SEG_THREADS * SEG_ITEMS;  // 1024 sorted positions per tile
 constexpr uint32_t SEG_SHORT = 32;  // longer voxels are reduced by a whole warp
+constexpr int SEG_GROUP = 4;  // columns gathered and summed together
 
 // Shared memory of k_voxel_segments<NC>: the tile's keys (plus one before and
 // one after), the scan scratch, and the tile's gathered point columns.
 struct SegmentSmemHead {
   uint64_t keys[SEG_TILE + 2];  // keys[0] = key before the tile, keys[1 + tile_n] = key after it
+  uint16_t start[SEG_TILE + 2];  // first position of each voxel that starts in the tile, then tile_n
+  uint16_t longs[SEG_TILE / SEG_SHORT + 2];  // the tile's voxels that a warp reduces
   uint32_t scratch[SEG_THREADS / 32];
-  uint32_t tile;
+  double inv[SEG_SHORT + 1];  // 1.0 / count of the short voxels
+  uint32_t tile;              // the tile at work, then the next one
+  uint32_t seg_base;
+  uint32_t num_longs;
   uint32_t pad;
 };
 __host__ __device__ constexpr size_t segment_smem_bytes(int nc) {
@@ -327,16 +333,17 @@ __device__ __forceinline__ int32_t voxel_agg(const Batch &bt, uint64_t key, uint
   return bt.vparams[b < bt.clouds ? b : 0].agg;
 }
 
-// Writes one voxel.  s: FP64 sums of every column in ascending point order;
-// first(c): column c of the voxel's first point, read only by the modes that
-// use it (so the default mode keeps no extra registers live).
+// Writes columns C0 .. C0 + G - 1 of one voxel, and with column 0 its key, count and
+// AoS record.  s: their FP64 sums in ascending point order; inv: 1.0 / cnt; first(c): column c of
+// the voxel's first point, read only by the modes that use it (so the default
+// mode keeps no extra registers live).
 //   AGG_FAST            (sum * (1.0 / count)) as f32, voxel.rs:531-536
 //   AGG_CENTROID_FIRST  positions (sum / count) as f32 (average_field,
 //                       voxel.rs:1156-1165), other fields from the first point
 //   AGG_FIRST           every field from the first point (voxel.rs:1144-1146)
-template <int NC, class First>
-__device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const double (&s)[NC],
-                                               First first, int32_t agg,
+template <int NC, int C0, int G, class First>
+__device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const double (&s)[G],
+                                               First first, int32_t agg, double inv,
                                                uint32_t cnt, uint32_t seg, uint64_t key,
                                                uint64_t *out_keys, uint32_t *out_counts,
                                                uint32_t n, uint32_t *status, float4 *aos_out) {
@@ -344,19 +351,137 @@ __device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const do
     atomicOr(status, ST_INTERNAL);
     return;
   }
-  const double inv = 1.0 / double(cnt);
-  float o[NC];
+  float o[G];
 #pragma unroll
-  for (int c = 0; c < NC; ++c) {
-    if (agg == AGG_FAST) o[c] = __double2float_rn(__dmul_rn(s[c], inv));
+  for (int g = 0; g < G; ++g) {
+    const int c = C0 + g;
+    if (agg == AGG_FAST) o[g] = __double2float_rn(__dmul_rn(s[g], inv));
     else if (agg == AGG_CENTROID_FIRST && c < 3)
-      o[c] = __double2float_rn(__ddiv_rn(s[c], double(cnt)));
-    else o[c] = first(c);
-    cols.out[c][seg] = o[c];
+      o[g] = __double2float_rn(__ddiv_rn(s[g], double(cnt)));
+    else o[g] = first(c);
+    cols.out[c][seg] = o[g];
   }
+  if (C0 > 0) return;
   if (aos_out) aos_out[seg] = make_float4(o[0], o[1], o[2], 0.0f);
   out_keys[seg] = key;
   out_counts[seg] = cnt;
+}
+
+// Columns 0 .. 3 of the points iv[]: from the AoS copy, one sector per point, where
+// there is one.
+template <int NC>
+__device__ __forceinline__ void gather_points(float4 (&pt)[SEG_ITEMS], const uint32_t (&iv)[SEG_ITEMS],
+                                              const Columns<NC> &cols, const float4 *aos_in,
+                                              uint32_t n) {
+#pragma unroll
+  for (int q = 0; q < SEG_ITEMS; ++q) {
+    pt[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (iv[q] >= n) continue;
+    if (aos_in) {
+      pt[q] = aos_in[iv[q]];
+    } else {
+      pt[q].x = cols.in[0][iv[q]];
+      pt[q].y = cols.in[1][iv[q]];
+      pt[q].z = cols.in[2][iv[q]];
+      if constexpr (NC > 3) pt[q].w = cols.in[3][iv[q]];
+    }
+  }
+}
+template <int NC>
+__device__ __forceinline__ void store_points(const float4 (&pt)[SEG_ITEMS], float *scol,
+                                             uint32_t tile_n) {
+#pragma unroll
+  for (int q = 0; q < SEG_ITEMS; ++q) {
+    const uint32_t j = threadIdx.x + uint32_t(q) * SEG_THREADS;
+    if (j >= tile_n) continue;
+    scol[0 * SEG_TILE + j] = pt[q].x;
+    scol[1 * SEG_TILE + j] = pt[q].y;
+    scol[2 * SEG_TILE + j] = pt[q].z;
+    if constexpr (NC > 3) scol[3 * SEG_TILE + j] = pt[q].w;
+  }
+}
+// The columns from C0 on, SEG_GROUP at a time.
+template <int NC, int C0>
+__device__ __forceinline__ void gather_more(const uint32_t (&iv)[SEG_ITEMS], const Columns<NC> &cols,
+                                            float *scol, uint32_t tile_n, uint32_t n) {
+  if constexpr (C0 < NC) {
+    constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
+    float a[SEG_ITEMS][G];
+#pragma unroll
+    for (int q = 0; q < SEG_ITEMS; ++q)
+#pragma unroll
+      for (int g = 0; g < G; ++g) a[q][g] = iv[q] < n ? cols.in[C0 + g][iv[q]] : 0.0f;
+#pragma unroll
+    for (int q = 0; q < SEG_ITEMS; ++q) {
+      const uint32_t j = threadIdx.x + uint32_t(q) * SEG_THREADS;
+      if (j >= tile_n) continue;
+#pragma unroll
+      for (int g = 0; g < G; ++g) scol[(C0 + g) * SEG_TILE + j] = a[q][g];
+    }
+    gather_more<NC, C0 + SEG_GROUP>(iv, cols, scol, tile_n, n);
+  }
+}
+
+// Columns from C0 on, SEG_GROUP at a time, of the short voxel at tile positions [j, e):
+// sums in ascending point index.
+template <int NC, int C0>
+__device__ __forceinline__ void short_voxel(const SegmentSmemHead &sm, const float *scol, uint32_t j,
+                                            uint32_t e, uint32_t seg, uint64_t key,
+                                            const Columns<NC> &cols, int32_t agg,
+                                            uint64_t *out_keys, uint32_t *out_counts, uint32_t n,
+                                            uint32_t *status, float4 *aos_out) {
+  constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
+  double s[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) s[g] = 0.0;
+#pragma unroll 2
+  for (uint32_t m = j; m < e; ++m) {
+#pragma unroll
+    for (int g = 0; g < G; ++g) s[g] += double(scol[(C0 + g) * SEG_TILE + m]);
+  }
+  write_centroid<NC, C0, G>(cols, s, [&](int c) { return scol[c * SEG_TILE + j]; }, agg,
+                            sm.inv[e - j], e - j, seg, key, out_keys, out_counts, n, status, aos_out);
+  if constexpr (C0 + SEG_GROUP < NC)
+    short_voxel<NC, C0 + SEG_GROUP>(sm, scol, j, e, seg, key, cols, agg, out_keys, out_counts, n,
+                                    status, aos_out);
+}
+
+// The columns of one voxel from C0 on, its sorted items [p, e) reduced by a warp.
+template <int NC, int C0>
+__device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uint32_t e, uint32_t seg,
+                                           uint64_t key, const Columns<NC> &cols, int32_t agg,
+                                           uint64_t *out_keys, uint32_t *out_counts, uint32_t n,
+                                           uint32_t *status, float4 *aos_out) {
+  constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
+  const uint32_t lane = threadIdx.x & 31u;
+  double s[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) s[g] = 0.0;
+  for (uint32_t m = p + lane; m < e; m += 32) {
+    const uint32_t v = sv.val(m);
+    if (v >= n) {
+      atomicOr(status, ST_INTERNAL);
+      continue;
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) s[g] += double(cols.in[C0 + g][v]);
+  }
+#pragma unroll
+  for (int g = 0; g < G; ++g)
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s[g] += __shfl_xor_sync(FULL_MASK, s[g], o);
+  if (lane == 0) {
+    // the voxel's first point is the first sorted item (stable sort)
+    auto first = [&](int c) {
+      const uint32_t v0 = sv.val(p);
+      return v0 < n ? cols.in[c][v0] : 0.0f;
+    };
+    write_centroid<NC, C0, G>(cols, s, first, agg, 1.0 / double(e - p), e - p, seg, key, out_keys,
+                              out_counts, n, status, aos_out);
+  }
+  if constexpr (C0 + SEG_GROUP < NC)
+    long_voxel<NC, C0 + SEG_GROUP>(sv, p, e, seg, key, cols, agg, out_keys, out_counts, n, status,
+                                   aos_out);
 }
 
 // Fused segment discovery + FP64 centroid reduction over the sorted
@@ -367,8 +492,15 @@ __device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const do
 // per short voxel (sequential FP64 sum in ascending point index, the
 // reference's order, voxel.rs:502-520), one warp per long voxel or per voxel
 // that runs past the tile end.
+// Bound by latency: at 2M points, 7 columns, 16% of the issue slots and a fifth of
+// L2's rate are used.  So nothing waits that need not: a thread's item loads, and
+// then its gathers, are issued together and stay in flight over the look-back, the
+// next tile is claimed meanwhile, a thread takes a voxel (not a range of
+// positions) and four columns at a time, and 64 registers keep all of that out of
+// local memory.  2M points: 4 columns 83 -> 65 us, 7 columns 158 -> 97; 14.6M
+// points of a batch 486 -> 380.
 template <int NC>
-__global__ void __launch_bounds__(SEG_THREADS, 5) k_voxel_segments(Control *ctl, SortBuffers sort,
+__global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl, SortBuffers sort,
                                                                  const SortState *sort_state,
                                                                  Columns<NC> cols,
                                                                  uint64_t *out_keys,
@@ -388,8 +520,11 @@ __global__ void __launch_bounds__(SEG_THREADS, 5) k_voxel_segments(Control *ctl,
   const uint32_t num_tiles = (n + SEG_TILE - 1) / SEG_TILE;
   const uint32_t t = threadIdx.x, lane = t & 31u;
 
+  const uint32_t vkey_bits = ctl->vkey_bits;
+  if (t == 0) sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
+  if (t >= 32 && t <= 32 + SEG_SHORT) sm.inv[t - 32] = 1.0 / double(t - 32);
+
   for (;;) {
-    if (t == 0) sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
     __syncthreads();
     const uint32_t tile = sm.tile;
     if (tile >= num_tiles) break;
@@ -397,55 +532,50 @@ __global__ void __launch_bounds__(SEG_THREADS, 5) k_voxel_segments(Control *ctl,
     const uint32_t tile_n = min(uint32_t(SEG_TILE), n - base);
     // The tile's sorted items, then their points: every thread issues all of
     // its SEG_ITEMS item loads, then all of its random point gathers, before
-    // any of them is consumed, so the gathers' latencies overlap.
-    uint64_t ik[SEG_ITEMS];
+    // any of them is consumed, so the gathers' latencies overlap -- with one
+    // another, and with the count of the voxel starts and the look-back over it,
+    // which need the keys alone.
     uint32_t iv[SEG_ITEMS];
-    uint64_t k_before = 0, k_after = 0;  // the keys either side of the tile (thread 0)
-    if (t == 0) {
-      k_before = base > 0 ? sv.key(base - 1) : ~sv.key(0);
-      k_after = base + tile_n < n ? sv.key(base + tile_n) : ~sv.key(n - 1);
-    }
+    {
+      uint64_t w[SEG_ITEMS], edge = 0;  // edge: the item either side of the tile (threads 0 and 1)
 #pragma unroll
-    for (int q = 0; q < SEG_ITEMS; ++q) {
-      const uint32_t j = t + uint32_t(q) * SEG_THREADS;
-      ik[q] = 0;
-      iv[q] = n;  // out of range: no gather
-      if (j < tile_n) sv.get(base + j, ik[q], iv[q]);
-    }
-    if (aos_in) {  // columns 0..3 from the AoS copy: one sector per point
-      float4 pt[SEG_ITEMS];
+      for (int q = 0; q < SEG_ITEMS; ++q) {
+        const uint32_t j = t + uint32_t(q) * SEG_THREADS;
+        w[q] = j < tile_n ? sv.keys[base + j] : 0ull;
+      }
+      if (t == 0) edge = sv.keys[base > 0 ? base - 1 : 0u];
+      if (t == 1) edge = sv.keys[base + tile_n < n ? base + tile_n : n - 1];
+      if (!sv.packed) {
 #pragma unroll
-      for (int q = 0; q < SEG_ITEMS; ++q)
-        pt[q] = iv[q] < n ? aos_in[iv[q]] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int q = 0; q < SEG_ITEMS; ++q) {
+          const uint32_t j = t + uint32_t(q) * SEG_THREADS;
+          iv[q] = j < tile_n ? sv.vals[base + j] : n;  // out of range: no gather
+        }
+      } else {
+#pragma unroll
+        for (int q = 0; q < SEG_ITEMS; ++q) {
+          const uint32_t j = t + uint32_t(q) * SEG_THREADS;
+          iv[q] = j < tile_n ? uint32_t(w[q] & ((1ull << sv.idx_bits) - 1)) : n;
+        }
+      }
+      const uint32_t key_shift = sv.packed ? sv.idx_bits : 0u;
 #pragma unroll
       for (int q = 0; q < SEG_ITEMS; ++q) {
         const uint32_t j = t + uint32_t(q) * SEG_THREADS;
         if (j >= tile_n) continue;
-        scol[0 * SEG_TILE + j] = pt[q].x;
-        scol[1 * SEG_TILE + j] = pt[q].y;
-        scol[2 * SEG_TILE + j] = pt[q].z;
-        if (NC > 3) scol[3 * SEG_TILE + j] = pt[q].w;
+        sm.keys[1 + j] = w[q] >> key_shift;
+        // a consistent sort never produces this; never read out of bounds
+        if (iv[q] >= n) atomicOr(&ctl->status, ST_INTERNAL);
       }
-    }
-#pragma unroll
-    for (int q = 0; q < SEG_ITEMS; ++q) {
-      const uint32_t j = t + uint32_t(q) * SEG_THREADS;
-      if (j >= tile_n) continue;
-      sm.keys[1 + j] = ik[q];
-      const uint32_t v = iv[q];
-      if (v < n) {
-#pragma unroll
-        for (int c = aos_in ? 4 : 0; c < NC; ++c) scol[c * SEG_TILE + j] = cols.in[c][v];
-      } else {  // a consistent sort never produces this; never read out of bounds
-        atomicOr(&ctl->status, ST_INTERNAL);
-#pragma unroll
-        for (int c = 0; c < NC; ++c) scol[c * SEG_TILE + j] = 0.0f;
+      edge >>= key_shift;
+      if (t == 0) {  // unlike the first key where there is none before it
+        sm.keys[0] = base > 0 ? edge : ~edge;
+        sm.num_longs = 0;
       }
+      if (t == 1) sm.keys[1 + tile_n] = base + tile_n < n ? edge : ~edge;
     }
-    if (t == 0) {
-      sm.keys[0] = k_before;
-      sm.keys[1 + tile_n] = k_after;
-    }
+    float4 pt[SEG_ITEMS];
+    gather_points<NC>(pt, iv, cols, aos_in, n);
     __syncthreads();
 
     const uint32_t j0 = t * SEG_ITEMS;
@@ -455,58 +585,46 @@ __global__ void __launch_bounds__(SEG_THREADS, 5) k_voxel_segments(Control *ctl,
       const uint32_t j = j0 + i;
       if (j < tile_n && sm.keys[1 + j] != sm.keys[j]) flags |= 1u << i;
     }
-    uint32_t tile_count;
-    const uint32_t local = block_exclusive_sum<SEG_THREADS>(__popc(flags), sm.scratch, &tile_count);
-    uint32_t seg_base = 0;
+    uint32_t voxels;
+    uint32_t local = block_exclusive_sum<SEG_THREADS>(__popc(flags), sm.scratch, &voxels);
     if (t < 32) {
-      seg_base = lookback_exclusive_warp(lookback, tile, tile_count, epoch, &ctl->status);
-      if (t == 0) sm.scratch[0] = seg_base;
+      const uint32_t seg_base =
+          lookback_exclusive_warp(lookback, tile, voxels, epoch, &ctl->status,
+                                  num_tiles <= gridDim.x);
+      if (t == 0) {
+        sm.seg_base = seg_base;
+        sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
+        sm.start[voxels] = uint16_t(tile_n);
+        if (tile == num_tiles - 1) ctl->n_voxels = seg_base + voxels;
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < SEG_ITEMS; ++i)
+      if (flags & (1u << i)) sm.start[local++] = uint16_t(j0 + i);
+    store_points<NC>(pt, scol, tile_n);
+    gather_more<NC, 4>(iv, cols, scol, tile_n, n);
+    __syncthreads();
+
+    // Short voxels: a thread each, from shared memory.  Long ones (more than SEG_SHORT
+    // points, or running past the tile) are listed.
+    for (uint32_t q = t; q < voxels; q += SEG_THREADS) {
+      const uint32_t j = sm.start[q], e = sm.start[q + 1];
+      const uint64_t key = sm.keys[1 + j];
+      if (e - j > SEG_SHORT || sm.keys[1 + e] == key)
+        sm.longs[atomicAdd(&sm.num_longs, 1u)] = uint16_t(q);
+      else
+        short_voxel<NC, 0>(sm, scol, j, e, sm.seg_base + q, key, cols,
+                           voxel_agg(bt, key, vkey_bits, agg_all), out_keys, out_counts, n,
+                           &ctl->status, aos_out);
     }
     __syncthreads();
-    seg_base = sm.scratch[0];
-    if (t == 0 && tile == num_tiles - 1) ctl->n_voxels = seg_base + tile_count;
-
-    // Short voxels: the owning thread reduces sequentially from shared memory.
-    // At most one voxel per thread (its last start) can be long or run past
-    // the tile.
-    bool deferred = false;
-    uint32_t def_pos = 0, def_seg = 0;
-    uint32_t seg = seg_base + local;
-    for (int i = 0; i < SEG_ITEMS; ++i) {
-      if (!(flags & (1u << i))) continue;
-      const uint32_t j = j0 + i;
+    // Long voxels: a warp finds the end and reduces from global memory.
+    for (uint32_t i = t >> 5; i < sm.num_longs; i += SEG_THREADS / 32) {
+      const uint32_t q = sm.longs[i];
+      const uint32_t j = sm.start[q];
       const uint64_t key = sm.keys[1 + j];
-      uint32_t e = j + 1;
-      while (e < tile_n && e - j <= SEG_SHORT && sm.keys[1 + e] == key) ++e;
-      const bool closed = sm.keys[1 + e] != key;  // keys[1 + tile_n] is the key after the tile
-      if (closed && e - j <= SEG_SHORT) {
-        double s[NC];
-#pragma unroll
-        for (int c = 0; c < NC; ++c) s[c] = 0.0;
-        for (uint32_t m = j; m < e; ++m) {
-#pragma unroll
-          for (int c = 0; c < NC; ++c) s[c] += double(scol[c * SEG_TILE + m]);
-        }
-        write_centroid<NC>(cols, s, [&](int c) { return scol[c * SEG_TILE + j]; },
-                           voxel_agg(bt, key, ctl->vkey_bits, agg_all), e - j, seg, key, out_keys,
-                           out_counts, n, &ctl->status, aos_out);
-      } else {
-        deferred = true;
-        def_pos = base + j;
-        def_seg = seg;
-      }
-      ++seg;
-    }
-    // Long voxels: the whole warp finds the end and reduces from global memory.
-    uint32_t pending = __ballot_sync(FULL_MASK, deferred);
-    while (pending) {
-      const uint32_t src_lane = __ffs(pending) - 1;
-      pending &= pending - 1;
-      const uint32_t p = __shfl_sync(FULL_MASK, def_pos, src_lane);
-      const uint32_t sg = __shfl_sync(FULL_MASK, def_seg, src_lane);
-      const uint64_t key = sv.key(p);
-      uint32_t e = p + 1;
-      for (;;) {
+      uint32_t e = base + sm.start[q + 1];
+      while (e < n) {
         const uint32_t idx = e + lane;
         const bool stop = idx >= n || sv.key(idx) != key;
         const uint32_t b = __ballot_sync(FULL_MASK, stop);
@@ -516,33 +634,10 @@ __global__ void __launch_bounds__(SEG_THREADS, 5) k_voxel_segments(Control *ctl,
         }
         e += 32;
       }
-      double s[NC];
-#pragma unroll
-      for (int c = 0; c < NC; ++c) s[c] = 0.0;
-      for (uint32_t m = p + lane; m < e; m += 32) {
-        const uint32_t v = sv.val(m);
-        if (v >= n) {
-          atomicOr(&ctl->status, ST_INTERNAL);
-          continue;
-        }
-#pragma unroll
-        for (int c = 0; c < NC; ++c) s[c] += double(cols.in[c][v]);
-      }
-#pragma unroll
-      for (int c = 0; c < NC; ++c)
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s[c] += __shfl_xor_sync(FULL_MASK, s[c], o);
-      if (lane == 0) {
-        // the voxel's first point is the first sorted item (stable sort)
-        auto first = [&](int c) {
-          const uint32_t v0 = sv.val(p);
-          return v0 < n ? cols.in[c][v0] : 0.0f;
-        };
-        write_centroid<NC>(cols, s, first, voxel_agg(bt, key, ctl->vkey_bits, agg_all), e - p, sg,
-                           key, out_keys, out_counts, n, &ctl->status, aos_out);
-      }
+      long_voxel<NC, 0>(sv, base + j, e, sm.seg_base + q, key, cols,
+                        voxel_agg(bt, key, vkey_bits, agg_all), out_keys, out_counts, n,
+                        &ctl->status, aos_out);
     }
-    __syncthreads();
   }
 }
 

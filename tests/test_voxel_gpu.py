@@ -156,6 +156,24 @@ def test_tile_boundaries(cuda_ctx, n):
     assert_voxel_parity(cuda_ctx, p[:, 0], p[:, 1], p[:, 2], [i], leaf=1.0)
 
 
+# voxels that end on, before and past a tile's end (1024 sorted points), and around
+# the 32 points up to which one thread reduces a voxel; up to three groups of columns.
+# Attributes are below 1, so the file's bound (1e-5) is 80 ulp of theirs.
+@pytest.mark.parametrize("n_attrs", [0, 1, 2, 5, 9])
+@pytest.mark.parametrize("lengths", [
+    [1024], [1023, 1], [1023, 2], [1025, 3], [992, 32, 5], [992, 33], [991, 33, 31],
+    [1] * 1024 + [32] * 33, [31, 32, 33, 34] * 24, [5000, 1, 1, 3000]])
+def test_voxels_at_tile_ends(cuda_ctx, lengths, n_attrs):
+    rng = np.random.default_rng(len(lengths) * 10 + n_attrs)
+    x = (np.repeat(np.arange(len(lengths)), lengths) + rng.uniform(0.1, 0.9, sum(lengths))).astype(F)
+    order = rng.permutation(len(x))
+    y, z = rng.uniform(0.1, 0.9, (2, len(x))).astype(F)
+    attrs = [rng.uniform(0, 1, len(x)).astype(F) for _ in range(n_attrs)]
+    starts = np.cumsum([0] + lengths)
+    short = all(b - a <= 32 and a // 1024 == (b - 1) // 1024 for a, b in zip(starts[:-1], starts[1:]))
+    assert_voxel_parity(cuda_ctx, x[order], y, z, attrs, leaf=1.0, origin=(0.0, 0.0, 0.0), exact=short)
+
+
 def test_explicit_origin_negative_keys(cuda_ctx):
     rng = np.random.default_rng(12)
     p = (rng.random((80_000, 3), dtype=np.float32) - F(0.5)) * F(40)

@@ -105,7 +105,7 @@ void noalloc_segments(cudaStream_t s, uint32_t grid, Control *ctl, const SortBuf
     cols.out[c] = out[c];
   }
   k_voxel_segments<NC><<<grid, SEG_THREADS, segment_smem_bytes(NC), s>>>(
-      ctl, sb, &ctl->vsort, cols, vkeys, vcounts, sb.lookback + 0, nullptr, nullptr, bt, -1);
+      ctl, sb, &ctl->vsort, cols, vkeys, vcounts, sb.lookback + 0, nullptr, nullptr, nullptr, bt, -1);
 }
 
 }  // namespace

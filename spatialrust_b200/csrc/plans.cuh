@@ -165,7 +165,7 @@ constexpr uint32_t EP_VSORT = 0;     // 8 passes
 constexpr uint32_t EP_VSEG = 8;
 constexpr uint32_t EP_CSORT = 16;    // 8 passes
 constexpr uint32_t EP_CELLS = 24;
-constexpr uint32_t EP_ORDER = 32;    // first-seen order sort of the plain-xyz path, 4 passes
+constexpr uint32_t EP_ORDER = 32;    // first-seen order of the plain-xyz path
 // Work-counter slots.
 constexpr int WK_VSORT = 0;   // 8 slots
 constexpr int WK_VSEG = 8;
@@ -175,7 +175,7 @@ constexpr int WK_NORMALS = 25;
 constexpr int WK_RANGES = 26;
 constexpr int WK_BOUNDS = 27;  // blocks of k_bounds that are done
 constexpr int WK_REFINE = 28;  // queries listed for k_normals_refine
-constexpr int WK_ORDER = 32;  // 4 slots
+constexpr int WK_ORDER = 32;  // first-seen order of the plain-xyz path
 
 __device__ __forceinline__ int64_t rs_sat_i64(float t) {
   if (isnan(t)) return 0;

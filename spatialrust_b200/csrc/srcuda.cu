@@ -74,7 +74,6 @@ struct srcu_ctx {
   // plain-xyz path: gathered voxels (x, y, z, counts, keys) and first points
   DevBuf xyz_tmp;
   bool xyz_order = false;  // this chain emits voxels in first-seen order (plain xyz)
-  int occ_sort_order = 1;
   DevBuf in_aos;  // AoS (x, y, z, first attribute) copy of the chain's input
   // radius grid
   DevBuf pts, pt_cell, cell_key, cell_start, table, ranges;
@@ -546,15 +545,6 @@ cudaError_t launch_sort_kernel(cudaStream_t stream, int num_sms, int occ, const 
                                      dim3(OS_THREADS), args, sizeof(OnesweepSmem), stream);
 }
 
-template <class Src>
-srcu_status launch_sort(srcu_ctx *ctx, const Src &src, uint64_t n_max, uint32_t *hist,
-                        uint32_t epoch_off, int work_slot, SortState *st, int occ, int sort_id) {
-  Launch l(ctx, sort_id);
-  CU_TRY(launch_sort_kernel(ctx->stream, ctx->num_sms, occ, src, ctx->ctl, hist, sort_buffers(ctx),
-                            epoch_off, work_slot, st, n_max));
-  return SRCU_OK;
-}
-
 // One launch shape of the sort: C indexes kSortItems / kSortMinBlocks.
 template <class Src, int C>
 cudaError_t launch_sort_config(cudaStream_t stream, uint32_t grid_cap, const Src &src,
@@ -681,7 +671,8 @@ srcu_status launch_sort_tuned(srcu_ctx *ctx, int kind, const Src &src, uint64_t 
 }
 
 template <int NC>
-void launch_segments_nc(srcu_ctx *ctx, const float **in, uint32_t grid, const Batch &bt) {
+void launch_segments_nc(srcu_ctx *ctx, const float **in, uint32_t grid, const Batch &bt,
+                        uint32_t *starts) {
   Columns<NC> cols;
   for (int c = 0; c < NC; ++c) {
     cols.in[c] = in[c];
@@ -690,45 +681,44 @@ void launch_segments_nc(srcu_ctx *ctx, const float **in, uint32_t grid, const Ba
   k_voxel_segments<NC><<<grid, SEG_THREADS, segment_smem_bytes(NC), ctx->stream>>>(
       ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, cols, ptr<uint64_t>(ctx->vkeys),
       ptr<uint32_t>(ctx->vcounts), ptr<uint64_t>(ctx->lb_seg), ptr<const float4>(ctx->in_aos),
-      ptr<float4>(ctx->vaos), bt, ctx->agg_all);
+      ptr<float4>(ctx->vaos), starts, bt, ctx->agg_all);
+}
+
+// Buffers of the plain-xyz path: the voxels in key order, where their sorted items
+// start (in the memory of x, see k_voxel_xyz_f32) and a word per point.
+struct XyzTmp {
+  float *x, *y, *z;
+  uint32_t *counts;
+  uint64_t *keys;
+  uint32_t *mark, *starts;
+};
+srcu_status xyz_tmp(srcu_ctx *ctx, uint64_t n, XyzTmp &t) {
+  ST_TRY(ensure(ctx, ctx->xyz_tmp, std::max<uint64_t>(n, 1) * 28));
+  t.x = ptr<float>(ctx->xyz_tmp);
+  t.y = t.x + n;
+  t.z = t.y + n;
+  t.counts = reinterpret_cast<uint32_t *>(t.z + n);
+  t.keys = reinterpret_cast<uint64_t *>(t.counts + n);  // byte offset 16 n: 8-aligned
+  t.mark = reinterpret_cast<uint32_t *>(t.keys + n);
+  t.starts = reinterpret_cast<uint32_t *>(t.x);
+  return SRCU_OK;
 }
 
 // The plain-xyz path after the segment kernel: f32 centroids in input order,
 // then the voxels (columns, counts, keys, AoS copy) in first-seen order.
-srcu_status enqueue_first_seen(srcu_ctx *ctx, const float **in, uint64_t n) {
-  ST_TRY(ensure(ctx, ctx->xyz_tmp, std::max<uint64_t>(n, 1) * 28));
-  float *tx = ptr<float>(ctx->xyz_tmp);
-  float *ty = tx + n;
-  float *tz = ty + n;
-  uint32_t *tc = reinterpret_cast<uint32_t *>(tz + n);
-  uint64_t *tk = reinterpret_cast<uint64_t *>(tc + n);  // byte offset 16 n: 8-aligned
-  uint32_t *first = reinterpret_cast<uint32_t *>(tk + n);
+srcu_status enqueue_first_seen(srcu_ctx *ctx, const XyzTmp &tmp, uint64_t n) {
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), ctx->num_sms * 8));
-  {
-    Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
-    k_voxel_xyz_f32<<<grid, 256, 0, ctx->stream>>>(
-        ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, in[0], in[1], in[2],
-        ptr<uint64_t>(ctx->vkeys), ptr<uint32_t>(ctx->vcounts), ptr<float>(ctx->vout[0]),
-        ptr<float>(ctx->vout[1]), ptr<float>(ctx->vout[2]), first);
-    CU_TRY(cudaGetLastError());
-  }
-  // The voxel sort is consumed: its histogram is reused, zeroed, by the order
-  // sort, whose state is the cell sort's (the cell sort, if any, comes after).
-  CU_TRY(cudaMemsetAsync(ctx->ctl->hist_v, 0, sizeof(ctx->ctl->hist_v), ctx->stream));
-  FirstSeenSrc src;
-  src.first = first;
-  src.bits = n > 1 ? bit_width_u64(n - 1) : 0u;
-  ST_TRY(launch_sort(ctx, src, n, ctx->ctl->hist_v, EP_ORDER, WK_ORDER, &ctx->ctl->csort,
-                     ctx->occ_sort_order, SRCU_K_VOXEL_SORT));
+  const uint32_t tiles = std::max<uint32_t>(1, ceil_div(n, SEG_TILE));
+  CU_TRY(cudaMemsetAsync(tmp.mark, 0, n * 4, ctx->stream));
   Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
-  k_voxel_first_seen_gather<<<grid, 256, 0, ctx->stream>>>(
-      ctx->ctl, sort_buffers(ctx), &ctx->ctl->csort, ptr<float>(ctx->vout[0]),
-      ptr<float>(ctx->vout[1]), ptr<float>(ctx->vout[2]), ptr<uint32_t>(ctx->vcounts),
-      ptr<uint64_t>(ctx->vkeys), tx, ty, tz, tc, tk);
-  k_voxel_copy_back<<<grid, 256, 0, ctx->stream>>>(
-      ctx->ctl, tx, ty, tz, tc, tk, ptr<float>(ctx->vout[0]), ptr<float>(ctx->vout[1]),
-      ptr<float>(ctx->vout[2]), ptr<uint32_t>(ctx->vcounts), ptr<uint64_t>(ctx->vkeys),
-      ptr<float4>(ctx->vaos));
+  k_voxel_xyz_f32<<<grid, 256, 0, ctx->stream>>>(
+      ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, ptr<const float4>(ctx->in_aos),
+      ptr<uint64_t>(ctx->vkeys), ptr<uint32_t>(ctx->vcounts), tmp.starts, tmp.x, tmp.y, tmp.z,
+      tmp.counts, tmp.keys, tmp.mark);
+  k_voxel_first_seen<<<std::min(tiles, uint32_t(ctx->num_sms) * 8), SEG_THREADS, 0, ctx->stream>>>(
+      ctx->ctl, tmp.mark, ptr<uint64_t>(ctx->lb_seg), tmp.x, tmp.y, tmp.z, tmp.counts, tmp.keys,
+      ptr<float>(ctx->vout[0]), ptr<float>(ctx->vout[1]), ptr<float>(ctx->vout[2]),
+      ptr<uint32_t>(ctx->vcounts), ptr<uint64_t>(ctx->vkeys), ptr<float4>(ctx->vaos));
   CU_TRY(cudaGetLastError());
   return SRCU_OK;
 }
@@ -767,25 +757,28 @@ srcu_status enqueue_voxel(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t
                            ctx->occ_sort_v, SRCU_K_VOXEL_SORT));
   const uint32_t tiles = std::max<uint32_t>(1, ceil_div(n, SEG_TILE));
   const uint32_t grid = std::min<uint32_t>(tiles, uint32_t(ctx->num_sms) * uint32_t(ctx->occ_seg));
+  const bool first_seen = ctx->xyz_order && bt.clouds == 1;
+  XyzTmp tmp{};
+  if (first_seen) ST_TRY(xyz_tmp(ctx, n, tmp));
   Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
   switch (nc) {
-    case 3: launch_segments_nc<3>(ctx, in, grid, bt); break;
-    case 4: launch_segments_nc<4>(ctx, in, grid, bt); break;
-    case 5: launch_segments_nc<5>(ctx, in, grid, bt); break;
-    case 6: launch_segments_nc<6>(ctx, in, grid, bt); break;
-    case 7: launch_segments_nc<7>(ctx, in, grid, bt); break;
-    case 8: launch_segments_nc<8>(ctx, in, grid, bt); break;
-    case 9: launch_segments_nc<9>(ctx, in, grid, bt); break;
-    case 10: launch_segments_nc<10>(ctx, in, grid, bt); break;
-    case 11: launch_segments_nc<11>(ctx, in, grid, bt); break;
-    case 12: launch_segments_nc<12>(ctx, in, grid, bt); break;
+    case 3: launch_segments_nc<3>(ctx, in, grid, bt, tmp.starts); break;
+    case 4: launch_segments_nc<4>(ctx, in, grid, bt, tmp.starts); break;
+    case 5: launch_segments_nc<5>(ctx, in, grid, bt, tmp.starts); break;
+    case 6: launch_segments_nc<6>(ctx, in, grid, bt, tmp.starts); break;
+    case 7: launch_segments_nc<7>(ctx, in, grid, bt, tmp.starts); break;
+    case 8: launch_segments_nc<8>(ctx, in, grid, bt, tmp.starts); break;
+    case 9: launch_segments_nc<9>(ctx, in, grid, bt, tmp.starts); break;
+    case 10: launch_segments_nc<10>(ctx, in, grid, bt, tmp.starts); break;
+    case 11: launch_segments_nc<11>(ctx, in, grid, bt, tmp.starts); break;
+    case 12: launch_segments_nc<12>(ctx, in, grid, bt, tmp.starts); break;
     default: return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "unsupported column count %u", nc);
   }
   if (bt.clouds > 1)  // one cloud's range is [0, V), read from the control block
     k_voxel_offsets<<<ceil_div(bt.clouds + 1, 128), 128, 0, ctx->stream>>>(
         ctx->ctl, ptr<uint64_t>(ctx->vkeys), bt);
   CU_TRY(cudaGetLastError());
-  if (ctx->xyz_order && bt.clouds == 1) ST_TRY(enqueue_first_seen(ctx, in, n));
+  if (first_seen) ST_TRY(enqueue_first_seen(ctx, tmp, n));
   return SRCU_OK;
 }
 
@@ -1136,8 +1129,7 @@ srcu_status srcu_create(int device, uint64_t hbm_budget_bytes, srcu_ctx **out) {
   // Kernels with more than 48 KB of dynamic shared memory opt in once; every
   // sort launch shape, with its co-resident block count.
   if (sort_setup<VoxelKeySrc>(ctx->occ_sort_v) != cudaSuccess ||
-      sort_setup<CellKeySrc>(ctx->occ_sort_c) != cudaSuccess ||
-      sort_config_setup<FirstSeenSrc, 0>(&ctx->occ_sort_order) != cudaSuccess)
+      sort_setup<CellKeySrc>(ctx->occ_sort_c) != cudaSuccess)
     return bail(SRCU_ERR_CUDA);
   for (int kind = 0; kind < SRCU_SORT_KINDS; ++kind) builtin_sort_tuning(ctx, kind);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&ctx->occ_normals, k_normals<true>, NM_THREADS, 0);

@@ -333,8 +333,19 @@ __device__ __forceinline__ int32_t voxel_agg(const Batch &bt, uint64_t key, uint
   return bt.vparams[b < bt.clouds ? b : 0].agg;
 }
 
+// Where k_voxel_segments writes a voxel besides its columns.
+struct VoxelDst {
+  uint64_t *keys;
+  uint32_t *counts;
+  float4 *aos;       // may be null
+  uint32_t *starts;  // each voxel's first sorted position; may be null
+  uint32_t n;
+  uint32_t *status;
+};
+
 // Writes columns C0 .. C0 + G - 1 of one voxel, and with column 0 its key, count and
-// AoS record.  s: their FP64 sums in ascending point order; inv: 1.0 / cnt; first(c): column c of
+// AoS record.  s: their FP64 sums in ascending point order; inv: 1.0 / cnt; pos: its
+// first sorted position; first(c): column c of
 // the voxel's first point, read only by the modes that use it (so the default
 // mode keeps no extra registers live).
 //   AGG_FAST            (sum * (1.0 / count)) as f32, voxel.rs:531-536
@@ -344,11 +355,10 @@ __device__ __forceinline__ int32_t voxel_agg(const Batch &bt, uint64_t key, uint
 template <int NC, int C0, int G, class First>
 __device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const double (&s)[G],
                                                First first, int32_t agg, double inv,
-                                               uint32_t cnt, uint32_t seg, uint64_t key,
-                                               uint64_t *out_keys, uint32_t *out_counts,
-                                               uint32_t n, uint32_t *status, float4 *aos_out) {
-  if (seg >= n) {  // cannot happen for a consistent sort; never write out of bounds
-    atomicOr(status, ST_INTERNAL);
+                                               uint32_t pos, uint32_t cnt, uint32_t seg,
+                                               uint64_t key, const VoxelDst &dst) {
+  if (seg >= dst.n) {  // cannot happen for a consistent sort; never write out of bounds
+    atomicOr(dst.status, ST_INTERNAL);
     return;
   }
   float o[G];
@@ -362,9 +372,10 @@ __device__ __forceinline__ void write_centroid(const Columns<NC> &cols, const do
     cols.out[c][seg] = o[g];
   }
   if (C0 > 0) return;
-  if (aos_out) aos_out[seg] = make_float4(o[0], o[1], o[2], 0.0f);
-  out_keys[seg] = key;
-  out_counts[seg] = cnt;
+  if (dst.aos) dst.aos[seg] = make_float4(o[0], o[1], o[2], 0.0f);
+  if (dst.starts) dst.starts[seg] = pos;
+  dst.keys[seg] = key;
+  dst.counts[seg] = cnt;
 }
 
 // Columns 0 .. 3 of the points iv[]: from the AoS copy, one sector per point, where
@@ -425,11 +436,10 @@ __device__ __forceinline__ void gather_more(const uint32_t (&iv)[SEG_ITEMS], con
 // Columns from C0 on, SEG_GROUP at a time, of the short voxel at tile positions [j, e):
 // sums in ascending point index.
 template <int NC, int C0>
-__device__ __forceinline__ void short_voxel(const SegmentSmemHead &sm, const float *scol, uint32_t j,
-                                            uint32_t e, uint32_t seg, uint64_t key,
-                                            const Columns<NC> &cols, int32_t agg,
-                                            uint64_t *out_keys, uint32_t *out_counts, uint32_t n,
-                                            uint32_t *status, float4 *aos_out) {
+__device__ __forceinline__ void short_voxel(const SegmentSmemHead &sm, const float *scol,
+                                            uint32_t base, uint32_t j, uint32_t e, uint32_t seg,
+                                            uint64_t key, const Columns<NC> &cols, int32_t agg,
+                                            const VoxelDst &dst) {
   constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
   double s[G];
 #pragma unroll
@@ -440,19 +450,18 @@ __device__ __forceinline__ void short_voxel(const SegmentSmemHead &sm, const flo
     for (int g = 0; g < G; ++g) s[g] += double(scol[(C0 + g) * SEG_TILE + m]);
   }
   write_centroid<NC, C0, G>(cols, s, [&](int c) { return scol[c * SEG_TILE + j]; }, agg,
-                            sm.inv[e - j], e - j, seg, key, out_keys, out_counts, n, status, aos_out);
+                            sm.inv[e - j], base + j, e - j, seg, key, dst);
   if constexpr (C0 + SEG_GROUP < NC)
-    short_voxel<NC, C0 + SEG_GROUP>(sm, scol, j, e, seg, key, cols, agg, out_keys, out_counts, n,
-                                    status, aos_out);
+    short_voxel<NC, C0 + SEG_GROUP>(sm, scol, base, j, e, seg, key, cols, agg, dst);
 }
 
 // The columns of one voxel from C0 on, its sorted items [p, e) reduced by a warp.
 template <int NC, int C0>
 __device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uint32_t e, uint32_t seg,
                                            uint64_t key, const Columns<NC> &cols, int32_t agg,
-                                           uint64_t *out_keys, uint32_t *out_counts, uint32_t n,
-                                           uint32_t *status, float4 *aos_out) {
+                                           const VoxelDst &dst) {
   constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
+  const uint32_t n = dst.n;
   const uint32_t lane = threadIdx.x & 31u;
   double s[G];
 #pragma unroll
@@ -460,7 +469,7 @@ __device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uin
   for (uint32_t m = p + lane; m < e; m += 32) {
     const uint32_t v = sv.val(m);
     if (v >= n) {
-      atomicOr(status, ST_INTERNAL);
+      atomicOr(dst.status, ST_INTERNAL);
       continue;
     }
 #pragma unroll
@@ -476,12 +485,10 @@ __device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uin
       const uint32_t v0 = sv.val(p);
       return v0 < n ? cols.in[c][v0] : 0.0f;
     };
-    write_centroid<NC, C0, G>(cols, s, first, agg, 1.0 / double(e - p), e - p, seg, key, out_keys,
-                              out_counts, n, status, aos_out);
+    write_centroid<NC, C0, G>(cols, s, first, agg, 1.0 / double(e - p), p, e - p, seg, key, dst);
   }
   if constexpr (C0 + SEG_GROUP < NC)
-    long_voxel<NC, C0 + SEG_GROUP>(sv, p, e, seg, key, cols, agg, out_keys, out_counts, n, status,
-                                   aos_out);
+    long_voxel<NC, C0 + SEG_GROUP>(sv, p, e, seg, key, cols, agg, dst);
 }
 
 // Fused segment discovery + FP64 centroid reduction over the sorted
@@ -507,7 +514,8 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
                                                                  uint32_t *out_counts,
                                                                  uint64_t *lookback,
                                                                  const float4 *aos_in,
-                                                                 float4 *aos_out, Batch bt,
+                                                                 float4 *aos_out,
+                                                                 uint32_t *out_starts, Batch bt,
                                                                  int32_t agg_all) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   SegmentSmemHead &sm = *reinterpret_cast<SegmentSmemHead *>(smem_raw);
@@ -521,6 +529,7 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
   const uint32_t t = threadIdx.x, lane = t & 31u;
 
   const uint32_t vkey_bits = ctl->vkey_bits;
+  const VoxelDst dst = {out_keys, out_counts, aos_out, out_starts, n, &ctl->status};
   if (t == 0) sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
   if (t >= 32 && t <= 32 + SEG_SHORT) sm.inv[t - 32] = 1.0 / double(t - 32);
 
@@ -613,9 +622,8 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
       if (e - j > SEG_SHORT || sm.keys[1 + e] == key)
         sm.longs[atomicAdd(&sm.num_longs, 1u)] = uint16_t(q);
       else
-        short_voxel<NC, 0>(sm, scol, j, e, sm.seg_base + q, key, cols,
-                           voxel_agg(bt, key, vkey_bits, agg_all), out_keys, out_counts, n,
-                           &ctl->status, aos_out);
+        short_voxel<NC, 0>(sm, scol, base, j, e, sm.seg_base + q, key, cols,
+                           voxel_agg(bt, key, vkey_bits, agg_all), dst);
     }
     __syncthreads();
     // Long voxels: a warp finds the end and reduces from global memory.
@@ -635,8 +643,7 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
         e += 32;
       }
       long_voxel<NC, 0>(sv, base + j, e, sm.seg_base + q, key, cols,
-                        voxel_agg(bt, key, vkey_bits, agg_all), out_keys, out_counts, n,
-                        &ctl->status, aos_out);
+                        voxel_agg(bt, key, vkey_bits, agg_all), dst);
     }
   }
 }
@@ -665,109 +672,117 @@ inline cudaError_t configure_segment_kernels() {
 // runs for clouds whose only fields are x, y, z: per voxel it sums x, y, z in
 // f32 in input order, emits sum * (1 / count) in f32, and emits the voxels in
 // the order of their first point.  After the segment kernel (same voxels, same
-// counts, key order), k_voxel_xyz_f32 recomputes those sums -- the stable sort
-// keeps each voxel's points in input order -- and records each voxel's first
-// point; a sort of the voxels by first point (FirstSeenSrc) and a gather then
-// put them in first-seen order.
+// counts, key order, and where each voxel's sorted items start), k_voxel_xyz_f32
+// recomputes those sums -- the stable sort keeps each voxel's points in input
+// order -- and marks each voxel's first point with the voxel; the count of marks
+// before a point is then its voxel's place, so one scan over the points
+// (k_voxel_first_seen) puts the voxels in first-seen order, without a sort.
+// Both kernels are bound by the latency of their gathers (11 and 21 us at 300k points
+// with cold caches).  With a sort of the voxels by first point (40 us alone), a
+// gather, a copy back and a binary search per voxel in their place, a call from
+// host memory took 663 us; it takes 612.
 
-// One thread per voxel start among the sorted items.
-__global__ void k_voxel_xyz_f32(Control *ctl, SortBuffers sort, const SortState *sort_state,
-                                const float *x, const float *y, const float *z,
-                                const uint64_t *vkeys, const uint32_t *vcounts, float *ox,
-                                float *oy, float *oz, uint32_t *first) {
+// One thread per voxel.  `starts` and tx may be the same memory: a thread reads its
+// start before it writes.  mark: a word per point, zeroed.
+__global__ void __launch_bounds__(256) k_voxel_xyz_f32(Control *ctl, SortBuffers sort,
+                                                       const SortState *sort_state,
+                                                       const float4 *aos, const uint64_t *vkeys,
+                                                       const uint32_t *vcounts,
+                                                       const uint32_t *starts, float *tx, float *ty,
+                                                       float *tz, uint32_t *tc, uint64_t *tk,
+                                                       uint32_t *mark) {
   if (ld_relaxed_u32(&ctl->status)) return;
   const uint32_t n = uint32_t(ctl->n_points);
   const uint32_t nv = uint32_t(ctl->n_voxels);
   const SortedView sv = sorted_view(sort, *sort_state);
-  for (uint32_t m = blockIdx.x * blockDim.x + threadIdx.x; m < n; m += gridDim.x * blockDim.x) {
-    const uint64_t key = sv.key(m);
-    if (m > 0 && sv.key(m - 1) == key) continue;
-    uint32_t lo = 0, hi = nv;  // the voxel of this key among the key-ordered voxels
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (vkeys[mid] < key) lo = mid + 1;
-      else hi = mid;
-    }
-    if (lo >= nv || vkeys[lo] != key || vcounts[lo] == 0 || vcounts[lo] > n - m) {
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
+    const uint32_t m = starts[v], cnt = vcounts[v];
+    const uint64_t key = vkeys[v];
+    if (m >= n || cnt == 0 || cnt > n - m) {
       atomicOr(&ctl->status, ST_INTERNAL);  // cannot happen for a consistent chain
       continue;
     }
-    const uint32_t cnt = vcounts[lo];
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    uint32_t i0 = 0;
     bool ok = true;
+#pragma unroll 4
     for (uint32_t q = 0; q < cnt; ++q) {
       const uint32_t i = sv.val(m + q);
-      if (i >= n) {
-        ok = false;
-        break;
-      }
-      if (q == 0) i0 = i;
-      sx = __fadd_rn(sx, x[i]);
-      sy = __fadd_rn(sy, y[i]);
-      sz = __fadd_rn(sz, z[i]);
+      ok &= i < n;
+      const float4 p = i < n ? aos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+      sx = __fadd_rn(sx, p.x);
+      sy = __fadd_rn(sy, p.y);
+      sz = __fadd_rn(sz, p.z);
     }
     if (!ok) {
       atomicOr(&ctl->status, ST_INTERNAL);
       continue;
     }
     const float inv = 1.0f / float(cnt);  // IEEE division: the library is built without fast math
-    ox[lo] = __fmul_rn(sx, inv);
-    oy[lo] = __fmul_rn(sy, inv);
-    oz[lo] = __fmul_rn(sz, inv);
-    first[lo] = i0;
+    tx[v] = __fmul_rn(sx, inv);
+    ty[v] = __fmul_rn(sy, inv);
+    tz[v] = __fmul_rn(sz, inv);
+    tc[v] = cnt;
+    tk[v] = key;
+    mark[sv.val(m)] = v + 1;
   }
 }
 
-// Sort key of the first-seen order: each voxel's first point index.
-struct FirstSeenSrc {
-  const uint32_t *first;
-  uint32_t bits;  // bits of the largest point index
-  __device__ __forceinline__ void prepare(const Control *) {}
-  __device__ __forceinline__ uint32_t count(const Control *ctl) const {
-    return uint32_t(ctl->n_voxels);
-  }
-  __device__ __forceinline__ uint32_t key_bits() const { return bits; }
-  __device__ __forceinline__ uint64_t key(uint32_t v) const { return first[v]; }
-};
-
-// Voxel j of the first-seen order <- voxel val(j) of the key order.
-__global__ void k_voxel_first_seen_gather(Control *ctl, SortBuffers sort, const SortState *order,
-                                          const float *ix, const float *iy, const float *iz,
-                                          const uint32_t *icnt, const uint64_t *ikey, float *ox,
-                                          float *oy, float *oz, uint32_t *ocnt, uint64_t *okey) {
+// The voxels into the chain's buffers (and the AoS copy the normals stage reads) in
+// the order of their marks: a count of marks over tiles of SEG_TILE points, with a
+// look-back, a thread to four consecutive points.
+__global__ void __launch_bounds__(SEG_THREADS) k_voxel_first_seen(
+    Control *ctl, const uint32_t *mark, uint64_t *lookback, const float *tx, const float *ty,
+    const float *tz, const uint32_t *tc, const uint64_t *tk, float *ox, float *oy, float *oz,
+    uint32_t *ocnt, uint64_t *okey, float4 *oaos) {
+  __shared__ uint32_t scratch[SEG_THREADS / 32];
+  __shared__ uint32_t s_tile, s_base;
   if (ld_relaxed_u32(&ctl->status)) return;
+  const uint32_t n = uint32_t(ctl->n_points);
   const uint32_t nv = uint32_t(ctl->n_voxels);
-  const SortedView sv = sorted_view(sort, *order);
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nv; j += gridDim.x * blockDim.x) {
-    const uint32_t v = sv.val(j);
-    if (v >= nv) {
-      atomicOr(&ctl->status, ST_INTERNAL);
-      continue;
+  const uint32_t num_tiles = (n + SEG_TILE - 1) / SEG_TILE;
+  const uint32_t t = threadIdx.x;
+  if (t == 0) s_tile = atomicAdd(&ctl->work[WK_ORDER], 1u);
+  for (;;) {
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile >= num_tiles) break;
+    const uint32_t i0 = tile * SEG_TILE + t * SEG_ITEMS;
+    uint32_t v[SEG_ITEMS], marks = 0;
+#pragma unroll
+    for (int q = 0; q < SEG_ITEMS; ++q) v[q] = i0 + q < n ? mark[i0 + q] : 0u;
+#pragma unroll
+    for (int q = 0; q < SEG_ITEMS; ++q) marks += v[q] != 0;
+    uint32_t total;
+    const uint32_t local = block_exclusive_sum<SEG_THREADS>(marks, scratch, &total);
+    if (t < 32) {
+      const uint32_t base = lookback_exclusive_warp(lookback, tile, total, ctl->epoch + EP_ORDER,
+                                                    &ctl->status, num_tiles <= gridDim.x);
+      if (t == 0) {
+        s_base = base;
+        s_tile = atomicAdd(&ctl->work[WK_ORDER], 1u);  // the next one
+        // every voxel has marked one point
+        if (tile == num_tiles - 1 && base + total != nv) atomicOr(&ctl->status, ST_INTERNAL);
+      }
     }
-    ox[j] = ix[v];
-    oy[j] = iy[v];
-    oz[j] = iz[v];
-    ocnt[j] = icnt[v];
-    okey[j] = ikey[v];
-  }
-}
-
-// The gathered voxels back into the chain's voxel buffers (and the AoS copy
-// the normals stage reads).
-__global__ void k_voxel_copy_back(const Control *ctl, const float *ix, const float *iy,
-                                  const float *iz, const uint32_t *icnt, const uint64_t *ikey,
-                                  float *ox, float *oy, float *oz, uint32_t *ocnt, uint64_t *okey,
-                                  float4 *aos) {
-  if (ld_relaxed_u32(&ctl->status)) return;
-  const uint32_t nv = uint32_t(ctl->n_voxels);
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < nv; j += gridDim.x * blockDim.x) {
-    ox[j] = ix[j];
-    oy[j] = iy[j];
-    oz[j] = iz[j];
-    ocnt[j] = icnt[j];
-    okey[j] = ikey[j];
-    if (aos) aos[j] = make_float4(ix[j], iy[j], iz[j], 0.0f);
+    __syncthreads();
+    uint32_t j = s_base + local;
+#pragma unroll
+    for (int q = 0; q < SEG_ITEMS; ++q) {
+      if (v[q] == 0) continue;
+      const uint32_t u = v[q] - 1;
+      if (u < nv && j < nv) {
+        const float x = tx[u], y = ty[u], z = tz[u];
+        ox[j] = x;
+        oy[j] = y;
+        oz[j] = z;
+        if (oaos) oaos[j] = make_float4(x, y, z, 0.0f);
+        ocnt[j] = tc[u];
+        okey[j] = tk[u];
+      } else {
+        atomicOr(&ctl->status, ST_INTERNAL);
+      }
+      ++j;
+    }
   }
 }
 

@@ -47,6 +47,15 @@ def test_shuffled_scan_bit_exact(cuda_ctx, leaf):
     assert counts.max() > 1
 
 
+# the first-seen scan takes tiles of 1024 points: their edges, more tiles than a wave
+# of blocks holds, and voxels of one point, of a few and of very many
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 2049, 150_001, 1_400_000])
+@pytest.mark.parametrize("leaf", [0.02, 3.0])
+def test_first_seen_scan_at_tile_edges(cuda_ctx, n, leaf):
+    x, y, z = shuffled_scan(n, seed=n % 97)
+    check(cuda_ctx, x, y, z, leaf)
+
+
 def test_explicit_origin_negative_keys(cuda_ctx):
     x, y, z = shuffled_scan(200_000, 32)
     check(cuda_ctx, x - F(50), y - F(80), z, 0.25, origin=(0.0, 0.0, 0.0))

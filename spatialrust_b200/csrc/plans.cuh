@@ -215,13 +215,14 @@ __host__ __device__ __forceinline__ void voxel_unpack(const VoxelPlan &pl, uint6
   out[2] = int64_t(oz + uint64_t(pl.kmin[2]));
 }
 
+// floor((p - o) * inv_h) held to [0, dim - 1]; 0 where p is not finite (never a
+// neighbour: the f32 predicate is false for it).  The saturating conversion cuts
+// towards zero, which is the floor of all that is not held to 0.  The sort's first
+// phase is bound by this arithmetic: with a floor and two FP64 comparisons an axis
+// instead, the sort of 13.9M cell keys took 720 us, 689 so.
 __device__ __forceinline__ uint32_t cell_axis(float p, double o, double inv_h, uint32_t dim) {
-  if (!isfinite(p)) return 0;  // never a neighbour: the f32 predicate is false for it
-  double u = (double(p) - o) * inv_h;
-  double f = floor(u);
-  if (!(f > 0.0)) return 0;
-  if (f >= double(dim - 1)) return dim - 1;
-  return uint32_t(f);
+  const uint32_t f = min(__double2uint_rz((double(p) - o) * inv_h), dim - 1);
+  return isfinite(p) ? f : 0u;
 }
 
 __device__ __forceinline__ uint64_t cell_pack(const CellPlan &pl, float x, float y, float z) {

@@ -996,6 +996,20 @@ bool takable(const srcu_ctx *ctx, const DevBuf &b, uint32_t words = 1) {
   return b.p && b.bytes >= size_t(ctx->last_points) * words * 4;
 }
 
+// Whether a kernel of this context can write 32-bit words to dst: this GPU's own or
+// managed memory, word-aligned.  Whatever else a caller passes as device memory is
+// left to a copy, which takes any alignment and refuses what it cannot reach.
+bool writable(const srcu_ctx *ctx, const void *dst) {
+  if (reinterpret_cast<uintptr_t>(dst) & 3u) return false;
+  cudaPointerAttributes at;
+  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  return at.type == cudaMemoryTypeManaged ||
+         (at.type == cudaMemoryTypeDevice && at.device == ctx->device);
+}
+
 void take_column(TakeColumns &t, void *dst, const void *src, uint32_t words) {
   if (!dst) return;
   t.src[t.count] = static_cast<const uint32_t *>(src);
@@ -1005,7 +1019,13 @@ void take_column(TakeColumns &t, void *dst, const void *src, uint32_t words) {
 
 void take_result(const srcu_ctx *ctx, TakeColumns &t, void *dst, const DevBuf &src,
                  uint32_t words = 1) {
-  if (takable(ctx, src, words)) take_column(t, dst, src.p, words);
+  if (dst && takable(ctx, src, words) && writable(ctx, dst)) take_column(t, dst, src.p, words);
+}
+
+bool taken(const TakeColumns &t, const void *dst, const void *src) {
+  for (uint32_t c = 0; c < t.count; ++c)
+    if (t.dst[c] == dst && t.src[c] == src) return true;
+  return false;
 }
 
 srcu_status take_columns(srcu_ctx *ctx, const TakeColumns &t, const unsigned long long *rows,
@@ -1020,10 +1040,11 @@ srcu_status take_columns(srcu_ctx *ctx, const TakeColumns &t, const unsigned lon
 
 // Queues the copies of the chain's results that go to device memory, their
 // row count (`rows`, a device word) unread: they run before the wait for the
-// control block, and not at all when the chain failed.
+// control block, and not at all when the chain failed.  t says which were queued.
 srcu_status take_results(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *vout,
-                         const srcu_normal_out *nout, const unsigned long long *rows) {
-  TakeColumns t{};
+                         const srcu_normal_out *nout, const unsigned long long *rows,
+                         TakeColumns &t) {
+  t.count = 0;
   if (vout && vout->on_device) {
     float *dst[MAX_COLS] = {vout->x, vout->y, vout->z};
     for (uint32_t a = 3; a < nc; ++a) dst[a] = vout->attrs ? vout->attrs[a - 3] : nullptr;
@@ -1040,31 +1061,33 @@ srcu_status take_results(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *vout,
 }
 
 // One result column of `rows` rows, unless take_results took it.
-srcu_status fetch_column(srcu_ctx *ctx, void *dst, const DevBuf &src, uint64_t rows, int on_device,
-                         cudaStream_t stream = nullptr, uint32_t words = 1) {
-  if (on_device && takable(ctx, src, words)) return SRCU_OK;
+srcu_status fetch_column(srcu_ctx *ctx, const TakeColumns &t, void *dst, const DevBuf &src,
+                         uint64_t rows, int on_device, cudaStream_t stream = nullptr,
+                         uint32_t words = 1) {
+  if (on_device && taken(t, dst, src.p)) return SRCU_OK;
   return copy_out(ctx, dst, src.p, rows * words * 4, on_device, stream);
 }
 
 // The results take_results left, once their row count is known.
-srcu_status fetch_voxels(srcu_ctx *ctx, uint32_t nc, const srcu_voxel_out *out, uint64_t v,
-                         cudaStream_t stream = nullptr, bool keys = true) {
+srcu_status fetch_voxels(srcu_ctx *ctx, const TakeColumns &t, uint32_t nc, const srcu_voxel_out *out,
+                         uint64_t v, cudaStream_t stream = nullptr, bool keys = true) {
   if (!out) return SRCU_OK;
   float *dst[MAX_COLS] = {out->x, out->y, out->z};
   for (uint32_t a = 3; a < nc; ++a) dst[a] = out->attrs ? out->attrs[a - 3] : nullptr;
   for (uint32_t c = 0; c < nc; ++c)
-    ST_TRY(fetch_column(ctx, dst[c], ctx->vout[c], v, out->on_device, stream));
-  ST_TRY(fetch_column(ctx, out->counts, ctx->vcounts, v, out->on_device, stream));
-  if (keys) ST_TRY(fetch_column(ctx, out->keys, ctx->vkeys3, v, out->on_device, stream, 6));
+    ST_TRY(fetch_column(ctx, t, dst[c], ctx->vout[c], v, out->on_device, stream));
+  ST_TRY(fetch_column(ctx, t, out->counts, ctx->vcounts, v, out->on_device, stream));
+  if (keys) ST_TRY(fetch_column(ctx, t, out->keys, ctx->vkeys3, v, out->on_device, stream, 6));
   return SRCU_OK;
 }
 
-srcu_status fetch_normals(srcu_ctx *ctx, const srcu_normal_out *out, uint64_t m,
+srcu_status fetch_normals(srcu_ctx *ctx, const TakeColumns &t, const srcu_normal_out *out, uint64_t m,
                           srcu_normal_stats *stats) {
   if (out) {
     float *dst[4] = {out->nx, out->ny, out->nz, out->curvature};
-    for (int c = 0; c < 4; ++c) ST_TRY(fetch_column(ctx, dst[c], ctx->nout[c], m, out->on_device));
-    ST_TRY(fetch_column(ctx, out->neighbor_counts, ctx->ncounts, m, out->on_device));
+    for (int c = 0; c < 4; ++c)
+      ST_TRY(fetch_column(ctx, t, dst[c], ctx->nout[c], m, out->on_device));
+    ST_TRY(fetch_column(ctx, t, out->neighbor_counts, ctx->ncounts, m, out->on_device));
   }
   if (stats) {
     stats->valid_count = ctx->ctl_host->ncount.valid;
@@ -1312,10 +1335,11 @@ srcu_status srcu_voxel_centroid(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(begin_chain(ctx, n, bt, 1, params, nullptr));
   ST_TRY(enqueue_voxel(ctx, cols, nc, n, bt, false));
   if (out && out->keys) ST_TRY(unpack_keys(ctx, n));
-  ST_TRY(take_results(ctx, nc, out, nullptr, &ctx->ctl->n_voxels));
+  TakeColumns take;
+  ST_TRY(take_results(ctx, nc, out, nullptr, &ctx->ctl->n_voxels, take));
   ST_TRY(read_control(ctx));
   const uint64_t v = ctx->ctl_host->n_voxels;
-  ST_TRY(fetch_voxels(ctx, nc, out, v));
+  ST_TRY(fetch_voxels(ctx, take, nc, out, v));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   if (out_voxels) *out_voxels = v;
   return SRCU_OK;
@@ -1342,9 +1366,10 @@ srcu_status srcu_radius_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
   ST_TRY(enqueue_bounds(ctx, cols, 3, n, bt, false, true));
   ST_TRY(enqueue_normals(ctx, cols[0], cols[1], cols[2], ptr<const float4>(ctx->in_aos), nullptr, n,
                          bt, nullptr));
-  ST_TRY(take_results(ctx, 3, nullptr, out, &ctx->ctl->n_points));
+  TakeColumns take;
+  ST_TRY(take_results(ctx, 3, nullptr, out, &ctx->ctl->n_points, take));
   ST_TRY(read_control(ctx));
-  ST_TRY(fetch_normals(ctx, out, n, stats));
+  ST_TRY(fetch_normals(ctx, take, out, n, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   return SRCU_OK;
 }
@@ -1440,7 +1465,7 @@ srcu_status srcu_plane_covariances(srcu_ctx *ctx, const srcu_cloud *cloud, float
   CU_TRY(cudaGetLastError());
   ST_TRY(read_control(ctx));
   if (!cloud->on_device) ST_TRY(copy_out(ctx, cov, dst, n * 24, 0));
-  ST_TRY(fetch_normals(ctx, nullptr, n, stats));
+  ST_TRY(fetch_normals(ctx, TakeColumns{}, nullptr, n, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   return SRCU_OK;
 }
@@ -1478,14 +1503,15 @@ srcu_status srcu_voxel_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
                          ptr<float>(ctx->vout[2]), ptr<const float4>(ctx->vaos),
                          &ctx->ctl->n_voxels, n, bt, ptr<uint64_t>(ctx->vkeys)));
   if (vout && vout->keys) ST_TRY(unpack_keys(ctx, n));
-  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels));
+  TakeColumns take;
+  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels, take));
   bool early = false;
   if (vout && !vout->on_device) {
     CU_TRY(cudaEventSynchronize(ctx->ev_voxel));
     const Control *head = reinterpret_cast<const Control *>(ctx->head_host);
     if (head->status == 0) {  // otherwise read_control below reports the failure
       CU_TRY(cudaStreamWaitEvent(ctx->side_stream, ctx->ev_voxel, 0));
-      ST_TRY(fetch_voxels(ctx, nc, vout, head->n_voxels, ctx->side_stream, false));
+      ST_TRY(fetch_voxels(ctx, take, nc, vout, head->n_voxels, ctx->side_stream, false));
       early = true;
     }
   }
@@ -1493,9 +1519,9 @@ srcu_status srcu_voxel_normals(srcu_ctx *ctx, const srcu_cloud *cloud,
   if (early && st != SRCU_OK) cudaStreamSynchronize(ctx->side_stream);  // no copy outlives the call
   if (st != SRCU_OK) return st;
   const uint64_t v = ctx->ctl_host->n_voxels;
-  if (!early) ST_TRY(fetch_voxels(ctx, nc, vout, v));
+  if (!early) ST_TRY(fetch_voxels(ctx, take, nc, vout, v));
   else if (vout->keys) ST_TRY(copy_out(ctx, vout->keys, ctx->vkeys3.p, v * 24, 0));
-  ST_TRY(fetch_normals(ctx, nout, v, stats));
+  ST_TRY(fetch_normals(ctx, take, nout, v, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   if (early) CU_TRY(cudaStreamSynchronize(ctx->side_stream));
   if (out_voxels) *out_voxels = v;
@@ -1712,7 +1738,7 @@ srcu_status srcu_frame_check(srcu_ctx *ctx, uint64_t *out_voxels, srcu_normal_st
   if (!ctx) return SRCU_ERR_INVALID_ARGUMENT;
   ST_TRY(read_control(ctx));
   if (out_voxels) *out_voxels = ctx->ctl_host->n_voxels;
-  return fetch_normals(ctx, nullptr, 0, stats);
+  return fetch_normals(ctx, TakeColumns{}, nullptr, 0, stats);
 }
 
 srcu_status srcu_frame_fetch(srcu_ctx *ctx, const srcu_voxel_out *vout, const srcu_normal_out *nout,
@@ -1723,11 +1749,12 @@ srcu_status srcu_frame_fetch(srcu_ctx *ctx, const srcu_voxel_out *vout, const sr
     return fail(ctx, SRCU_ERR_INVALID_ARGUMENT, "frame read-back does not unpack voxel keys");
   }
   const uint32_t nc = 3 + ctx->last_attrs;
-  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels));
+  TakeColumns take;
+  ST_TRY(take_results(ctx, nc, vout, nout, &ctx->ctl->n_voxels, take));
   ST_TRY(read_control(ctx));
   const uint64_t v = ctx->ctl_host->n_voxels;
-  ST_TRY(fetch_voxels(ctx, nc, vout, v));
-  ST_TRY(fetch_normals(ctx, nout, v, stats));
+  ST_TRY(fetch_voxels(ctx, take, nc, vout, v));
+  ST_TRY(fetch_normals(ctx, take, nout, v, stats));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   if (out_voxels) *out_voxels = v;
   return SRCU_OK;

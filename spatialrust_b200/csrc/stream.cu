@@ -442,7 +442,8 @@ srcu_status srcu_stream_voxel_fetch(srcu_stream_voxel *sv, uint64_t first, uint6
   TakeColumns t{};
   auto column = [&](void *dst, const DevBuf &src, uint32_t words) -> srcu_status {
     const uint32_t *from = static_cast<const uint32_t *>(src.p) + first * words;
-    if (!out->on_device) return copy_out(ctx, dst, from, count * words * 4, 0);
+    if (!out->on_device || !dst || !writable(ctx, dst))
+      return copy_out(ctx, dst, from, count * words * 4, out->on_device);
     take_column(t, dst, from, words);
     return SRCU_OK;
   };

@@ -205,3 +205,28 @@ def test_device_columns_off_their_alignment(cuda_ctx):
         sv.close()
     for a, b in zip(*out):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+def test_fetch_to_device_at_any_alignment(cuda_ctx, offset):
+    """Device columns that start off a word or a 16-byte boundary hold the bytes that
+    host columns hold, with nothing written past them."""
+    import ctypes
+    import torch
+    rng = np.random.default_rng(5)
+    sv = _native.StreamVoxel(cuda_ctx, 0.5, [True])
+    sv.push(*rng.uniform(0, 9, (3, 3000)).astype(F), [rng.normal(0, 1, 3000)])
+    sv.finish()
+    x, y, z, a, keys, counts = sv.fetch()
+    want = [x, y, z, a[:, 0], keys, counts]
+    bufs = [torch.full((w.nbytes + 16,), 0xA5, dtype=torch.uint8, device="cuda") for w in want]
+    at = [b.data_ptr() + offset for b in bufs]
+    attrs = (ctypes.c_void_p * 1)(at[3])
+    out = _native.SrcuStreamVoxelOut(*at[:3], ctypes.cast(attrs, ctypes.c_void_p), at[4], at[5], 1)
+    cuda_ctx._check(cuda_ctx._lib.srcu_stream_voxel_fetch(sv._h, 0, len(x), ctypes.byref(out)))
+    sv.close()
+    for b, w in zip(bufs, want):
+        w = np.ascontiguousarray(w).reshape(-1).view(np.uint8)
+        got = b.cpu().numpy()
+        assert np.array_equal(got[offset:offset + len(w)], w)
+        assert np.all(got[:offset] == 0xA5) and np.all(got[offset + len(w):] == 0xA5)

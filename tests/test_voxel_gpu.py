@@ -339,3 +339,38 @@ def test_voxel_centroid_enqueue_matches_sync(cuda_ctx):
     assert np.array_equal(got["counts"], sync_counts)
     for a, b in zip(got["columns"], sync_cols):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("offset", [0, 1, 2, 4])
+@pytest.mark.parametrize("n", [1, 1025, 40_000])
+def test_device_results_at_any_alignment(cuda_ctx, n, offset):
+    """Result columns in device memory that start off a word or a 16-byte boundary hold
+    the bytes that host columns hold, with nothing written past them."""
+    import ctypes
+    import torch
+    c = synthetic.georef_scan(n, seed=21)
+    ref = cuda_ctx.voxel_normals(c.x, c.y, c.z, [c.intensity], leaf=0.3, radius=0.6,
+                                 want_keys=True)
+    v = len(ref["counts"])
+    room = 24 * n + 16
+    bufs = [torch.full((room,), 0xA5, dtype=torch.uint8, device="cuda") for _ in range(11)]
+    at = [b.data_ptr() + offset for b in bufs]
+    attrs = (ctypes.c_void_p * 1)(at[3])
+    vout = _native.SrcuVoxelOut(*at[:3], ctypes.cast(attrs, ctypes.c_void_p), at[4], at[5], 1)
+    nout = _native.SrcuNormalOut(*at[6:11], 1)
+    keep = _native._Keep()
+    cloud = _native.make_cloud(c.x, c.y, c.z, [c.intensity], keep)
+    vp = _native._voxel_params(0.3, None, False, False, False)
+    np_ = _native._normal_params(0.6, 3, None, False)
+    rows, stats = ctypes.c_uint64(0), _native.SrcuNormalStats()
+    cuda_ctx._check(cuda_ctx._lib.srcu_voxel_normals(
+        cuda_ctx.handle, ctypes.byref(cloud), ctypes.byref(vp), ctypes.byref(np_),
+        ctypes.byref(vout), ctypes.byref(nout), ctypes.byref(rows), ctypes.byref(stats)))
+    assert rows.value == v
+    want = ref["columns"] + [ref["keys"], ref["counts"], ref["nx"], ref["ny"], ref["nz"],
+                             ref["curvature"], ref["neighbor_counts"]]
+    for b, w in zip(bufs, want):
+        w = np.ascontiguousarray(w).reshape(-1).view(np.uint8)
+        got = b.cpu().numpy()
+        assert np.array_equal(got[offset:offset + len(w)], w)
+        assert np.all(got[:offset] == 0xA5) and np.all(got[offset + len(w):] == 0xA5)

@@ -84,27 +84,28 @@ srcu_status srcu_las_decode(srcu_ctx *ctx, const void *records, uint64_t n, int3
   for (int c = 0; c < 3; ++c) o.rgb[c] = static_cast<uint16_t *>(dev[6 + c]);
   const uint64_t tiles = (n + d.per_tile - 1) / d.per_tile;
   const size_t smem = 2 * size_t(d.buf_bytes);  // two tile buffers
-  CU_TRY(cudaFuncSetAttribute(k_las_decode, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              int(2 * (LAS_BUF_MAX + 48))));
+  if (smem > (48u << 10))  // more than a launch has without asking
+    CU_TRY(cudaFuncSetAttribute(k_las_decode, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                int(2 * (LAS_BUF_MAX + 48))));
   int per_sm = 1;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_las_decode, LAS_THREADS, smem);
   const uint32_t grid = uint32_t(std::min<uint64_t>(
       tiles, uint64_t(ctx->num_sms) * uint64_t(std::max(per_sm, 1))));
-  uint32_t *status = &ctx->ctl->status;
-  CU_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t), ctx->stream));
+  // The status word is the context's pinned host copy, which nothing else writes between
+  // two waits: a word on the device costs a call a fill before the kernel and a copy after it.
+  volatile uint32_t *status = &ctx->ctl_host->status;
+  *status = 0;
   {
     Launch l(ctx, SRCU_K_LAS_DECODE);
-    k_las_decode<<<grid, LAS_THREADS, smem, ctx->stream>>>(src, d, o, status);
+    k_las_decode<<<grid, LAS_THREADS, smem, ctx->stream>>>(src, d, o, &ctx->ctl_host->status);
   }
   CU_TRY(cudaGetLastError());
-  CU_TRY(cudaMemcpyAsync(&ctx->ctl_host->status, status, sizeof(uint32_t), cudaMemcpyDeviceToHost,
-                         ctx->stream));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
-  if (ctx->ctl_host->status & ST_TIMEOUT)
+  if (*status & ST_TIMEOUT)
     return fail(ctx, SRCU_ERR_TIMEOUT, "a bounded wait for a LAS record copy gave up");
-  if (!out->on_device)
-    for (int c = 0; c < 9; ++c)
-      if (dst[c]) ST_TRY(copy_out(ctx, dst[c], dev[c], n * elem[c], 0));
+  if (out->on_device) return SRCU_OK;
+  for (int c = 0; c < 9; ++c)
+    if (dst[c]) ST_TRY(copy_out(ctx, dst[c], dev[c], n * elem[c], 0));
   CU_TRY(cudaStreamSynchronize(ctx->stream));
   return SRCU_OK;
 }

@@ -122,7 +122,7 @@ __device__ __forceinline__ LasTile las_tile(const uint8_t *records, const LasDec
 }
 
 __global__ void __launch_bounds__(LAS_THREADS) k_las_decode(const uint8_t *records, LasDecodeDev d,
-                                                           LasOutDev o, uint32_t *status) {
+                                                           LasOutDev o, volatile uint32_t *status) {
   extern __shared__ __align__(128) uint8_t las_smem[];
   __shared__ __align__(8) uint64_t bars[2];
   const uint64_t tiles = (d.n + d.per_tile - 1) / d.per_tile;
@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(LAS_THREADS) k_las_decode(const uint8_t *recor
     const bool ok = wait(k);
     // plain-loaded head/tail bytes of tile k are visible after this barrier
     if (__syncthreads_or(!ok)) {
-      if (t == 0) atomicOr(status, ST_TIMEOUT);
+      if (t == 0) *status = ST_TIMEOUT;
       if (k + 1 < mine) wait(k + 1);  // the copy in flight, again bounded
       return;
     }

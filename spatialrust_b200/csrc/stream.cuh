@@ -414,11 +414,12 @@ __device__ __forceinline__ void stream_fields(const StreamLayout &lay, uint32_t 
   }
 }
 
-// A compensated sum that starts from its first value as it is; `more` when others
-// follow (they start from 0.0 + v, which differs for v = -0).
+// The first value of a compensated sum that is still empty: a lone one is the sum as it
+// is; with `more` to follow it is added like the rest, so that an infinity leaves its
+// correction NaN and the sum of what follows NaN, as CompensatedSum's is.
 __device__ __forceinline__ void stream_first(Kahan &k, double v, bool more) {
-  k.s = more ? __dadd_rn(0.0, v) : v;
-  k.c = 0.0;
+  if (more) k.add(v);
+  else k.s = v;
 }
 
 // Reduces the voxel at sorted positions [i, j), one thread in sorted order, into

@@ -124,6 +124,29 @@ def test_non_finite_points_are_skipped_and_negative_keys(cuda_ctx):
     assert info["finite_points"] == finite and info["points"] == 50_000
 
 
+@pytest.mark.parametrize("f64", [False, True])
+@pytest.mark.parametrize("device_run", [0, 1, 2, 5])
+def test_non_finite_attributes(cuda_ctx, device_run, f64):
+    # a voxel per sequence, in one run and over merged runs: an infinity that others
+    # follow ends as NaN, as the compensated sum of the whole stream does, a last one as
+    # itself.  Sums of small integers: nothing rounds but the mean, one division.
+    inf, nan = np.inf, np.nan
+    sequences = [[inf, 1.0], [1.0, inf], [inf, 1.0, 2.0], [1.0, inf, 2.0], [1.0, 2.0, -inf], [-inf],
+                 [-inf, 3.0], [inf, -inf], [inf, inf], [nan, 1.0], [1.0, nan], [-0.0], [-0.0, -0.0],
+                 [-0.0, inf], [4.0, 5.0, 6.0], [inf] + [1.0] * 80]
+    x = np.concatenate([[F(v)] * len(s) for v, s in enumerate(sequences)]).astype(F)
+    values = np.concatenate(sequences).astype(np.float64 if f64 else F)
+    zero = np.zeros_like(x)
+    sv = _native.StreamVoxel(cuda_ctx, 1.0, [f64], device_run_points=device_run)
+    sv.push(x, zero, zero, [values])
+    assert sv.finish()["voxels"] == len(sequences)
+    attrs, counts = sv.fetch()[3], sv.fetch()[5]
+    sv.close()
+    ref = oracle.stream_voxel(x, zero, zero, [values.astype(np.float64)], leaf=1.0)
+    assert np.array_equal(counts, ref.counts)
+    assert np.array_equal(attrs, ref.attrs, equal_nan=True)
+
+
 def test_all_points_non_finite_or_empty(cuda_ctx):
     sv = _native.StreamVoxel(cuda_ctx, 1.0)
     sv.push(np.full(10, np.nan, F), np.zeros(10, F), np.zeros(10, F))

@@ -705,6 +705,23 @@ __device__ __forceinline__ uint32_t moments_fp64(const float4 *pts, const uint2 
   return hits;
 }
 
+// Whether some candidate lies on the query's shell, each looked at by itself: for the
+// radii whose square overflows, where the packed walk's least |d2 - r2| cannot tell
+// the query from the others.
+__device__ __noinline__ uint32_t shell_overflowed(const float4 *pts, const uint2 *rg, float4 qp,
+                                                  float r2, float shell_tol) {
+  for (int r = 0; r < 9; ++r) {
+    const uint2 range = rg[r];
+    for (uint32_t j = range.x; j < range.y; ++j) {
+      const float4 c = __ldg(pts + j);
+      const float dx = __fsub_rn(c.x, qp.x), dy = __fsub_rn(c.y, qp.y), dz = __fsub_rn(c.z, qp.z);
+      const float d2 = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+      if (d2 != 0.f && fabsf(__fsub_rn(d2, r2)) <= shell_tol) return 1;
+    }
+  }
+  return 0;
+}
+
 // Where the normals kernels write, by original point index.
 struct NormalDst {
   float *nx, *ny, *nz, *curv;
@@ -1135,8 +1152,9 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
 #pragma unroll
       for (int k = 0; k < 9; ++k) S[k] = sums[k * NM_THREADS];
       // on the shell: d2 != 0 and |d2 - r2| <= tol; d2 = 0 is within tol of r2 only
-      // at r2 = 0, where no other d2 is
-      if (CountShell && prm.count_shell && r2 > 0.f && shell_min <= shell_tol) shell = 1;
+      // at r2 = 0, where no other d2 is, and where r2 has overflowed
+      if (CountShell && prm.count_shell && r2 > 0.f)
+        shell = isinf(r2) ? shell_overflowed(pts, rg, qp, r2, shell_tol) : shell_min <= shell_tol;
     } else {
       uint2 next = rg[0];
 #pragma unroll 1

@@ -202,6 +202,34 @@ def test_duplicates_and_shell_points(cuda_ctx):
     assert stats["shell_points"] == int(ref.shell.sum())
 
 
+@pytest.mark.parametrize("walk", [0, 1, 2])
+@pytest.mark.parametrize("name", ["alone", "duplicates", "few", "many", "far"])
+def test_shell_points_of_a_radius_whose_square_overflows(cuda_ctx, name, walk):
+    # r^2 = inf: every other point at a finite, non-zero d^2 is on the shell, the query
+    # itself, its duplicates, NaN points and d^2 = inf are not.  One cell holds them all:
+    # from eight points on the deep walk, below the sparse one.
+    rng = np.random.default_rng(3)
+    clouds = dict(alone=np.zeros((1, 3)), duplicates=np.ones((20, 3)), few=rng.normal(size=(5, 3)),
+                  many=rng.normal(size=(40, 3)),
+                  far=np.repeat([[0.0, 0, 0], [3e19, 0, 0]], 6, axis=0))
+    p = clouds[name].astype(np.float32)
+    if name in ("few", "many"):
+        p[1] = np.nan
+    r = np.float32(2e19)
+    with np.errstate(over="ignore", invalid="ignore"):
+        r2 = r * r
+        d = p[None] - p[:, None]
+        d2 = (d[..., 0] * d[..., 0] + d[..., 1] * d[..., 1]) + d[..., 2] * d[..., 2]
+        shell = ((d2 != 0) & (np.abs(d2 - r2) <= np.float32(1e-6) * r2)).any(1)
+    staging = cuda_ctx.neighbor_staging()
+    cuda_ctx.set_neighbor_staging(walk)
+    try:
+        stats = cuda_ctx.radius_normals(p[:, 0], p[:, 1], p[:, 2], float(r))[5]
+    finally:
+        cuda_ctx.set_neighbor_staging(staging)
+    assert stats["shell_points"] == int(shell.sum())
+
+
 # ---- chained voxel -> normals (MvpPipeline) ----------------------------------
 
 def test_voxel_then_normals_chain(cuda_ctx):

@@ -996,18 +996,23 @@ bool takable(const srcu_ctx *ctx, const DevBuf &b, uint32_t words = 1) {
   return b.p && b.bytes >= size_t(ctx->last_points) * words * 4;
 }
 
-// Whether a kernel of this context can write 32-bit words to dst: this GPU's own or
-// managed memory, word-aligned.  Whatever else a caller passes as device memory is
-// left to a copy, which takes any alignment and refuses what it cannot reach.
-bool writable(const srcu_ctx *ctx, const void *dst) {
-  if (reinterpret_cast<uintptr_t>(dst) & 3u) return false;
+// Whether a kernel of this context may read and write at p: this GPU's own or managed
+// memory.  Whatever else a caller passes as device memory (another GPU's, the host's) is
+// left to a copy, which takes what it can reach and refuses the rest, where a kernel's
+// access would end the context.
+bool own_memory(const srcu_ctx *ctx, const void *p) {
   cudaPointerAttributes at;
-  if (cudaPointerGetAttributes(&at, dst) != cudaSuccess) {
+  if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
     cudaGetLastError();
     return false;
   }
   return at.type == cudaMemoryTypeManaged ||
          (at.type == cudaMemoryTypeDevice && at.device == ctx->device);
+}
+
+// Whether a kernel may write 32-bit words to dst; a copy takes any alignment.
+bool writable(const srcu_ctx *ctx, const void *dst) {
+  return (reinterpret_cast<uintptr_t>(dst) & 3u) == 0 && own_memory(ctx, dst);
 }
 
 void take_column(TakeColumns &t, void *dst, const void *src, uint32_t words) {

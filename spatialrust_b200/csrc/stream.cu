@@ -29,7 +29,7 @@ struct srcu_stream_voxel {
   StreamLayout lay{};
   int occ_point[2] = {1, 1}, occ_record[2] = {1, 1};  // by kStreamSort shape
   DevBuf run;                                  // run buffer: packed points
-  DevBuf stage[MAX_COLS];                      // columns of a host (or misaligned) chunk
+  DevBuf stage[MAX_COLS];                      // columns of a chunk not read in place
   DevBuf rk[3], rcnt, rsum[MAX_COLS];          // partial records
   DevBuf opos[3], oattr[MAX_COLS], okeys, ocnt; // finished outputs
   DevBuf tile_heads, tile_off, long_list, plan, state;
@@ -371,11 +371,13 @@ srcu_status srcu_stream_voxel_push(srcu_stream_voxel *sv, const srcu_cloud *chun
   CU_TRY(cudaSetDevice(ctx->device));
   const void *src[MAX_COLS] = {chunk->x, chunk->y, chunk->z};
   for (uint32_t a = 0; a < chunk->n_attrs; ++a) src[3 + a] = chunk->attrs[a];
-  // device columns are read where they are, unless one is not aligned to its elements
+  // device columns are read where they are, unless one is not aligned to its elements or
+  // not in memory that a kernel may read: a chunk with such a column is staged by copies
   const cudaMemcpyKind kind = chunk->on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
   bool in_place = chunk->on_device != 0;
   for (uint32_t c = 0; c < sv->nc; ++c)
-    in_place = in_place && reinterpret_cast<uintptr_t>(src[c]) % sv_elem(sv, c) == 0;
+    in_place = in_place && reinterpret_cast<uintptr_t>(src[c]) % sv_elem(sv, c) == 0 &&
+               (chunk->n == 0 || own_memory(ctx, src[c]));
   uint64_t done = 0;
   while (done < chunk->n) {
     uint64_t take = std::min<uint64_t>(chunk->n - done, sv->dev_run - sv->fill);

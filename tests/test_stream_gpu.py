@@ -253,3 +253,30 @@ def test_fetch_to_device_at_any_alignment(cuda_ctx, offset):
         got = b.cpu().numpy()
         assert np.array_equal(got[offset:offset + len(w)], w)
         assert np.all(got[:offset] == 0xA5) and np.all(got[offset + len(w):] == 0xA5)
+
+
+def test_chunks_outside_device_memory_are_staged(cuda_ctx):
+    # pinned host memory marked as device memory: no kernel reads the caller's columns,
+    # they are copied into staging columns, which the context's byte count shows
+    import ctypes
+    import torch
+    n = 5000
+    c = synthetic.shapes_scene(n, seed=4)
+    cols = [torch.from_numpy(np.ascontiguousarray(a, F)) for a in (c.x, c.y, c.z)]
+    got, staged = {}, {}
+    for name, held in (("device", [t.cuda() for t in cols]), ("pinned", [t.pin_memory() for t in cols])):
+        torch.cuda.synchronize()
+        ctx = _native.Context(0)
+        sv = _native.StreamVoxel(ctx, 0.05, device_run_points=n)
+        before = ctx.device_bytes()
+        chunk = _native.SrcuCloud(*[t.data_ptr() for t in held], None, 0, 1, n)
+        ctx._check(ctx._lib.srcu_stream_voxel_push(sv._h, ctypes.byref(chunk)))
+        # the chunk fills the run, whose reduction allocates the same for both
+        staged[name] = ctx.device_bytes() - before
+        sv.finish()
+        got[name] = sv.fetch()
+        sv.close()
+        ctx.close()
+    assert staged["pinned"] - staged["device"] >= 3 * 4 * n
+    for a, b in zip(got["device"], got["pinned"]):
+        assert np.array_equal(a, b)

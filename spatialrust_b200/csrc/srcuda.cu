@@ -1418,10 +1418,10 @@ srcu_status srcu_euclidean_cluster_roots(srcu_ctx *ctx, const srcu_cloud *cloud,
     k_cluster_init<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link);
     k_cluster_union<true><<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, cell, ranges, r2,
                                                                 link);
-    k_cluster_flatten<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, link);
+    k_cluster_flatten<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link, nullptr);
     k_cluster_union<false><<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, cell, ranges, r2,
                                                                  link);
-    k_cluster_roots<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link, dst);
+    k_cluster_flatten<<<grid, CL_THREADS, 0, ctx->stream>>>(ctx->ctl, pts, link, dst);
   }
   CU_TRY(cudaGetLastError());
   ST_TRY(read_control(ctx));

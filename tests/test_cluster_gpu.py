@@ -139,3 +139,45 @@ def test_chain_roots_in_any_index_order(cuda_ctx, n, order):
     zero = np.zeros(n + 2, F)
     got = cuda_ctx.euclidean_cluster_roots(x, zero, zero, 1.0)
     assert np.array_equal(got, np.append(expect, n + 1))
+
+
+@pytest.mark.parametrize("order", ["ascending", "descending", "even points first"])
+def test_one_component_along_three_million_points(cuda_ctx, order):
+    """Chains of links longer than any bounded walk: points half a tolerance apart along
+    a line, numbered along it, against it and in two runs over it (5.7 points per cell:
+    the grid's cells are as wide as the extent asks)."""
+    import torch
+    x = torch.arange(3_000_000, device="cuda", dtype=torch.float32) * 0.5
+    if order == "descending":
+        x = x.flip(0).contiguous()
+    if order == "even points first":
+        x = torch.cat([x[::2], x[1::2]])
+    zero = torch.zeros_like(x)
+    torch.cuda.synchronize()
+    roots = cuda_ctx.euclidean_cluster_roots(x, zero, zero, 1.0)
+    assert cuda_ctx.chain_info()["cells"] < 1_000_000
+    assert int(roots.abs().max()) == 0
+
+
+@pytest.mark.parametrize("extra", [-1, 0, 1])
+@pytest.mark.parametrize("pattern, groups", [((2, 1, 1, 1, 1), 1), ((2, 1, 1, 1, 1), 37),
+                                             ((2, 1, 1, 1, 1), 5000), ((2, 2, 2, 1), 226_000)])
+def test_roots_on_either_side_of_the_density_line(cuda_ctx, pattern, groups, extra):
+    """6 points in 5 cells (7 in 4 of a large cloud), and a point fewer or more: the two
+    forests.  The cells of a group touch, in rows of ten groups."""
+    rng = np.random.default_rng(groups * 3 + extra)
+    k, per = len(pattern), sum(pattern)
+    cell = np.repeat(np.arange(k * groups), np.tile(pattern, groups))
+    cell = cell[1:] if extra < 0 else np.append(cell, [0] * extra)
+    p = rng.uniform(0.3, 0.7, (len(cell), 3))
+    p[0] = 0.1  # the grid's origin, in cell 0: every other point is well inside its cell
+    group = cell // k
+    p[:, 0] += cell % k + 8 * (group % 10)
+    p[:, 1] += 3 * (group // 10 % 1000)
+    p[:, 2] += 3 * (group // 10_000)
+    p = rng.permutation(p * (1 + 1e-5)).astype(F)  # a cell is this much wider than the tolerance
+    got = cuda_ctx.euclidean_cluster_roots(p[:, 0], p[:, 1], p[:, 2], 1.0)
+    ref = oracle.euclidean_roots(p[:, 0], p[:, 1], p[:, 2], 1.0, sparse=True)
+    info = cuda_ctx.chain_info()
+    assert (info["points"], info["cells"]) == (per * groups + extra, k * groups)
+    assert np.array_equal(got, ref)

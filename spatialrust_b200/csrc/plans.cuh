@@ -175,6 +175,7 @@ constexpr int WK_NORMALS = 25;
 constexpr int WK_RANGES = 26;
 constexpr int WK_BOUNDS = 27;  // blocks of k_bounds that are done
 constexpr int WK_REFINE = 28;  // queries listed for k_normals_refine
+constexpr int WK_PLANS = 29;   // blocks of k_plans that are done
 constexpr int WK_ORDER = 32;  // first-seen order of the plain-xyz path
 
 __device__ __forceinline__ int64_t rs_sat_i64(float t) {
@@ -359,7 +360,7 @@ __device__ __noinline__ void cell_plan(Control *ctl, const Batch &bt, uint32_t b
 // Places every cloud's (cx, cy) columns in one dense table when all of them
 // fit its `capacity` slots: col_base per cloud by a block scan over clouds.
 // Otherwise the chain keeps the column hash.  One block of 256 threads, after
-// its own cell plans; scratch holds 256 words.
+// the cell plans, its own and other blocks'; scratch holds 256 words.
 __device__ __noinline__ void column_bases(Control *ctl, const Batch &bt, uint64_t capacity,
                                           unsigned long long *scratch) {
   unsigned long long running = 0;
@@ -375,7 +376,8 @@ __device__ __noinline__ void column_bases(Control *ctl, const Batch &bt, uint64_
   for (uint32_t b0 = 0; b0 < bt.clouds; b0 += 256) {
     const uint32_t b = b0 + threadIdx.x;
     unsigned long long cols = 0;
-    if (b < bt.clouds) cols = (unsigned long long)bt.cplans[b].dims[0] * bt.cplans[b].dims[1];
+    if (b < bt.clouds)
+      cols = (unsigned long long)__ldcg(&bt.cplans[b].dims[0]) * __ldcg(&bt.cplans[b].dims[1]);
     scratch[threadIdx.x] = cols;
     __syncthreads();
     for (uint32_t off = 1; off < 256; off <<= 1) {  // inclusive Hillis-Steele scan
@@ -394,7 +396,13 @@ __device__ __noinline__ void column_bases(Control *ctl, const Batch &bt, uint64_
   }
 }
 
-// What the last block of k_bounds derives from the bounds.
+// Clouds whose plans the last block of k_bounds makes: two rounds of its threads.  A
+// round takes 3 us, so more clouds get a launch of their own (k_plans): a chain of 1000
+// clouds of 1000 points 502 -> 485 us, 5000 of 200 779 -> 710, 60000 of 40 2999 -> 2144;
+// with 257 to 512 clouds it is even.
+constexpr uint32_t PLAN_TAIL_CLOUDS = 256;
+
+// The plans a chain derives from the bounds.
 struct PlanTasks {
   uint32_t voxel;         // the voxel-key plans
   uint32_t cell;          // the cell plans and the column bases

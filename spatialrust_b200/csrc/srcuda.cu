@@ -733,10 +733,17 @@ srcu_status enqueue_bounds(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_
   tasks.voxel = voxel;
   tasks.cell = cell;
   tasks.col_capacity = uint64_t(1) << ctx->table_log2;
-  Launch l(ctx, SRCU_K_BOUNDS);
-  k_bounds<<<grid, BND_THREADS, 0, ctx->stream>>>(in[0], in[1], in[2], ctx->ctl, nullptr,
-                                                  nc > 3 ? in[3] : nullptr,
-                                                  ptr<float4>(ctx->in_aos), bt, tasks);
+  {
+    Launch l(ctx, SRCU_K_BOUNDS);
+    k_bounds<<<grid, BND_THREADS, 0, ctx->stream>>>(in[0], in[1], in[2], ctx->ctl, nullptr,
+                                                    nc > 3 ? in[3] : nullptr,
+                                                    ptr<float4>(ctx->in_aos), bt, tasks);
+  }
+  if (bt.clouds > PLAN_TAIL_CLOUDS) {
+    Launch l(ctx, SRCU_K_VOXEL_PLAN);
+    k_plans<<<ceil_div(bt.clouds, PLAN_CLOUDS), 2 * PLAN_CLOUDS, 0, ctx->stream>>>(ctx->ctl, bt,
+                                                                                  tasks);
+  }
   CU_TRY(cudaGetLastError());
   return SRCU_OK;
 }

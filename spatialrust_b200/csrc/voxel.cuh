@@ -240,7 +240,7 @@ __device__ __forceinline__ void bounds_many_clouds(const float *x, const float *
 // The block that finishes last derives the chain's plans from the bounds: they
 // move no data, so as launches of their own (voxel plans, cell plans, column
 // bases) they cost a launch latency each, 10 us of a chain, against 4 us in this
-// kernel's tail.  Six blocks per SM: the plans' registers would leave five, which
+// kernel's tail.  With more than PLAN_TAIL_CLOUDS clouds k_plans makes them.  Six blocks per SM: the plans' registers would leave five, which
 // cost the loop 8 us at 2M points.
 __global__ void __launch_bounds__(BND_THREADS, 6) k_bounds(const float *x, const float *y,
                                                         const float *z, Control *ctl,
@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(BND_THREADS, 6) k_bounds(const float *x, const
   const uint64_t n = count_dev ? *count_dev : ctl->n_points;
   if (bt.clouds == 1) bounds_one_cloud(x, y, z, n, a0, aos, bt.bounds);
   else bounds_many_clouds(x, y, z, n, a0, aos, bt);
+  if (bt.clouds > PLAN_TAIL_CLOUDS) return;
 
   __shared__ uint32_t last;
   __shared__ unsigned long long scratch[256];
@@ -269,6 +270,30 @@ __global__ void __launch_bounds__(BND_THREADS, 6) k_bounds(const float *x, const
     for (uint32_t b = t - HALF; b < bt.clouds; b += HALF) cell_plan(ctl, bt, b);
   __syncthreads();
   if (tasks.cell) column_bases(ctl, bt, tasks.col_capacity, scratch);
+}
+
+// The plans of many clouds: PLAN_CLOUDS of each kind a block, and the column bases by
+// the block that finishes last.
+constexpr uint32_t PLAN_CLOUDS = 128;
+__global__ void __launch_bounds__(2 * PLAN_CLOUDS) k_plans(Control *ctl, Batch bt, PlanTasks tasks) {
+  if (ld_relaxed_u32(&ctl->status)) return;
+  const uint32_t t = threadIdx.x;
+  const uint32_t b = blockIdx.x * PLAN_CLOUDS + t % PLAN_CLOUDS;
+  if (b < bt.clouds) {
+    if (tasks.voxel && t < PLAN_CLOUDS) voxel_plan(ctl, bt, b);
+    if (tasks.cell && t >= PLAN_CLOUDS) cell_plan(ctl, bt, b);
+  }
+  if (!tasks.cell) return;
+  __shared__ uint32_t last;
+  __shared__ unsigned long long scratch[256];
+  __threadfence();  // this thread's plan, before the block counts as done
+  __syncthreads();
+  if (t == 0) last = atomicAdd(&ctl->work[WK_PLANS], 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  static_assert(2 * PLAN_CLOUDS == 256, "column_bases takes 256 threads");
+  column_bases(ctl, bt, tasks.col_capacity, scratch);
 }
 
 // Key source for the voxel sort: the reference's voxel key of point i,

@@ -87,6 +87,35 @@ def test_batch_with_empty_clouds(cuda_ctx):
     assert int(out["counts"][voff[4]:].sum()) == b.n
 
 
+@pytest.mark.parametrize("count", [255, 256, 257, 384, 385, 3000])
+def test_batch_of_many_small_clouds(cuda_ctx, count):
+    """Either side of the count from which the plans get a launch of their own, and of
+    its blocks' 128 clouds: every cloud as it is alone, its plan from its own leaf,
+    radius and bounds."""
+    import torch
+    rng = np.random.default_rng(count)
+    clouds = [synthetic.uniform_cube(int(n), seed=b, extent=float(e))
+              for b, (n, e) in enumerate(zip(rng.integers(0, 40, count), rng.uniform(1, 30, count)))]
+    leaves = rng.choice([0.5, 1.0, 2.0], count).tolist()
+    radii = [3.0 * leaf for leaf in leaves]
+    cuda_ctx.profile_read(reset=True)
+    voff, out = run_batch(cuda_ctx, torch, clouds, leaves, radii)
+    assert cuda_ctx.profile_read(reset=True)["voxel_plan"]["launches"] == (count > 256)
+    assert len(voff) == count + 1
+    for b in {0, 1, 127, 128, 254, count // 2, count - 2, count - 1}:
+        c, mine = clouds[b], slice_out(out, int(voff[b]), int(voff[b + 1]))
+        if c.n == 0:
+            assert len(mine["counts"]) == 0
+            continue
+        vox = oracle.voxel_centroid(c.x, c.y, c.z, [c.intensity], leaf=leaves[b])
+        assert np.array_equal(mine["counts"], vox.counts)
+        for g, r in zip(mine["columns"], vox.fields):
+            assert np.array_equal(g, r)
+        ref = oracle.radius_normals_fp64(vox.x, vox.y, vox.z, radii[b], 3)
+        assert np.array_equal(mine["neighbor_counts"], ref.counts)
+    assert int(out["counts"].sum()) == sum(c.n for c in clouds)
+
+
 def test_batch_rejects_bad_offsets(cuda_ctx):
     import torch
     c = synthetic.uniform_cube(1000, seed=3)

@@ -19,7 +19,9 @@ struct srcu_stream_voxel {
   uint32_t nc = 3;
   double leaf = 0.0;
   uint64_t dev_run = 0;   // points per device run
-  uint64_t fill = 0;      // points in the run buffer
+  uint64_t fill = 0;      // points of the run so far, the last `staged` of them unpacked
+  uint64_t staged = 0;    // points in the staging columns
+  uint64_t stage_cap = 0; // points they hold
   uint64_t points = 0;    // points pushed
   uint64_t device_runs = 0;
   uint64_t records = 0;   // partial records stored
@@ -38,7 +40,11 @@ struct srcu_stream_voxel {
 
 namespace {
 
-constexpr uint64_t kStreamStage = uint64_t(1) << 20;  // points of a chunk staged at a time
+// Points of a chunk staged at a time, and points that small chunks gather to before they
+// are packed.  A kernel for every push makes it longer (1000 host points with nine f64
+// attributes 50 us, 46 gathered; 16384 with two 60, 50 gathered).
+constexpr uint64_t kStreamStage = uint64_t(1) << 20;
+constexpr uint64_t kStreamGather = uint64_t(1) << 16;
 
 uint32_t sv_elem(const srcu_stream_voxel *sv, uint32_t c) {
   return (c >= 3 && ((sv->prm.attr_f64_mask >> (c - 3)) & 1u)) ? 8u : 4u;
@@ -176,12 +182,54 @@ srcu_status sv_sync(srcu_stream_voxel *sv) {
   return s;
 }
 
+// Columns of n points -> records of the run from point `at` on.
+srcu_status sv_pack(srcu_stream_voxel *sv, const StreamChunk &ch, uint64_t at, uint64_t n) {
+  srcu_ctx *ctx = sv->ctx;
+  const uint32_t grid = std::min<uint32_t>(ceil_div(n, 256), uint32_t(ctx->num_sms) * 8);
+  k_stream_pack<<<grid, 256, 0, ctx->stream>>>(ch, sv->lay, n,
+                                               ptr<uint4>(sv->run) + at * sv->lay.units);
+  CU_TRY(cudaGetLastError());
+  return SRCU_OK;
+}
+
+srcu_status sv_pack_staged(srcu_stream_voxel *sv) {
+  const uint64_t n = sv->staged;
+  if (n == 0) return SRCU_OK;
+  StreamChunk ch{};
+  for (uint32_t c = 0; c < sv->nc; ++c) ch.col[c] = sv->stage[c].p;
+  sv->staged = 0;
+  return sv_pack(sv, ch, sv->fill - n, n);
+}
+
+// Copies n points of a chunk (its columns from point `first` on) behind the staged ones.
+srcu_status sv_stage(srcu_stream_voxel *sv, const void *const *src, uint64_t first, uint64_t n,
+                     cudaMemcpyKind kind) {
+  srcu_ctx *ctx = sv->ctx;
+  if (sv->staged + n > sv->stage_cap) {
+    ST_TRY(sv_pack_staged(sv));
+    if (n > sv->stage_cap) {
+      const uint64_t cap = std::max(n, std::min(kStreamGather, sv->dev_run));
+      sv->stage_cap = 0;
+      for (uint32_t c = 0; c < sv->nc; ++c) ST_TRY(ensure(ctx, sv->stage[c], cap * sv_elem(sv, c)));
+      sv->stage_cap = cap;
+    }
+  }
+  for (uint32_t c = 0; c < sv->nc; ++c) {
+    const uint32_t e = sv_elem(sv, c);
+    CU_TRY(cudaMemcpyAsync(ptr<char>(sv->stage[c]) + sv->staged * e,
+                           static_cast<const char *>(src[c]) + first * e, n * e, kind, ctx->stream));
+  }
+  sv->staged += n;
+  return SRCU_OK;
+}
+
 // Sorts and reduces the run buffer into partial records, or, as the stream's only
 // run, into the outputs.
 template <bool Final>
 srcu_status sv_flush(srcu_stream_voxel *sv) {
   const uint64_t n = sv->fill;
   if (n == 0) return SRCU_OK;
+  ST_TRY(sv_pack_staged(sv));
   srcu_ctx *ctx = sv->ctx;
   StreamOut out{};
   if (Final) {
@@ -318,7 +366,8 @@ srcu_status srcu_stream_voxel_create(srcu_ctx *ctx, const srcu_stream_voxel_para
   sv->nc = 3 + params->n_attrs;
   sv->leaf = double(params->leaf_size);
   sv->fill = sv->points = sv->device_runs = sv->records = sv->voxels = 0;
-  sv->rec_cap = 0;  // re-derived from the kept buffers' sizes as records arrive
+  // re-derived from the kept buffers' sizes as points and records arrive
+  sv->staged = sv->stage_cap = sv->rec_cap = 0;
   sv->finished = false;
   // By default a device run holds at least 2^22 points whatever run_points
   // is: the run size only partitions the sums, the voxels do not depend on it,
@@ -382,21 +431,14 @@ srcu_status srcu_stream_voxel_push(srcu_stream_voxel *sv, const srcu_cloud *chun
   while (done < chunk->n) {
     uint64_t take = std::min<uint64_t>(chunk->n - done, sv->dev_run - sv->fill);
     if (!in_place) take = std::min(take, kStreamStage);
-    StreamChunk ch{};
-    for (uint32_t c = 0; c < sv->nc; ++c) {
-      const uint32_t e = sv_elem(sv, c);
-      const char *from = static_cast<const char *>(src[c]) + done * e;
-      ch.col[c] = from;
-      if (in_place) continue;
-      ST_TRY(ensure(ctx, sv->stage[c], take * e));
-      if (take) CU_TRY(cudaMemcpyAsync(sv->stage[c].p, from, take * e, kind, ctx->stream));
-      ch.col[c] = sv->stage[c].p;
-    }
-    if (take) {
-      const uint32_t grid = std::min<uint32_t>(ceil_div(take, 256), uint32_t(ctx->num_sms) * 8);
-      k_stream_pack<<<grid, 256, 0, ctx->stream>>>(ch, sv->lay, take,
-                                                   ptr<uint4>(sv->run) + sv->fill * sv->lay.units);
-      CU_TRY(cudaGetLastError());
+    if (take && in_place) {
+      ST_TRY(sv_pack_staged(sv));
+      StreamChunk ch{};
+      for (uint32_t c = 0; c < sv->nc; ++c)
+        ch.col[c] = static_cast<const char *>(src[c]) + done * sv_elem(sv, c);
+      ST_TRY(sv_pack(sv, ch, sv->fill, take));
+    } else if (take) {
+      ST_TRY(sv_stage(sv, src, done, take, kind));
     }
     sv->fill += take;
     done += take;

@@ -280,3 +280,35 @@ def test_chunks_outside_device_memory_are_staged(cuda_ctx):
     assert staged["pinned"] - staged["device"] >= 3 * 4 * n
     for a, b in zip(got["device"], got["pinned"]):
         assert np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("device_run", [0, 1, 64, 1000, 65_537])
+def test_host_and_device_chunks_in_turn(cuda_ctx, device_run):
+    """Chunks gathered in the staging columns, chunks read in place between them, and
+    the ends of runs and of the staging columns: as if pushed at once, and twice over
+    with the buffers of the first stream, whose columns had other types."""
+    import torch
+    rng = np.random.default_rng(device_run)
+    sizes = [1, 3, 0, 63, 64, 65, 2, 700, 1, 300] if device_run in (1, 64) else \
+        [1, 3, 0, 65_536, 1, 65_535, 2, 70_000, 700, 1]
+    n = sum(sizes)
+    p = rng.uniform(0, 12, (n, 3)).astype(F)
+    extra = [rng.random(n), rng.random(n)]
+    for f64 in ([True, False], [False, True]):
+        attrs = [a.astype(np.float64 if f else F) for a, f in zip(extra, f64)]
+        cols = [np.ascontiguousarray(p[:, k]) for k in range(3)] + attrs
+        sv = _native.StreamVoxel(cuda_ctx, 1.0, f64, device_run_points=device_run)
+        lo = 0
+        for i, m in enumerate(sizes):
+            part = [c[lo:lo + m] for c in cols]
+            if i % 3 == 2:
+                part = [torch.from_numpy(np.ascontiguousarray(c)).cuda() for c in part]
+                torch.cuda.synchronize()
+            sv.push(*part[:3], part[3:])
+            lo += m
+        assert sv.finish()["points"] == n
+        got = sv.fetch()
+        sv.close()
+        ref = oracle.stream_voxel(*cols[:3], [a.astype(np.float64) for a in attrs], leaf=1.0)
+        assert np.array_equal(got[4], ref.keys) and np.array_equal(got[5], ref.counts)
+        assert np.allclose(got[3], ref.attrs, rtol=1e-12, atol=0)

@@ -600,16 +600,18 @@ srcu_status srcu_server_stats_reset(srcu_server *server);
 
 /* ---- launch accounting and kernel timing ---------------------------------- */
 
-/* Kernel groups of the chain, in launch order. */
+/* Kernel groups of the chain, in launch order.  Kernels that only copy are not counted:
+ * interleaved records to columns, a stream's chunks to its records, results to a
+ * caller's device columns. */
 typedef enum srcu_kernel_id {
   SRCU_K_BEGIN = 0,      /* control-block reset */
-  SRCU_K_BOUNDS,         /* per-axis min/max */
-  SRCU_K_VOXEL_PLAN,     /* voxel-key packing plan */
+  SRCU_K_BOUNDS,         /* per-axis min/max, and the plans that follow from them */
+  SRCU_K_VOXEL_PLAN,     /* plans in a launch of their own: streams, batches above 256 clouds */
   SRCU_K_VOXEL_HIST,     /* reserved: the histograms run inside SRCU_K_VOXEL_SORT */
   SRCU_K_VOXEL_SORT,     /* persistent onesweep sort of the voxel keys (histograms + passes) */
   SRCU_K_VOXEL_SEGMENTS, /* fused voxel segmentation + FP64 centroid reduction */
   SRCU_K_UNPACK_KEYS,    /* packed key -> (ix, iy, iz) */
-  SRCU_K_CELL_PLAN,      /* radius-grid plan */
+  SRCU_K_CELL_PLAN,      /* reserved: the radius-grid plans are made with the voxel plans */
   SRCU_K_CELL_HIST,      /* reserved: the histograms run inside SRCU_K_CELL_SORT */
   SRCU_K_CELL_SORT,      /* persistent onesweep sort of the cell keys (histograms + passes) */
   SRCU_K_CELLS,          /* cell table + cell-sorted point records */

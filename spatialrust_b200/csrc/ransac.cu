@@ -112,7 +112,7 @@ srcu_status ransac_score(srcu_ctx *ctx, uint64_t n, const float **cols, const ui
                          ctx->stream));
   uint32_t *status = &ctx->ctl->status;
   CU_TRY(cudaMemsetAsync(status, 0, sizeof(uint32_t), ctx->stream));
-  Launch l(ctx, SRCU_K_RANSAC);
+  Launch l(ctx, SRCU_K_RANSAC, 2);
   k_ransac_planes<<<ceil_div(count, 256), 256, 0, ctx->stream>>>(
       cols[0], cols[1], cols[2], n, ptr<const uint32_t>(ctx->rs_hyp), count,
       ptr<float4>(ctx->rs_planes), ptr<uint32_t>(ctx->rs_valid), ptr<uint32_t>(ctx->rs_counts),
@@ -234,7 +234,7 @@ srcu_status srcu_ransac_plane_segment(srcu_ctx *ctx, const srcu_cloud *cloud,
   if (count) {
     ST_TRY(ransac_score(ctx, n, cols, hyp.data(), count, params->distance_threshold));
     {
-      Launch l(ctx, SRCU_K_RANSAC);
+      Launch l(ctx, SRCU_K_RANSAC, 4);
       k_ransac_best<<<1, 1024, 0, ctx->stream>>>(ptr<const float4>(ctx->rs_planes),
                                                  ptr<const uint32_t>(ctx->rs_valid),
                                                  ptr<const uint32_t>(ctx->rs_counts), count,

@@ -710,7 +710,7 @@ srcu_status enqueue_first_seen(srcu_ctx *ctx, const XyzTmp &tmp, uint64_t n) {
   const uint32_t grid = std::max<uint32_t>(1, std::min<uint32_t>(ceil_div(n, 256), ctx->num_sms * 8));
   const uint32_t tiles = std::max<uint32_t>(1, ceil_div(n, SEG_TILE));
   CU_TRY(cudaMemsetAsync(tmp.mark, 0, n * 4, ctx->stream));
-  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
+  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS, 2);
   k_voxel_xyz_f32<<<grid, 256, 0, ctx->stream>>>(
       ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort, ptr<const float4>(ctx->in_aos),
       ptr<uint64_t>(ctx->vkeys), ptr<uint32_t>(ctx->vcounts), tmp.starts, tmp.x, tmp.y, tmp.z,
@@ -767,7 +767,7 @@ srcu_status enqueue_voxel(srcu_ctx *ctx, const float **in, uint32_t nc, uint64_t
   const bool first_seen = ctx->xyz_order && bt.clouds == 1;
   XyzTmp tmp{};
   if (first_seen) ST_TRY(xyz_tmp(ctx, n, tmp));
-  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
+  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS, bt.clouds > 1 ? 2 : 1);
   switch (nc) {
     case 3: launch_segments_nc<3>(ctx, in, grid, bt, tmp.starts); break;
     case 4: launch_segments_nc<4>(ctx, in, grid, bt, tmp.starts); break;
@@ -836,12 +836,15 @@ srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const fl
 }
 
 // The normals kernels over the grid, in the context's neighbour walk.  raw: the
-// points are a caller's cloud, whose cells may be dense or not; voxel centroids
-// never fill a cell as the deep walk wants, so their chains do without it.
+// points are a caller's cloud, whose cells may be dense or not.  Chains do without the
+// deep walk and its launch: at a radius of three leaves a cell holds at most nine
+// centroids of a flat surface, 4.4 on the scans.  (At five to ten leaves a dense surface
+// fills 25 to 100 a cell, where the deep walk takes about 0.88 of the sparse one's time.)
 template <bool Shell, bool PlaneCov>
 srcu_status launch_normals(srcu_ctx *ctx, const unsigned long long *count_dev, const Batch &bt,
                            NormalDst dst, bool raw) {
-  Launch l(ctx, SRCU_K_NORMALS, 2);
+  const bool by_density = raw && ctx->neighbor_staging == WALK_PACKED;
+  Launch l(ctx, SRCU_K_NORMALS, by_density ? 3 : 2);
   const uint32_t sms = uint32_t(ctx->num_sms);
   const float4 *pts = ptr<float4>(ctx->pts);
   const uint32_t *pt_cell = ptr<uint32_t>(ctx->pt_cell);
@@ -853,7 +856,7 @@ srcu_status launch_normals(srcu_ctx *ctx, const unsigned long long *count_dev, c
   if (ctx->neighbor_staging == WALK_PACKED) {
     kernel = k_normals<Shell, PlaneCov, WALK_PACKED>;
     occ = ctx->occ_normals_packed;
-    if (raw) {
+    if (by_density) {
       grid = GRID_SPARSE;
       k_normals<Shell, PlaneCov, WALK_DEEP><<<sms * uint32_t(ctx->occ_normals_deep), NM_THREADS, 0,
                                               ctx->stream>>>(ctx->ctl, pts, pt_cell, ranges,
@@ -1416,7 +1419,7 @@ srcu_status srcu_euclidean_cluster_roots(srcu_ctx *ctx, const srcu_cloud *cloud,
                                                                   uint32_t(ctx->num_sms) * 8));
   uint32_t *dst = cloud->on_device ? roots : ptr<uint32_t>(ctx->nout[0]);
   {
-    Launch l(ctx, SRCU_K_CLUSTER);
+    Launch l(ctx, SRCU_K_CLUSTER, 5);
     // the grid has consumed the cell sort: its key buffer holds the forest
     uint64_t *link = ptr<uint64_t>(ctx->keys[0]);
     const float4 *pts = ptr<const float4>(ctx->pts);

@@ -150,7 +150,7 @@ srcu_status sv_reduce(srcu_stream_voxel *sv, uint64_t n, const StreamIn &in, con
       1, std::min<uint32_t>(uint32_t(tiles), uint32_t(ctx->num_sms) * 8));
   StreamState *st = ptr<StreamState>(sv->state);
   const StreamPlan *pl = ptr<const StreamPlan>(sv->plan);
-  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS);
+  Launch l(ctx, SRCU_K_VOXEL_SEGMENTS, 4);
   k_stream_flags<<<grid, SV_THREADS, 0, ctx->stream>>>(ctx->ctl, sort_buffers(ctx), &ctx->ctl->vsort,
                                                        pl, ptr<uint32_t>(sv->tile_heads), st,
                                                        count_finite);

@@ -352,3 +352,29 @@ def test_refined_queries_alone_and_in_long_lists(cuda_ctx, copies):
                                        viewpoint=(0.0, 50.0, 100.0))
         for k, v in first.items():
             assert np.array_equal(alone[k], v, equal_nan=True), k
+
+
+def test_launch_counts(cuda_ctx):
+    # kernels per group, as srcu_profile_read reports them
+    c = synthetic.shapes_scene(5000, seed=2)
+
+    def launches(group, call):
+        cuda_ctx.profile_read(reset=True)
+        call()
+        return cuda_ctx.profile_read(reset=True)[group]["launches"]
+
+    raw = lambda: cuda_ctx.radius_normals(c.x, c.y, c.z, 0.3)
+    staging = cuda_ctx.neighbor_staging()
+    try:
+        for walk, kernels in ((0, 2), (1, 2), (2, 3)):  # the packed walk: sparse, dense, refined
+            cuda_ctx.set_neighbor_staging(walk)
+            assert launches("normals", raw) == kernels
+    finally:
+        cuda_ctx.set_neighbor_staging(staging)
+    assert launches("cell_plan", raw) == launches("voxel_plan", raw) == 0
+    chain = lambda **kw: cuda_ctx.voxel_normals(c.x, c.y, c.z, leaf=0.1, radius=0.3, **kw)
+    assert launches("normals", chain) == 2
+    assert launches("voxel_segments", chain) == 1
+    assert launches("voxel_segments", lambda: chain(plain_xyz=True)) == 3
+    assert launches("cluster", lambda: cuda_ctx.euclidean_cluster_roots(c.x, c.y, c.z, 0.1)) == 5
+    assert launches("ransac", lambda: cuda_ctx.ransac_plane_segment(c.x, c.y, c.z, 0.05, 50)) == 6

@@ -137,3 +137,25 @@ def test_too_few_inliers_leave_a_device_mask_alone(cuda_ctx):
                                                  mask.data_ptr())
     assert st == _native.SRCU_ERR_INVALID_ARGUMENT
     assert bool((mask == 7).all())
+
+
+@pytest.mark.parametrize("n, count", [(3, 67), (1024, 67), (1025, 67), (4097, 1), (4097, 32),
+                                      (4097, 33), (4097, 511), (4097, 513), (4097, 1025),
+                                      (303_103, 40), (303_104, 40), (303_105, 40)])
+def test_every_score_at_tile_and_chunk_edges(cuda_ctx, n, count):
+    """The inlier count of every hypothesis: 0 for a degenerate one (an index twice, the
+    zero plane), else the CPU segmenter's f32 expression over all points."""
+    rng = np.random.default_rng([n, count])
+    p = rng.normal(0, 1, (3, n)).astype(F)
+    p[2, : n // 2] *= F(0.01)
+    hyp = rng.integers(0, n, (count, 3)).astype(np.uint32)
+    hyp[::5, 1] = hyp[::5, 0]
+    got = cuda_ctx.ransac_plane_scores(*p, hyp, 0.02)
+    assert len(got) == count
+    for (inliers, normal, d), triple in zip(got, hyp):
+        if len(set(triple.tolist())) < 3:
+            assert (inliers, normal, d) == (0, (0.0, 0.0, 0.0), 0.0)
+            continue
+        a, b, c = (F(v) for v in normal)
+        s = ((a * p[0] + b * p[1]) + c * p[2]) + F(d)
+        assert inliers == int((np.abs(s) <= F(0.02)).sum())

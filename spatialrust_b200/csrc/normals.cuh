@@ -1218,7 +1218,7 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
         ++tally.invalid;
       }
       tally.shell += shell;
-      if (o.counts) o.counts[qidx] = PlaneCov ? c.n_eff : (prm.include_self ? c.n_eff : c.cnt);
+      if (o.counts) o.counts[qidx] = c.n_eff;
       if (exact_moments || small_gap) {
         refine = i | (small_gap ? REFINE_SOLVE : 0u);
         if (small_gap) ++tally.fp64;

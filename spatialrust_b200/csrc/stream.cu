@@ -115,10 +115,10 @@ srcu_status sv_final_out(srcu_stream_voxel *sv, uint64_t r, StreamOut &o) {
   return SRCU_OK;
 }
 
-// The streams' sorts run in two of the sort's launch shapes, as the voxel sort's
-// table has them: 8 keys per thread x 3 blocks of 256 threads up to 441k keys, 8 x 2
-// x 512 with 9-bit digits above (16 x 2 x 256, used for all before: 4.2M points
-// 238 us, 205 us here).
+// The streams' sorts run in two of the sort's launch shapes whatever tuning a context
+// has: 8 keys per thread x 3 blocks of 256 threads up to 441k keys, 8 x 2 x 512 with
+// 9-bit digits above (16 x 2 x 256, used for all before: 4.2M points 238 us, 205 us
+// here).  The voxel sort's built-in table has another shape between 623k and 882k keys.
 constexpr int kStreamSort[2] = {1, 6};
 constexpr uint64_t kStreamSortSmall = 441000;
 

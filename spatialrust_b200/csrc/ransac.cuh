@@ -74,15 +74,19 @@ __device__ __forceinline__ bool plane_inlier(float4 pl, float px, float py, floa
   return fabsf(s) <= thr;
 }
 
-// Packed f32x2 arithmetic: two IEEE round-to-nearest operations, one per half.
+// Packed f32x2 arithmetic: two IEEE round-to-nearest operations, one per half.  A product
+// is written as a fused multiply-add of -0, which rounds it and keeps its sign: the
+// assembler fuses mul.rn.f32x2 with an add.rn.f32x2 that follows, explicit rounding or
+// not, and the sum is then not the reference's (over georeferenced coordinates counts
+// went wrong by hundreds).  The zero comes as a kernel argument, out of its sight.
 __device__ __forceinline__ uint64_t rs_pack(float lo, float hi) {
   uint64_t r;
   asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
   return r;
 }
-__device__ __forceinline__ uint64_t rs_mul(uint64_t a, uint64_t b) {
+__device__ __forceinline__ uint64_t rs_mul(uint64_t a, uint64_t b, uint64_t minus_zero) {
   uint64_t r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(minus_zero));
   return r;
 }
 __device__ __forceinline__ uint64_t rs_add(uint64_t a, uint64_t b) {
@@ -90,6 +94,7 @@ __device__ __forceinline__ uint64_t rs_add(uint64_t a, uint64_t b) {
   asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+constexpr uint64_t RS_MINUS_ZERO = 0x8000000080000000ull;  // (-0, -0)
 
 // counts[h] += inliers of plane h among this block's points, for the planes
 // [blockIdx.y * per_chunk, +per_chunk): the second grid dimension splits the
@@ -98,13 +103,14 @@ __device__ __forceinline__ uint64_t rs_add(uint64_t a, uint64_t b) {
 // plane_inlier's operations in its order, on two points at a time: six packed
 // instructions for what takes twelve apart, which leaves the comparison and the
 // count.  PAIRS pairs of points per thread share each plane's loads, its warp
-// reduction and its shared-memory atomic.  460k points x 1000 planes: 126 us,
+// reduction and its shared-memory atomic.  460k points x 1000 planes: 142 us,
 // 179 us with scalar arithmetic and eight points per thread.
 template <int PAIRS>
 __global__ void __launch_bounds__(RS_THREADS) k_ransac_score(const float *x, const float *y,
                                                              const float *z, uint64_t n,
                                                              const float4 *planes, uint32_t count,
                                                              uint32_t per_chunk, float thr,
+                                                             uint64_t minus_zero,
                                                              uint32_t *counts) {
   __shared__ ulonglong2 sp[RS_PLANES][2];  // (a, a) (b, b) / (c, c) (d, d)
   __shared__ uint32_t sc[RS_PLANES];
@@ -137,8 +143,10 @@ __global__ void __launch_bounds__(RS_THREADS) k_ransac_score(const float *x, con
       uint32_t c = 0;
 #pragma unroll
       for (int k = 0; k < PAIRS; ++k) {
-        const uint64_t s = rs_add(
-            rs_add(rs_add(rs_mul(ab.x, px[k]), rs_mul(ab.y, py[k])), rs_mul(cd.x, pz[k])), cd.y);
+        const uint64_t s =
+            rs_add(rs_add(rs_add(rs_mul(ab.x, px[k], minus_zero), rs_mul(ab.y, py[k], minus_zero)),
+                          rs_mul(cd.x, pz[k], minus_zero)),
+                   cd.y);
         float s0, s1;
         asm("mov.b64 {%0, %1}, %2;" : "=f"(s0), "=f"(s1) : "l"(s));
         c += fabsf(s0) <= thr ? 1u : 0u;

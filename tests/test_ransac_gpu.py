@@ -159,3 +159,22 @@ def test_every_score_at_tile_and_chunk_edges(cuda_ctx, n, count):
         a, b, c = (F(v) for v in normal)
         s = ((a * p[0] + b * p[1]) + c * p[2]) + F(d)
         assert inliers == int((np.abs(s) <= F(0.02)).sum())
+
+
+@pytest.mark.parametrize("n", [500, 40_000, 320_000])
+def test_scores_of_georeferenced_coordinates(cuda_ctx, n):
+    """Coordinates of hundreds of kilometres, where a plane's distance is a difference of
+    large f32 products: every rounding of the expression shows in the counts."""
+    rng = np.random.default_rng(n)
+    p = rng.normal(0, 3, (3, n))
+    p[2, : n // 2] *= 0.01
+    p = (p + np.array([[4.5e5], [3.9e6], [50.0]])).astype(F)
+    hyp = rng.integers(0, n, (70, 3)).astype(np.uint32)
+    for inliers, normal, d in cuda_ctx.ransac_plane_scores(*p, hyp, 0.05):
+        a, b, c = (F(v) for v in normal)
+        s = ((a * p[0] + b * p[1]) + c * p[2]) + F(d)
+        assert inliers == (int((np.abs(s) <= F(0.05)).sum()) if any(normal) else 0)
+    ref = oracle.ransac_plane(*p, 0.05, 200, 1, 7)
+    info, mask = cuda_ctx.ransac_plane_segment(*p, 0.05, 200, 1, 7)
+    assert info["best_hypothesis"] == ref["best_index"]
+    assert info["inlier_count"] == ref["inlier_count"] == mask.sum()

@@ -335,6 +335,10 @@ constexpr int SEG_ITEMS = 4;
 constexpr int SEG_TILE = SEG_THREADS * SEG_ITEMS;  // 1024 sorted positions per tile
 constexpr uint32_t SEG_SHORT = 32;  // longer voxels are reduced by a whole warp
 constexpr int SEG_GROUP = 4;  // columns gathered and summed together
+// A long voxel's columns go to warps LONG_FIRST columns, then LONG_NEXT at a time; a lane
+// has LONG_LOADS gathers in flight, or four items' keys.
+constexpr int LONG_FIRST = 4, LONG_NEXT = 2, LONG_LOADS = 16;
+constexpr int LONG_KEYS = 4;
 
 // Shared memory of k_voxel_segments<NC>: the tile's keys (plus one before and
 // one after), the scan scratch, and the tile's gathered point columns.
@@ -342,6 +346,7 @@ struct SegmentSmemHead {
   uint64_t keys[SEG_TILE + 2];  // keys[0] = key before the tile, keys[1 + tile_n] = key after it
   uint16_t start[SEG_TILE + 2];  // first position of each voxel that starts in the tile, then tile_n
   uint16_t longs[SEG_TILE / SEG_SHORT + 2];  // the tile's voxels that a warp reduces
+  uint32_t ends[SEG_TILE / SEG_SHORT + 2];   // where they end among the sorted items
   uint32_t scratch[SEG_THREADS / 32];
   double inv[SEG_SHORT + 1];  // 1.0 / count of the short voxels
   uint32_t tile;              // the tile at work, then the next one
@@ -484,25 +489,51 @@ __device__ __forceinline__ void short_voxel(const SegmentSmemHead &sm, const flo
     short_voxel<NC, C0 + SEG_GROUP>(sm, scol, base, j, e, seg, key, cols, agg, dst);
 }
 
-// The columns of one voxel from C0 on, its sorted items [p, e) reduced by a warp.
+// Some columns of one voxel from C0 on, its sorted items [p, e) reduced by a warp: lane l
+// sums items l, l + 32, ... in order.
 template <int NC, int C0>
 __device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uint32_t e, uint32_t seg,
-                                           uint64_t key, const Columns<NC> &cols, int32_t agg,
-                                           const VoxelDst &dst) {
-  constexpr int G = NC - C0 < SEG_GROUP ? NC - C0 : SEG_GROUP;
+                                           uint64_t key, const Columns<NC> &cols,
+                                           const float4 *aos_in, int32_t agg, const VoxelDst &dst) {
+  constexpr int W = C0 == 0 ? LONG_FIRST : LONG_NEXT;
+  constexpr int G = NC - C0 < W ? NC - C0 : W;
+  constexpr int AHEAD = LONG_LOADS / W;
   const uint32_t n = dst.n;
   const uint32_t lane = threadIdx.x & 31u;
   double s[G];
 #pragma unroll
   for (int g = 0; g < G; ++g) s[g] = 0.0;
-  for (uint32_t m = p + lane; m < e; m += 32) {
-    const uint32_t v = sv.val(m);
-    if (v >= n) {
-      atomicOr(dst.status, ST_INTERNAL);
-      continue;
+  for (uint32_t m = p + lane; m < e; m += 32 * AHEAD) {
+    uint32_t v[AHEAD];
+    float a[AHEAD][W];
+#pragma unroll
+    for (int q = 0; q < AHEAD; ++q) v[q] = m + 32 * q < e ? sv.val(m + 32 * q) : n;
+    bool gathered = false;
+    if constexpr (C0 == 0) {
+      if (aos_in) {  // one sector per point
+        gathered = true;
+#pragma unroll
+        for (int q = 0; q < AHEAD; ++q) {
+          const float4 pt = v[q] < n ? aos_in[v[q]] : make_float4(0.f, 0.f, 0.f, 0.f);
+          a[q][0] = pt.x, a[q][1] = pt.y, a[q][2] = pt.z, a[q][3] = pt.w;
+        }
+      }
+    }
+    if (!gathered) {
+#pragma unroll
+      for (int q = 0; q < AHEAD; ++q)
+#pragma unroll
+        for (int g = 0; g < G; ++g) a[q][g] = v[q] < n ? cols.in[C0 + g][v[q]] : 0.0f;
     }
 #pragma unroll
-    for (int g = 0; g < G; ++g) s[g] += double(cols.in[C0 + g][v]);
+    for (int q = 0; q < AHEAD; ++q) {
+      if (v[q] < n) {
+#pragma unroll
+        for (int g = 0; g < G; ++g) s[g] += double(a[q][g]);
+      } else if (m + 32 * q < e) {
+        atomicOr(dst.status, ST_INTERNAL);
+      }
+    }
   }
 #pragma unroll
   for (int g = 0; g < G; ++g)
@@ -516,8 +547,36 @@ __device__ __forceinline__ void long_voxel(const SortedView &sv, uint32_t p, uin
     };
     write_centroid<NC, C0, G>(cols, s, first, agg, 1.0 / double(e - p), p, e - p, seg, key, dst);
   }
-  if constexpr (C0 + SEG_GROUP < NC)
-    long_voxel<NC, C0 + SEG_GROUP>(sv, p, e, seg, key, cols, agg, dst);
+}
+
+// The task-th share of a long voxel's columns.
+template <int NC, int C0 = 0>
+__device__ __forceinline__ void long_share(uint32_t task, const SortedView &sv, uint32_t p,
+                                           uint32_t e, uint32_t seg, uint64_t key,
+                                           const Columns<NC> &cols, const float4 *aos_in,
+                                           int32_t agg, const VoxelDst &dst) {
+  constexpr int NEXT = C0 + (C0 == 0 ? LONG_FIRST : LONG_NEXT);
+  if (task == 0) long_voxel<NC, C0>(sv, p, e, seg, key, cols, aos_in, agg, dst);
+  else if constexpr (NEXT < NC)
+    long_share<NC, NEXT>(task - 1, sv, p, e, seg, key, cols, aos_in, agg, dst);
+}
+
+// Where the voxel of `key` ends, from sorted item e on, by a warp.
+__device__ __forceinline__ uint32_t voxel_end(const SortedView &sv, uint64_t key, uint32_t e,
+                                              uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (bool open = true; open && e < n;) {
+    uint64_t at[LONG_KEYS];
+#pragma unroll
+    for (int k = 0; k < LONG_KEYS; ++k) at[k] = e + 32 * k + lane < n ? sv.key(e + 32 * k + lane) : ~key;
+#pragma unroll
+    for (int k = 0; k < LONG_KEYS; ++k) {
+      const uint32_t stop = __ballot_sync(FULL_MASK, at[k] != key);
+      if (open) e += stop ? __ffs(stop) - 1 : 32;
+      open = open && !stop;
+    }
+  }
+  return e;
 }
 
 // Fused segment discovery + FP64 centroid reduction over the sorted
@@ -655,24 +714,25 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
                            voxel_agg(bt, key, vkey_bits, agg_all), dst);
     }
     __syncthreads();
-    // Long voxels: a warp finds the end and reduces from global memory.
-    for (uint32_t i = t >> 5; i < sm.num_longs; i += SEG_THREADS / 32) {
+    // Long voxels: a warp finds the end; then a warp for every share of its columns reduces
+    // them from global memory.  One warp for all columns, an item at a time, waited for
+    // its gathers: 2M points in 1600 voxels 373 us at three columns and 1934 at twelve,
+    // 140 and 540 so; in 100 voxels 2.3 and 12.8 ms, 0.8 and 2.1 so.
+    const uint32_t longs = sm.num_longs;
+    if (longs == 0) continue;
+    for (uint32_t i = t >> 5; i < longs; i += SEG_THREADS / 32) {
       const uint32_t q = sm.longs[i];
-      const uint32_t j = sm.start[q];
-      const uint64_t key = sm.keys[1 + j];
-      uint32_t e = base + sm.start[q + 1];
-      while (e < n) {
-        const uint32_t idx = e + lane;
-        const bool stop = idx >= n || sv.key(idx) != key;
-        const uint32_t b = __ballot_sync(FULL_MASK, stop);
-        if (b) {
-          e += __ffs(b) - 1;
-          break;
-        }
-        e += 32;
-      }
-      long_voxel<NC, 0>(sv, base + j, e, sm.seg_base + q, key, cols,
-                        voxel_agg(bt, key, vkey_bits, agg_all), dst);
+      const uint32_t e = voxel_end(sv, sm.keys[1 + sm.start[q]], base + sm.start[q + 1], n);
+      if (lane == 0) sm.ends[i] = e;
+    }
+    __syncthreads();
+    constexpr uint32_t SHARES =
+        NC <= LONG_FIRST ? 1 : 1 + (NC - LONG_FIRST + LONG_NEXT - 1) / LONG_NEXT;
+    for (uint32_t i = t >> 5; i < longs * SHARES; i += SEG_THREADS / 32) {
+      const uint32_t q = sm.longs[i / SHARES];
+      const uint64_t key = sm.keys[1 + sm.start[q]];
+      long_share<NC>(i % SHARES, sv, base + sm.start[q], sm.ends[i / SHARES], sm.seg_base + q, key,
+                     cols, aos_in, voxel_agg(bt, key, vkey_bits, agg_all), dst);
     }
   }
 }
@@ -711,41 +771,90 @@ inline cudaError_t configure_segment_kernels() {
 // gather, a copy back and a binary search per voxel in their place, a call from
 // host memory took 663 us; it takes 612.
 
-// One thread per voxel.  `starts` and tx may be the same memory: a thread reads its
-// start before it writes.  mark: a word per point, zeroed.
-__global__ void __launch_bounds__(256) k_voxel_xyz_f32(Control *ctl, SortBuffers sort,
-                                                       const SortState *sort_state,
-                                                       const float4 *aos, const uint64_t *vkeys,
-                                                       const uint32_t *vcounts,
-                                                       const uint32_t *starts, float *tx, float *ty,
-                                                       float *tz, uint32_t *tc, uint64_t *tk,
-                                                       uint32_t *mark) {
+constexpr uint32_t XYZ_THREADS = 256;
+constexpr uint32_t XYZ_SHORT = 128;  // points of a voxel that its thread sums alone
+
+// One thread per voxel; a voxel of more than XYZ_SHORT points is summed by its warp,
+// whose lanes gather 32 points at a time, the next 32 while three of them add a
+// coordinate each in order (one thread alone waits for the gathers: 100 voxels of 20k
+// points 27 ms, 2.3 so).  `starts` and tx may be the same memory: a
+// thread reads its start before it writes.  mark: a word per point, zeroed.
+__global__ void __launch_bounds__(XYZ_THREADS) k_voxel_xyz_f32(
+    Control *ctl, SortBuffers sort, const SortState *sort_state, const float4 *aos,
+    const uint64_t *vkeys, const uint32_t *vcounts, const uint32_t *starts, float *tx, float *ty,
+    float *tz, uint32_t *tc, uint64_t *tk, uint32_t *mark) {
+  __shared__ float rows[XYZ_THREADS / 32][3][32];
   if (ld_relaxed_u32(&ctl->status)) return;
   const uint32_t n = uint32_t(ctl->n_points);
   const uint32_t nv = uint32_t(ctl->n_voxels);
   const SortedView sv = sorted_view(sort, *sort_state);
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    const uint32_t m = starts[v], cnt = vcounts[v];
-    const uint64_t key = vkeys[v];
-    if (m >= n || cnt == 0 || cnt > n - m) {
-      atomicOr(&ctl->status, ST_INTERNAL);  // cannot happen for a consistent chain
-      continue;
+  const uint32_t lane = threadIdx.x & 31u;
+  float(*row)[32] = rows[threadIdx.x >> 5];
+  // few voxels are spread over the warps: a warp takes its long ones one after another
+  const uint32_t warps = gridDim.x * (XYZ_THREADS / 32);
+  const uint32_t per = max(1u, min(32u, (nv + warps - 1) / warps));
+  for (uint32_t v0 = (blockIdx.x * (XYZ_THREADS / 32) + (threadIdx.x >> 5)) * per; v0 < nv;
+       v0 += warps * per) {
+    const uint32_t v = v0 + lane;
+    uint32_t m = 0, cnt = 0;
+    uint64_t key = 0;
+    bool ok = lane < per && v < nv;
+    if (ok) {
+      m = starts[v];
+      cnt = vcounts[v];
+      key = vkeys[v];
+      ok = m < n && cnt > 0 && cnt <= n - m;
+      if (!ok) atomicOr(&ctl->status, ST_INTERNAL);  // cannot happen for a consistent chain
     }
+    auto point = [&](uint32_t at, bool in, bool &good) {
+      const uint32_t i = in ? sv.val(at) : n;
+      good &= !in || i < n;
+      return i < n ? aos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    };
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
-    bool ok = true;
+    if (ok && cnt <= XYZ_SHORT) {
 #pragma unroll 4
-    for (uint32_t q = 0; q < cnt; ++q) {
-      const uint32_t i = sv.val(m + q);
-      ok &= i < n;
-      const float4 p = i < n ? aos[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-      sx = __fadd_rn(sx, p.x);
-      sy = __fadd_rn(sy, p.y);
-      sz = __fadd_rn(sz, p.z);
+      for (uint32_t q = 0; q < cnt; ++q) {
+        const float4 p = point(m + q, true, ok);
+        sx = __fadd_rn(sx, p.x);
+        sy = __fadd_rn(sy, p.y);
+        sz = __fadd_rn(sz, p.z);
+      }
+      if (!ok) atomicOr(&ctl->status, ST_INTERNAL);
     }
-    if (!ok) {
-      atomicOr(&ctl->status, ST_INTERNAL);
-      continue;
+    for (uint32_t todo = __ballot_sync(FULL_MASK, ok && cnt > XYZ_SHORT); todo; todo &= todo - 1) {
+      const uint32_t owner = __ffs(todo) - 1;
+      const uint32_t m0 = __shfl_sync(FULL_MASK, m, owner), c0 = __shfl_sync(FULL_MASK, cnt, owner);
+      bool good = true;
+      float sum = 0.0f;  // lanes 0 to 2: x, y, z
+      float4 next = point(m0 + lane, lane < c0, good);
+      for (uint32_t q = 0; q < c0; q += 32) {
+        row[0][lane] = next.x;
+        row[1][lane] = next.y;
+        row[2][lane] = next.z;
+        __syncwarp();
+        if (q + 32 < c0) next = point(m0 + q + 32 + lane, q + 32 + lane < c0, good);
+        if (lane < 3) {
+          const uint32_t k = min(32u, c0 - q);
+          if (k == 32) {
+#pragma unroll
+            for (uint32_t j = 0; j < 32; ++j) sum = __fadd_rn(sum, row[lane][j]);
+          } else {
+            for (uint32_t j = 0; j < k; ++j) sum = __fadd_rn(sum, row[lane][j]);
+          }
+        }
+        __syncwarp();
+      }
+      good = __all_sync(FULL_MASK, good);
+      const float x = __shfl_sync(FULL_MASK, sum, 0), y = __shfl_sync(FULL_MASK, sum, 1);
+      const float z = __shfl_sync(FULL_MASK, sum, 2);
+      if (lane == owner) {
+        sx = x, sy = y, sz = z;
+        ok = good;
+        if (!good) atomicOr(&ctl->status, ST_INTERNAL);
+      }
     }
+    if (!ok) continue;
     const float inv = 1.0f / float(cnt);  // IEEE division: the library is built without fast math
     tx[v] = __fmul_rn(sx, inv);
     ty[v] = __fmul_rn(sy, inv);

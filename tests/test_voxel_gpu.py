@@ -374,3 +374,48 @@ def test_device_results_at_any_alignment(cuda_ctx, n, offset):
         got = b.cpu().numpy()
         assert np.array_equal(got[offset:offset + len(w)], w)
         assert np.all(got[:offset] == 0xA5) and np.all(got[offset + len(w):] == 0xA5)
+
+
+@pytest.mark.parametrize("n_attrs", range(10))
+def test_long_voxels_of_every_column_count(cuda_ctx, n_attrs):
+    """Voxels at the edges of what a thread, a warp's step and a tile hold, points in
+    random order: every share of the columns against the oracle.  The device sums a long
+    voxel's FP64 columns over lanes, so a mean may differ from the sequential one by its
+    last f32 bit."""
+    rng = np.random.default_rng(n_attrs)
+    sizes = [1, 31, 32, 33, 64, 65, 127, 128, 129, 256, 257, 511, 513, 1023, 1024, 1025, 2049, 5000]
+    at = rng.permutation(np.repeat(np.arange(len(sizes)), sizes))
+    p = rng.uniform(0.01, 0.99, (len(at), 3))
+    p[:, 0] += at
+    p[0] = 0.0
+    x, y, z = np.ascontiguousarray(p.T.astype(F))
+    attrs = [rng.normal(100, 5, len(at)).astype(F) for _ in range(n_attrs)]
+    cols, keys, counts = cuda_ctx.voxel_centroid(x, y, z, attrs, leaf=1.0, want_keys=True)
+    ref = oracle.voxel_centroid(x, y, z, attrs, leaf=1.0)
+    assert np.array_equal(keys, ref.keys) and np.array_equal(counts, ref.counts)
+    for g, r in zip(cols, ref.fields):
+        assert np.all(np.abs(g - r) <= np.spacing(np.abs(r)))
+
+
+@pytest.mark.parametrize("sizes", [[1, 2, 127, 128, 129], [160, 161, 1000, 31, 5000],
+                                   [130] * 400 + [1] * 1000])
+def test_long_voxels_of_bare_positions(cuda_ctx, sizes):
+    """The plain-xyz path's f32 sums run in input order: bit-exact for voxels summed by a
+    thread and by a warp."""
+    rng = np.random.default_rng(len(sizes))
+    at = rng.permutation(np.repeat(np.arange(len(sizes)), sizes))
+    p = rng.uniform(0.01, 0.99, (len(at), 3))
+    p[:, 0] += at
+    p[0] = 0.0
+    x, y, z = np.ascontiguousarray(p.T.astype(F))
+    cols, keys, counts = cuda_ctx.voxel_centroid(x, y, z, leaf=1.0, plain_xyz=True, want_keys=True)
+    order = {}
+    for i, k in enumerate(map(int, np.floor(x))):
+        order.setdefault(k, []).append(i)
+    assert [int(c) for c in counts] == [len(v) for v in order.values()]
+    for j, members in enumerate(order.values()):
+        for g, c in zip(cols, (x, y, z)):
+            total = F(0)
+            for v in c[members]:
+                total = F(total + v)
+            assert g[j] == total * (F(1) / F(len(members)))

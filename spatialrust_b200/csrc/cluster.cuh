@@ -132,6 +132,8 @@ __device__ __forceinline__ uint64_t uf_join(uint64_t *link, uint32_t i, uint64_t
 // before its odd ones, took 235 ms, 200 us so (the index forest: 410 us).  The scans
 // gain from it as well: 2M points at 2.5 per cell 525 -> 430 us.
 constexpr uint32_t CL_CLIMB = 16;
+constexpr uint32_t CL_LOOK = 32;
+constexpr uint32_t CL_STEP = 4;
 
 // ---- kernels -------------------------------------------------------------------
 
@@ -151,9 +153,16 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_init(Control *ctl, const
 
 // One lane per cell-sorted point i: the candidates j > i of its 27-cell
 // neighbourhood (each unordered pair once) that pass the predicate are joined
-// with it -- all of them, or with Sample only the first of each column.  The
+// with it -- all of them, or with Sample only the first of each column, sought among
+// its first CL_LOOK.  The
 // columns before the query's own in key order hold no position above i, so
 // the walk starts at its own column (range 4).  The index forest has no sampled pass.
+//
+// Where a range of the warp is longer than CL_LOOK its lanes walk in step, CL_STEP
+// candidates between votes: once a join has parted them they walk the rest of a range
+// one after another, which long ranges with few hits make most of (100k points with an
+// outlier that widens the cells to 400 points: 10.3 ms, 0.94 so; 1M points at 50 a cell
+// 3.8 ms, 1.6 so).  Short ranges, where the votes cost more than they give, go without.
 //
 // A lane whose point and candidate hang under different words climbs by
 // dependent loads from L2 while its warp waits, so the cost is the number of
@@ -171,39 +180,70 @@ __global__ void __launch_bounds__(CL_THREADS) k_cluster_union(Control *ctl, cons
   const uint32_t n = uint32_t(ctl->n_points);
   const uint64_t u_count = ctl->n_cells;
   uint32_t *parent = reinterpret_cast<uint32_t *>(link);
-  for (uint32_t i = blockIdx.x * CL_THREADS + threadIdx.x; i < n; i += gridDim.x * CL_THREADS) {
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint32_t base = blockIdx.x * CL_THREADS + (threadIdx.x - lane); base < n;
+       base += gridDim.x * CL_THREADS) {
+    const uint32_t i = min(base + lane, n - 1);
     const float4 q = pts[i];
     const uint32_t u = pt_cell[i];
     const uint32_t a = __float_as_uint(q.w);
+    bool active = base + lane < n;  // the other lanes stay for the warp's votes
     if (u >= u_count || a >= n) {  // cannot happen for a consistent cell table
       atomicOr(&ctl->status, ST_INTERNAL);
-      continue;
+      active = false;
     }
-    const uint2 *rg = ranges + size_t(u) * 9;
+    // a NaN coordinate is near nothing, and all of a cloud's NaN points share one cell
+    if (isnan(q.x) || isnan(q.y) || isnan(q.z)) active = false;
+    const uint2 *rg = active ? ranges + size_t(u) * 9 : nm_no_ranges;
     uint64_t root = dense ? ld_relaxed(link + i) : 0;  // the highest ancestor of i met so far
+    auto near = [&](uint32_t j) {
+      const float4 c = __ldg(pts + j);
+      const float dx = __fsub_rn(c.x, q.x);
+      const float dy = __fsub_rn(c.y, q.y);
+      const float dz = __fsub_rn(c.z, q.z);
+      return __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)) <= r2;
+    };
+    auto join = [&](uint32_t j) {
+      if (Sample || dense) {
+        const uint64_t w = ld_relaxed(link + j);
+        if (w == root) return;
+        const uint64_t up = uf_join<Sample ? CL_CLIMB : SPIN_LIMIT>(link, i, root, j, w);
+        if (up != UF_NONE) root = up;
+        else if (!Sample) atomicOr(&ctl->status, ST_TIMEOUT);
+      } else {
+        const uint32_t b = __float_as_uint(pts[j].w);
+        if (b < n) uf_union(parent, a, b, &ctl->status);
+        else atomicOr(&ctl->status, ST_INTERNAL);
+      }
+    };
 #pragma unroll 1
     for (int r = 4; r < 9; ++r) {
       const uint2 range = rg[r];
-      for (uint32_t j = range.x > i + 1 ? range.x : i + 1; j < range.y; ++j) {
-        const float4 c = __ldg(pts + j);
-        const float dx = __fsub_rn(c.x, q.x);
-        const float dy = __fsub_rn(c.y, q.y);
-        const float dz = __fsub_rn(c.z, q.z);
-        const float d2 =
-            __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
-        if (!(d2 <= r2)) continue;
-        if (Sample || dense) {
-          const uint64_t w = ld_relaxed(link + j);
-          if (w != root) {
-            const uint64_t up = uf_join<Sample ? CL_CLIMB : SPIN_LIMIT>(link, i, root, j, w);
-            if (up != UF_NONE) root = up;
-            else if (!Sample) atomicOr(&ctl->status, ST_TIMEOUT);
+      uint32_t j = max(range.x, i + 1), end = range.y;
+      const bool in_step = dense && __any_sync(FULL_MASK, end > j + CL_LOOK);
+      if (Sample) end = min(end, j + CL_LOOK);
+      if (!in_step) {
+        for (; j < end; ++j)
+          if (near(j)) {
+            join(j);
+            if (Sample) break;
           }
-          if (Sample) break;
-        } else {
-          const uint32_t b = __float_as_uint(c.w);
-          if (b < n) uf_union(parent, a, b, &ctl->status);
-          else atomicOr(&ctl->status, ST_INTERNAL);
+        continue;
+      }
+      for (; __any_sync(FULL_MASK, j < end); j += CL_STEP) {
+        uint32_t hits = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < CL_STEP; ++k)
+          if (j + k < end && near(j + k)) hits |= 1u << k;
+        if (Sample && hits) {
+          hits &= 0u - hits;  // the first
+          end = 0;
+        }
+        if (!__any_sync(FULL_MASK, hits != 0)) continue;
+#pragma unroll 1
+        for (uint32_t k = 0; k < CL_STEP; ++k) {
+          if ((hits >> k) & 1u) join(j + k);
+          __syncwarp();
         }
       }
     }

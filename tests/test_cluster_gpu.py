@@ -181,3 +181,17 @@ def test_roots_on_either_side_of_the_density_line(cuda_ctx, pattern, groups, ext
     info = cuda_ctx.chain_info()
     assert (info["points"], info["cells"]) == (per * groups + extra, k * groups)
     assert np.array_equal(got, ref)
+
+
+@pytest.mark.parametrize("spread", [1.0, 8.0])
+@pytest.mark.parametrize("n", [31, 33, 36, 37, 65, 300, 5000])
+def test_cells_far_wider_than_the_tolerance(cuda_ctx, n, spread):
+    """A point 10,000 km away makes the cells 19 m wide: long ranges of candidates, walked
+    in step, with many hits (spread 1) or few; and NaN points, which share a cell."""
+    rng = np.random.default_rng(n)
+    p = rng.normal(0, spread, (n, 3)).astype(F)
+    p[3::7] = np.nan
+    p[n // 2] = 1e7
+    got = cuda_ctx.euclidean_cluster_roots(p[:, 0], p[:, 1], p[:, 2], 0.3)
+    assert cuda_ctx.chain_info()["cell_size"] > 10
+    assert np.array_equal(got, oracle.euclidean_roots(p[:, 0], p[:, 1], p[:, 2], 0.3, sparse=True))

@@ -541,7 +541,7 @@ __device__ __forceinline__ void nm_bulk(void *dst, const void *src, uint32_t byt
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(nm_smem_addr(dst)), "l"(src), "r"(bytes), "r"(nm_smem_addr(bar)) : "memory");
 }
-__device__ const uint2 nm_no_ranges[9] = {};  // the walk of a lane whose cell is out of range
+__device__ const uint2 nm_no_ranges[9] = {};  // the walk of a lane that has none
 
 // The neighbour walks of k_normals.
 constexpr int WALK_L1 = 0;      // range by range through L1, two candidates per step
@@ -575,6 +575,9 @@ __device__ __forceinline__ uint64_t f2_sub(uint64_t a, uint64_t b) {
   asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
   return r;
 }
+// The assembler may fuse this with an f2_add of its result, explicit rounding or not.
+// Where it is used the product's halves are needed by themselves too, and it does not:
+// the walks' normals are compared bit by bit in the tests.
 __device__ __forceinline__ uint64_t f2_mul(uint64_t a, uint64_t b) {
   uint64_t r;
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
@@ -934,7 +937,9 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
     const NormalParamsDev prm = bt.nparams[cb];
     const float r2 = bt.cplans[cb].r2;
     const float shell_tol = bt.cplans[cb].shell_tol;
-    const uint2 *rg = bad ? nm_no_ranges : ranges + size_t(u) * 9;
+    // a NaN query has no neighbour, and all of a cloud's NaN points share one cell
+    const bool walks = !bad && !isnan(qp.x) && !isnan(qp.y) && !isnan(qp.z);
+    const uint2 *rg = walks ? ranges + size_t(u) * 9 : nm_no_ranges;
     float hits = 0.f;
     uint32_t shell = 0;
     double S[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};  // sx sy sz sxx syy szz sxy sxz syz

@@ -1258,7 +1258,11 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
 // kernel registers (batch of 14M points: 1990 us in one kernel; 1280 us and 230 us
 // here for the 628k points of this list).
 //
-// Long lists go one lane per query.  Short ones would leave most of the chip
+// Long lists go one lane per query, from 16 queries a warp of the grid on, and over cells
+// of 32 points and more from four: queries that share a cell's thousands of candidates
+// then share their loads (31k queries of 1M points at 67 a cell: both kernels 3520 us a
+// warp each, 3047 so; at 10 a cell and less four queries a warp already lose 5%).  Short
+// ones would leave most of the chip
 // idle behind a few lanes' chains of candidate loads, so there a warp takes its
 // few queries one after the other: the lanes test 32 candidates at a time and
 // nine of them add the hits' terms in the walk's order, the same operations in
@@ -1283,7 +1287,8 @@ __global__ void __launch_bounds__(NM_THREADS, RF_BLOCKS) k_normals_refine(
   const uint32_t lane = threadIdx.x & 31u;
   const uint32_t warps = gridDim.x * (NM_THREADS / 32);
   const uint32_t warp = blockIdx.x * (NM_THREADS / 32) + (threadIdx.x >> 5);
-  const bool alone = count >= warps * 16;  // one lane per query
+  // one lane per query
+  const bool alone = count >= warps * 16 || (count >= warps * 4 && n >= 32 * u_count);
   const uint32_t per = alone ? 32 : max(1u, min(32u, (count + warps - 1) / warps));
   RefineWarp &sh = rw[threadIdx.x >> 5];
   for (uint64_t first = uint64_t(warp) * per; first < count; first += uint64_t(warps) * per) {

@@ -335,6 +335,11 @@ constexpr int SEG_ITEMS = 4;
 constexpr int SEG_TILE = SEG_THREADS * SEG_ITEMS;  // 1024 sorted positions per tile
 constexpr uint32_t SEG_SHORT = 32;  // longer voxels are reduced by a whole warp
 constexpr int SEG_GROUP = 4;  // columns gathered and summed together
+// A claimed tile keeps all later ones waiting in their look-back until it is counted, so a
+// block that long voxels will hold -- the tile's average SEG_MEAN points and more, or its
+// last goes on for SEG_RUN beyond it -- claims its next tile after them (2M points in
+// 100 voxels: 0.82 ms with the claim ahead of them, 0.32 so; 4M in 16 53 ms and 3.6).
+constexpr uint32_t SEG_MEAN = 64, SEG_RUN = 256;
 // A long voxel's columns go to warps LONG_FIRST columns, then LONG_NEXT at a time; a lane
 // has LONG_LOADS gathers in flight, or four items' keys.
 constexpr int LONG_FIRST = 4, LONG_NEXT = 2, LONG_LOADS = 16;
@@ -352,7 +357,8 @@ struct SegmentSmemHead {
   uint32_t tile;              // the tile at work, then the next one
   uint32_t seg_base;
   uint32_t num_longs;
-  uint32_t pad;
+  uint32_t late;              // 1: the next tile is claimed after the long voxels
+  uint64_t ahead;             // the key SEG_RUN items after the tile
 };
 __host__ __device__ constexpr size_t segment_smem_bytes(int nc) {
   return sizeof(SegmentSmemHead) + size_t(nc) * SEG_TILE * sizeof(float);
@@ -642,6 +648,7 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
       }
       if (t == 0) edge = sv.keys[base > 0 ? base - 1 : 0u];
       if (t == 1) edge = sv.keys[base + tile_n < n ? base + tile_n : n - 1];
+      if (t == 2) edge = sv.keys[base + tile_n + SEG_RUN < n ? base + tile_n + SEG_RUN : n - 1];
       if (!sv.packed) {
 #pragma unroll
         for (int q = 0; q < SEG_ITEMS; ++q) {
@@ -670,6 +677,7 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
         sm.num_longs = 0;
       }
       if (t == 1) sm.keys[1 + tile_n] = base + tile_n < n ? edge : ~edge;
+      if (t == 2) sm.ahead = base + tile_n + SEG_RUN < n ? edge : ~edge;
     }
     float4 pt[SEG_ITEMS];
     gather_points<NC>(pt, iv, cols, aos_in, n);
@@ -690,7 +698,8 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
                                   num_tiles <= gridDim.x);
       if (t == 0) {
         sm.seg_base = seg_base;
-        sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
+        sm.late = voxels * SEG_MEAN < tile_n || sm.ahead == sm.keys[tile_n];
+        if (!sm.late) sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
         sm.start[voxels] = uint16_t(tile_n);
         if (tile == num_tiles - 1) ctl->n_voxels = seg_base + voxels;
       }
@@ -715,25 +724,26 @@ __global__ void __launch_bounds__(SEG_THREADS, 4) k_voxel_segments(Control *ctl,
     }
     __syncthreads();
     // Long voxels: a warp finds the end; then a warp for every share of its columns reduces
-    // them from global memory.  One warp for all columns, an item at a time, waited for
-    // its gathers: 2M points in 1600 voxels 373 us at three columns and 1934 at twelve,
-    // 140 and 540 so; in 100 voxels 2.3 and 12.8 ms, 0.8 and 2.1 so.
-    const uint32_t longs = sm.num_longs;
-    if (longs == 0) continue;
-    for (uint32_t i = t >> 5; i < longs; i += SEG_THREADS / 32) {
-      const uint32_t q = sm.longs[i];
-      const uint32_t e = voxel_end(sv, sm.keys[1 + sm.start[q]], base + sm.start[q + 1], n);
-      if (lane == 0) sm.ends[i] = e;
+    // them from global memory.  With one warp for all columns, an item at a time, and the
+    // next tile claimed before, 2M points in 1600 voxels took 373 us at three columns and
+    // 1934 at twelve, 119 and 457 so; in 100 voxels 2.3 and 12.7 ms, 0.32 and 0.76.
+    if (const uint32_t longs = sm.num_longs) {
+      for (uint32_t i = t >> 5; i < longs; i += SEG_THREADS / 32) {
+        const uint32_t q = sm.longs[i];
+        const uint32_t e = voxel_end(sv, sm.keys[1 + sm.start[q]], base + sm.start[q + 1], n);
+        if (lane == 0) sm.ends[i] = e;
+      }
+      __syncthreads();
+      constexpr uint32_t SHARES =
+          NC <= LONG_FIRST ? 1 : 1 + (NC - LONG_FIRST + LONG_NEXT - 1) / LONG_NEXT;
+      for (uint32_t i = t >> 5; i < longs * SHARES; i += SEG_THREADS / 32) {
+        const uint32_t q = sm.longs[i / SHARES];
+        const uint64_t key = sm.keys[1 + sm.start[q]];
+        long_share<NC>(i % SHARES, sv, base + sm.start[q], sm.ends[i / SHARES], sm.seg_base + q,
+                       key, cols, aos_in, voxel_agg(bt, key, vkey_bits, agg_all), dst);
+      }
     }
-    __syncthreads();
-    constexpr uint32_t SHARES =
-        NC <= LONG_FIRST ? 1 : 1 + (NC - LONG_FIRST + LONG_NEXT - 1) / LONG_NEXT;
-    for (uint32_t i = t >> 5; i < longs * SHARES; i += SEG_THREADS / 32) {
-      const uint32_t q = sm.longs[i / SHARES];
-      const uint64_t key = sm.keys[1 + sm.start[q]];
-      long_share<NC>(i % SHARES, sv, base + sm.start[q], sm.ends[i / SHARES], sm.seg_base + q, key,
-                     cols, aos_in, voxel_agg(bt, key, vkey_bits, agg_all), dst);
-    }
+    if (t == 0 && sm.late) sm.tile = atomicAdd(&ctl->work[WK_VSEG], 1u);
   }
 }
 
@@ -777,7 +787,7 @@ constexpr uint32_t XYZ_SHORT = 128;  // points of a voxel that its thread sums a
 // One thread per voxel; a voxel of more than XYZ_SHORT points is summed by its warp,
 // whose lanes gather 32 points at a time, the next 32 while three of them add a
 // coordinate each in order (one thread alone waits for the gathers: 100 voxels of 20k
-// points 27 ms, 2.3 so).  `starts` and tx may be the same memory: a
+// points 27 ms, 1.7 so).  `starts` and tx may be the same memory: a
 // thread reads its start before it writes.  mark: a word per point, zeroed.
 __global__ void __launch_bounds__(XYZ_THREADS) k_voxel_xyz_f32(
     Control *ctl, SortBuffers sort, const SortState *sort_state, const float4 *aos,

@@ -548,6 +548,7 @@ constexpr int WALK_L1 = 0;      // range by range through L1, two candidates per
 constexpr int WALK_STAGED = 1;  // range by range from shared memory filled by bulk copies
 constexpr int WALK_PACKED = 2;  // range by range through L1, packed f32x2 arithmetic
 constexpr int WALK_DEEP = 3;    // the packed walk with more loads in flight, for dense cells
+constexpr int WALK_RAW = 4;     // the packed walk of a raw cloud, which may hold NaN points
 
 // Which of the packed walks a launch is for: a launch that is not for the grid
 // at hand returns at once.
@@ -881,7 +882,7 @@ constexpr uint32_t REFINE_SOLVE = 1u << 31;
 // walk reads through L1 instead; which one a context runs is a tuning choice
 // (srcu_set_neighbor_staging).
 template <bool CountShell, bool PlaneCov = false, int Walk = WALK_L1>
-__global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_normals(Control *ctl, const float4 *pts,
+__global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED || Walk == WALK_RAW ? 5 : 4) k_normals(Control *ctl, const float4 *pts,
                                                            const uint32_t *pt_cell,
                                                            const uint2 *ranges,
                                                            const uint64_t *cell_key, Batch bt,
@@ -900,7 +901,7 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
   uint32_t phase = 0;
   bool timed_out = false;
   constexpr bool Staged = Walk == WALK_STAGED;
-  constexpr bool Packed = Walk == WALK_PACKED || Walk == WALK_DEEP;
+  constexpr bool Packed = Walk == WALK_PACKED || Walk == WALK_RAW || Walk == WALK_DEEP;
   if constexpr (Staged) {
     __shared__ float4 nm_stage[(NM_THREADS / 32) * NM_STAGE];
     __shared__ __align__(8) uint64_t nm_bar[NM_THREADS / 32];
@@ -937,8 +938,11 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED ? 5 : 4) k_nor
     const NormalParamsDev prm = bt.nparams[cb];
     const float r2 = bt.cplans[cb].r2;
     const float shell_tol = bt.cplans[cb].shell_tol;
-    // a NaN query has no neighbour, and all of a cloud's NaN points share one cell
-    const bool walks = !bad && !isnan(qp.x) && !isnan(qp.y) && !isnan(qp.z);
+    // A NaN query has no neighbour, and all of a cloud's NaN points share one cell.  (In
+    // the walk of centroids the test costs 2%.)
+    bool walks = !bad;
+    if constexpr (Walk == WALK_RAW || Walk == WALK_DEEP)
+      walks = walks && !isnan(qp.x) && !isnan(qp.y) && !isnan(qp.z);
     const uint2 *rg = walks ? ranges + size_t(u) * 9 : nm_no_ranges;
     float hits = 0.f;
     uint32_t shell = 0;

@@ -835,6 +835,10 @@ srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const fl
   return SRCU_OK;
 }
 
+// Raw clouds below this do without the deep walk: its launch costs a call of 33 points 3
+// of 93 us.
+constexpr uint64_t kDeepPoints = 1024;
+
 // The normals kernels over the grid, in the context's neighbour walk.  raw: the
 // points are a caller's cloud, whose cells may be dense or not.  Chains do without the
 // deep walk and its launch: at a radius of three leaves a cell holds at most nine
@@ -843,7 +847,8 @@ srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const fl
 template <bool Shell, bool PlaneCov>
 srcu_status launch_normals(srcu_ctx *ctx, const unsigned long long *count_dev, const Batch &bt,
                            NormalDst dst, bool raw) {
-  const bool by_density = raw && ctx->neighbor_staging == WALK_PACKED;
+  const bool by_density =
+      raw && ctx->neighbor_staging == WALK_PACKED && ctx->last_points >= kDeepPoints;
   Launch l(ctx, SRCU_K_NORMALS, by_density ? 3 : 2);
   const uint32_t sms = uint32_t(ctx->num_sms);
   const float4 *pts = ptr<float4>(ctx->pts);
@@ -854,7 +859,8 @@ srcu_status launch_normals(srcu_ctx *ctx, const unsigned long long *count_dev, c
   auto kernel = k_normals<Shell, PlaneCov, WALK_L1>;
   int occ = ctx->occ_normals, grid = GRID_ANY;
   if (ctx->neighbor_staging == WALK_PACKED) {
-    kernel = k_normals<Shell, PlaneCov, WALK_PACKED>;
+    if constexpr (PlaneCov) kernel = k_normals<Shell, PlaneCov, WALK_RAW>;  // raw clouds alone
+    else kernel = raw ? k_normals<Shell, PlaneCov, WALK_RAW> : k_normals<Shell, PlaneCov, WALK_PACKED>;
     occ = ctx->occ_normals_packed;
     if (by_density) {
       grid = GRID_SPARSE;

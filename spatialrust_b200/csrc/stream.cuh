@@ -41,6 +41,10 @@ constexpr int SV_THREADS = 256;
 constexpr int SV_ITEMS = 4;
 constexpr int SV_TILE = SV_THREADS * SV_ITEMS;  // sorted positions per tile
 constexpr uint32_t SV_SHORT = 64;  // longer segments are reduced by a whole block
+// Of those: points a thread loads before it adds them.  A sum alone in its loop waits
+// for each point (2M points of five columns in one voxel: 11.1 ms, 5.8 with four ahead;
+// in some 800 voxels 1.03 ms, 0.70).
+constexpr uint32_t SV_AHEAD = 4;
 constexpr double SV_I64_EDGE = 9223372036854775808.0;  // 2^63: i64::MIN and i64::MAX as f64
 
 // Packing of one sort: per-axis key minimum and bit widths.  Bit total_bits
@@ -616,7 +620,18 @@ __global__ void __launch_bounds__(SV_THREADS) k_stream_long(Control *ctl, SortBu
     } else {
       for (uint32_t u = 0; u < in.lay.units; ++u) {
         Kahan k[4];
-        for (uint32_t p = start + t; p < end; p += SV_THREADS)
+        uint32_t p = start + t;
+        for (; p + (SV_AHEAD - 1) * SV_THREADS < end;
+             p += SV_AHEAD * SV_THREADS) {
+          uint4 q[SV_AHEAD];
+#pragma unroll
+          for (uint32_t a = 0; a < SV_AHEAD; ++a)
+            q[a] = in.points[uint64_t(sv.val(p + a * SV_THREADS)) * in.lay.units + u];
+#pragma unroll
+          for (uint32_t a = 0; a < SV_AHEAD; ++a)
+            stream_fields(in.lay, u, q[a], [&](uint32_t s, uint32_t, double x) { k[s].add(x); });
+        }
+        for (; p < end; p += SV_THREADS)
           stream_fields(in.lay, u, in.points[uint64_t(sv.val(p)) * in.lay.units + u],
                         [&](uint32_t s, uint32_t, double x) { k[s].add(x); });
         stream_fields(in.lay, u, make_uint4(0, 0, 0, 0),

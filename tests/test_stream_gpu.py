@@ -113,6 +113,19 @@ def test_long_voxels_in_runs_and_in_the_merge(cuda_ctx):
     assert info["voxels"] == 3 and info["device_runs"] == 300
 
 
+@pytest.mark.parametrize("f64", ["", "fd", "fdfdfd"])
+def test_long_voxels_at_the_edges_of_a_block(cuda_ctx, f64):
+    # one voxel per length: about the short limit (64), a block (256), the points a
+    # block loads ahead (1024), and a block's rest after them
+    sizes = [64, 65, 255, 256, 257, 767, 768, 769, 1023, 1024, 1025, 1279, 1280, 1281, 2047, 2049]
+    rng = np.random.default_rng(23)
+    x = rng.permutation(np.repeat(np.arange(len(sizes)), sizes)).astype(F) + F(0.25)
+    y = rng.uniform(0, 0.9, len(x)).astype(F)
+    z = rng.uniform(0, 0.9, len(x)).astype(F)
+    attrs = [rng.uniform(1, 2, len(x)).astype(np.float64 if t == "d" else F) for t in f64]
+    check_stream(cuda_ctx, x, y, z, attrs, leaf=1.0)
+
+
 def test_non_finite_points_are_skipped_and_negative_keys(cuda_ctx):
     rng = np.random.default_rng(8)
     p = rng.normal(0, 5, (50_000, 3)).astype(F)

@@ -279,7 +279,7 @@ srcu_status srcu_get_sort_tuning(srcu_ctx *ctx, int32_t kind, uint64_t *max_poin
  * block) first staged in shared memory by non-multicast cp.async.bulk copies.
  * 2: walk 0 with the predicate and the moments in packed f32x2 arithmetic.
  * Every walk gives the same neighbour sets and counts, and walks 0 and 2 give
- * bit-identical outputs.  -1 restores the built-in choice (measured by the
+ * bit-identical normals (covariances agree to rounding).  -1 restores the built-in choice (measured by the
  * autotuner).  Plane covariances take walk 2 when it is chosen, else 0. */
 srcu_status srcu_set_neighbor_staging(srcu_ctx *ctx, int32_t mode);
 int32_t srcu_get_neighbor_staging(srcu_ctx *ctx);

@@ -1070,7 +1070,7 @@ __global__ void __launch_bounds__(NM_THREADS, Walk == WALK_PACKED || Walk == WAL
     } else if constexpr (Packed) {
       // The L1 walk's candidate order and flush points, with the predicate and
       // the moments in packed f32x2 arithmetic: the same IEEE operation on each
-      // half, so every result is bit-identical to WALK_L1's.  The walk waits on
+      // half, so neighbours and normals are bit-identical to WALK_L1's.  It waits on
       // L2: a record's sector is shared by one other record only, so every two
       // candidates miss L1.  So candidates are loaded a group ahead of the one
       // being visited (the FP64 sums live in shared memory to make room), up to

@@ -835,9 +835,11 @@ srcu_status enqueue_grid(srcu_ctx *ctx, const float *x, const float *y, const fl
   return SRCU_OK;
 }
 
-// Raw clouds below this do without the deep walk: its launch costs a call of 33 points 3
-// of 93 us.
-constexpr uint64_t kDeepPoints = 1024;
+// Raw clouds below this do without the deep walk: the launch that a sparse cloud gives it
+// in vain costs as much as a dense one gains.  Covariances with it / without, us: 2000
+// points at 0.5 per cell 106 / 103, at 100 per cell 167 / 169; 4000 at 4 per cell
+// 117 / 108, at 100 per cell 181 / 187; 16k at 0.5 119 / 115, at 100 231 / 252.
+constexpr uint64_t kDeepPoints = 4096;
 
 // The normals kernels over the grid, in the context's neighbour walk.  raw: the
 // points are a caller's cloud, whose cells may be dense or not.  Chains do without the

@@ -207,10 +207,10 @@ def test_duplicates_and_shell_points(cuda_ctx):
 def test_shell_points_of_a_radius_whose_square_overflows(cuda_ctx, name, walk):
     # r^2 = inf: every other point at a finite, non-zero d^2 is on the shell, the query
     # itself, its duplicates, NaN points and d^2 = inf are not.  One cell holds them all:
-    # the deep walk at 1500 points, the sparse one below 1024.
+    # the deep walk at 4200 points, the sparse one below 4096.
     rng = np.random.default_rng(3)
     clouds = dict(alone=np.zeros((1, 3)), duplicates=np.ones((20, 3)), few=rng.normal(size=(5, 3)),
-                  many=rng.normal(size=(1500, 3)),
+                  many=rng.normal(size=(4200, 3)),
                   far=np.repeat([[0.0, 0, 0], [3e19, 0, 0]], 6, axis=0))
     p = clouds[name].astype(np.float32)
     if name in ("few", "many"):
